@@ -33,6 +33,7 @@ UNITS = {
     "context.cu": [],
     "ns_kernels.cu": [],
     "krylov.cu": [],
+    "separable.cu": [],
     "amg.cu": [],
     "fused_solve.cu": [],
     "fused_op1.cu": [],

@@ -525,6 +525,8 @@ std::string load_case(const std::string &folder_in, int argc, const char **argv,
             ok = cli_value(argv[++i], P.solverPack) && (P.solverPack == 1 || P.solverPack == 2);
         else if (!strcmp(a, "-saStructured"))
             ok = cli_value(argv[++i], P.saStructured) && P.saStructured >= -1 && P.saStructured <= 1;
+        else if (!strcmp(a, "-separable"))
+            ok = cli_value(argv[++i], P.separable) && P.separable >= -1 && P.separable <= 1;
         else if (!strcmp(a, "-solverThreads"))
             ok = cli_value(argv[++i], P.solverThreads) && P.solverThreads >= 0 && P.solverThreads <= 512 &&
                  P.solverThreads % 32 == 0;

@@ -17,6 +17,7 @@
 #include <sys/stat.h>
 
 #include "../../include/cuibm.h"
+#include "separable.h"
 #include "solver.h"
 #include "batch_member.h"
 
@@ -650,6 +651,7 @@ cudaGraph_t cuibm_batch_member_graph(cuibm_ctx *h)
     if (!h) return nullptr;
     const Context &c = h->c;
     if (!c.initialised || !c.use_graph || c.profile_phases || c.sa_rebuild || !c.step_exec) return nullptr;
+    if (c.sys1.sep || c.sys2.sep) return nullptr;  // conditional nodes are not taken in a child graph
     return c.step_graph;
 }
 
@@ -1053,8 +1055,11 @@ int cuibm_launch_count(cuibm_ctx *h, long long *per_step)
         if (!c.step_exec) return fail(h, CUIBM_ERR_STATE, "launch counts need the step graph");
         if (strong_coupling(c))
             return fail(h, CUIBM_ERR_STATE, "a strongly coupled step's launches vary with its sub-iterations");
-        *per_step = c.static_kernels + (long long)c.sys1.body_kernels * read_body_runs(c, c.sys1) +
-                    (long long)c.sys2.body_kernels * read_body_runs(c, c.sys2);
+        *per_step = c.static_kernels;
+        for (LinearSystem *S : {&c.sys1, &c.sys2}) {
+            const int runs = read_body_runs(c, *S);
+            *per_step += S->sep ? separable_body_launches(*S, runs) : (long long)S->body_kernels * runs;
+        }
     });
     return CUIBM_OK;
 }
@@ -1199,6 +1204,8 @@ void cuibm_destroy(cuibm_ctx *h)
     free_sa_hierarchy(c.sys2);
     free_fused(c.sys1);
     free_fused(c.sys2);
+    free_separable(c.sys1);
+    free_separable(c.sys2);
     free_adjoint(c);
     if (c.arena) cudaFree(c.arena);
     if (c.h_scalars) cudaFreeHost(c.h_scalars);

@@ -2,6 +2,7 @@
 // fused_kernels.cuh, instantiated by fused_op1.cu, fused_op2.cu, fused_mixed_op1.cu and
 // fused_mixed_op2.cu).
 #include "fused_kernels.cuh"
+#include "separable.h"
 
 namespace cuibm {
 
@@ -368,6 +369,7 @@ void set_fused_trace(Context &c, LinearSystem &S, bool on)
 // bound, so this is a floor on traffic, not the bound.
 double solve_bytes(const LinearSystem &S, int it)
 {
+    if (S.sep) return separable_bytes(S, it);
     // mixed precision: the multigrid levels' vectors and matrix values are float (and,
     // for refinement, the Krylov vectors too; its FP64 residual phases are left out)
     const bool mixed = S.precision == PRECISION_MIXED && S.mixed;
@@ -422,7 +424,7 @@ double solve_bytes(const LinearSystem &S, int it)
 // BiCGSTAB iteration, one per CG iteration and one before it), apart from solve_bytes
 double solve_dense_bytes(const LinearSystem &S, int it)
 {
-    if (S.precond != PC_SMOOTHED_AGGREGATION || S.amg.empty()) return 0;
+    if (S.precond != PC_SMOOTHED_AGGREGATION || S.amg.empty() || S.sep) return 0;
     const double nc = S.amg.back()->n;
     const double cycles = S.krylov == KRYLOV_CG ? it + 1.0 : 2.0 * it;
     return cycles * 8.0 * nc * nc;

@@ -1,0 +1,1223 @@
+// The pressure system's separable preconditioner and the Krylov solves that use it.
+//
+// On the tensor-product pressure grid the operator of NavierStokes/kernels/LHS2.cu
+// (dt D G) is A0 = X (x) I + I (x) Y with tridiagonal X (entries of the column spacing)
+// and Y (of the row spacing), plus one or two doubled diagonals (the pinned cells) and,
+// for the immersed-boundary methods that patch it, the rows at the body.  A0 is inverted
+// directly: X = V diag(lambda) V^-1 with V = D^-1/2 Q, Q orthonormal (X is symmetric in
+// the column widths D), so
+//     r^ = Q^T D^1/2 r   (one dense product per row of the grid),
+//     (Y + lambda_k) z^_k = r^_k   (one tridiagonal solve per mode k),
+//     z = D^-1/2 Q z^    (the second dense product),
+// and the pinned cells are a rank-two or rank-three correction (Woodbury) of z^ before
+// the second product.  Q comes from the implicitly shifted QR iteration on the symmetric
+// tridiagonal matrix (Golub and Van Loan, Matrix Computations, ch. 8.3): the rotations
+// are found on the host in O(n^2) and applied to the identity on the GPU.
+//
+// Why: smoothed aggregation needed 70 to 330 BiCGSTAB iterations a step on the stretched,
+// nearly singular operators of the cylinder grids (Re 550, 922 x 922, to 1e-13: 250
+// iterations, 95 ms); this preconditioner is the inverse to rounding, so the solve ends
+// after one application or two.  It stays a preconditioner of the same Krylov method, with
+// the same stopping rule on the FP64 residual, so what the dense products' rounding leaves
+// (about 1e-9 of the residual at 922 x 922, as FP64 products leave it) the iteration
+// removes.
+//
+// The dense products are 2 n_m^2 n_r multiply-adds each, which at GB300's FP64 rate
+// (1.25 TFLOP/s) would take 1.25 ms at 922 x 922.  They run on the tensor cores instead,
+// exactly: a row is scaled by a power of two and written as kDigits base-256 digits in
+// [-128, 128] (55 bits below the row's largest value for 7 digits), each digit a BF16
+// value, and the products of digit i of one factor with digit j of the other, i + j <
+// kDigits, are accumulated as whole numbers below 2^24, which FP32 accumulators hold
+// exactly; every 128 terms the sums of equal i + j go into one 64-bit integer.  What is
+// dropped (i + j >= 7) is 2^-51 of the factors' row maxima, below the rounding of an FP64
+// sum of the same terms (the splitting of Ozaki, Ogita, Oishi and Rump, Numer. Algorithms
+// 59, 2012).
+#include <cuda_bf16.h>
+
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+#include <vector>
+
+#include "krylov_device.cuh"
+#include "separable.h"
+
+namespace cuibm {
+
+constexpr int kDigits = 7;       // digits of the FP64 solves: 28 products a dense product
+constexpr int kDigitsMixed = 4;  // mixed precision: 31 bits below the row's largest value, 10 products
+constexpr int kKC = 32;          // terms of a chunk of the dense product's sum
+constexpr int kFlush = 4;        // chunks between flushes: 7 x 128 x 2^14 < 2^24
+// Transforms up to this length; from there on the products (n_m^2 n_r) and the tables
+// (28 n_m^2 bytes) outgrow what was measured, and the accumulators' range ends at 4096
+constexpr int kSepMax = 2048;
+constexpr int kTriThreads = 512;
+
+// device view of the plan (a kernel argument)
+struct SepDev {
+    int nm, nr;            // modes (length of the transformed direction), rows (the other)
+    int sm, sr;            // strides of a field: element (row R, place m) at R sr + m sm
+    int nch;               // chunks of kKC terms in a transform
+    const __nv_bfloat16 *B1, *B2;  // digits of Q^T and of Q
+    const double *sB1, *sB2;       // their row scales (and the output's D^-1/2)
+    __nv_bfloat16 *A;      // digits of the operand at hand
+    double *sA;
+    double *h;             // r^, then z^: [row][mode]
+    const double *l, *c, *inv;     // tridiagonal factors [row][mode]
+    const double *Pf, *Pb;         // products of l and c over a thread's rows [thread row][mode]
+    const double *cm, *cr;         // input scaling per place and per row (cr null: 1)
+    // pinned cells: functionals F (rows R0, R1), responses G, the constant's response gm
+    int pins, R[2], k0;
+    const double *F[2], *G[2], *gm;
+    double K[9], mean;
+};
+
+struct SepPlan {
+    SepDev d{};
+    int digits = kDigits;
+    char *block = nullptr;  // one device allocation
+    int first_kernels = 0;  // kernels of the conditional body after the first half iteration
+};
+
+// ---- digits -------------------------------------------------------------------------
+// base-256 digits, most significant first, of v scaled so that |v| < 2^(8 L - 1)
+template <int L>
+__device__ __forceinline__ void digits_of(double v, double scale, float (&dg)[L])
+{
+    long long x = __double2ll_rn(v * scale);
+#pragma unroll
+    for (int i = L - 1; i > 0; --i) {
+        const int lo = (int)(signed char)(unsigned char)(x & 255);
+        dg[i] = (float)lo;
+        x = (x - lo) >> 8;
+    }
+    dg[0] = (float)(int)x;
+}
+
+// 2^k as a double, -1022 <= k <= 1023
+__device__ __forceinline__ double pow2(int k) { return __longlong_as_double((long long)(k + 1023) << 52); }
+
+// the power of two above a row's largest magnitude (its bits); false: not finite
+__device__ __forceinline__ bool row_exponent(long long maxbits, int &e)
+{
+    const int be = (int)(maxbits >> 52);
+    e = max(be, 122) - 1022;  // rows below 2^-900 count as zero
+    return be < 0x7ff;
+}
+
+__device__ __forceinline__ long long block_max(long long v)
+{
+    __shared__ long long sh[32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
+    if (lane == 0) sh[w] = v;
+    __syncthreads();
+    v = sh[lane < nw ? lane : 0];
+    for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+
+// A row of n values (value(m)) to digits: [chunk][digit][kKC], zero from n on to the end
+// of the last chunk.  A thread takes pairs of neighbours, NP of them, kept in registers
+// between the search for the largest and the splitting.  Returns the row's scale.
+template <int L, int NP, class Value>
+__device__ __forceinline__ double split_row(int n, int nch, __nv_bfloat16 *out, const Value &value)
+{
+    double v[2 * NP];
+    long long mx = 0;
+#pragma unroll
+    for (int q = 0; q < NP; ++q) {
+        const int m = 2 * (threadIdx.x + q * blockDim.x);
+        v[2 * q] = m < n ? value(m) : 0.0;
+        v[2 * q + 1] = m + 1 < n ? value(m + 1) : 0.0;
+    }
+#pragma unroll
+    for (int q = 0; q < 2 * NP; ++q) mx = max(mx, __double_as_longlong(fabs(v[q])));
+    mx = block_max(mx);
+    int e;
+    const bool finite = row_exponent(mx, e);
+    const double scale = finite ? pow2(8 * L - 1 - e) : 0.0;
+#pragma unroll
+    for (int q = 0; q < NP; ++q) {
+        const int m = 2 * (threadIdx.x + q * blockDim.x);
+        if (m >= nch * kKC) break;
+        float a[L], b[L];
+        digits_of<L>(finite ? v[2 * q] : 0.0, scale, a);
+        digits_of<L>(finite ? v[2 * q + 1] : 0.0, scale, b);
+        __nv_bfloat16 *o = out + (size_t)(m / kKC) * (L * kKC) + m % kKC;
+#pragma unroll
+        for (int i = 0; i < L; ++i)
+            *reinterpret_cast<__nv_bfloat162 *>(o + i * kKC) = __floats2bfloat162_rn(a[i], b[i]);
+    }
+    return finite ? pow2(e) : __longlong_as_double(0x7ff8000000000000ll);
+}
+
+// rows of a table: src[r ld_r + m ld_m], the scale of row r times 2^-50 and extra[r]
+template <int L, int NP>
+__global__ void k_sep_split_table(const double *__restrict__ src, int n, int nch, int ld_r, int ld_m,
+                                  const double *__restrict__ extra, __nv_bfloat16 *out, double *scale)
+{
+    const int r = blockIdx.x;
+    const double s = split_row<L, NP>(n, nch, out + (size_t)r * nch * L * kKC,
+                                      [&](int m) { return src[(size_t)r * ld_r + (size_t)m * ld_m]; });
+    if (threadIdx.x == 0) scale[r] = s * pow2(-50) * (extra ? extra[r] : 1.0);
+}
+
+__device__ __forceinline__ double block_sum(double v)
+{
+    __shared__ double sh[32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    __syncthreads();
+    if (lane == 0) sh[w] = v;
+    __syncthreads();
+    v = 0;
+    for (int k = 0; k < nw; ++k) v += sh[k];
+    return v;
+}
+
+// One grid row to digits, a block a row.  SPEC false: a field (times the scaling that
+// makes the transform orthonormal); true: z^, with the pinned cells' correction.  A row of
+// 922 is 7 values a thread: bound by one round of loads, the conversion and the stores.
+template <int L, int NP, bool SPEC>
+__global__ void __launch_bounds__(128) k_sep_split(SepDev d, const double *__restrict__ in)
+{
+    const int R = blockIdx.x, n = d.nm;
+    __nv_bfloat16 *out = d.A + (size_t)R * d.nch * L * kKC;
+    double s;
+    if (!SPEC) {
+        const double *row = in + (size_t)R * d.sr;
+        const double cr = d.cr ? d.cr[R] : 1.0;
+        s = split_row<L, NP>(n, d.nch, out, [&](int m) { return row[(size_t)m * d.sm] * (d.cm[m] * cr); });
+    } else {
+        // q = K^-1 (values of z at the pinned cells, mean of row 0), the same in every block
+        double f[3] = {0, 0, 0}, q[3] = {0, 0, 0};
+        for (int p = 0; p < d.pins; ++p) {
+            double v = 0;
+            const double *row = d.h + (size_t)d.R[p] * n;
+            for (int k = threadIdx.x; k < n; k += blockDim.x) v += d.F[p][k] * row[k];
+            f[p] = block_sum(v);
+        }
+        const int nq = d.pins + 1;
+        f[d.pins] = d.h[d.k0] * d.mean;
+        for (int a = 0; a < nq; ++a)
+            for (int b = 0; b < nq; ++b) q[a] += d.K[3 * a + b] * f[b];
+        const double qm = q[d.pins] * d.gm[R];
+        const double *row = d.h + (size_t)R * n;
+        const double *g0 = d.G[0] + (size_t)R * n, *g1 = d.pins > 1 ? d.G[1] + (size_t)R * n : nullptr;
+        s = split_row<L, NP>(n, d.nch, out, [&](int m) {
+            double v = row[m] - q[0] * g0[m];
+            if (g1) v -= q[1] * g1[m];
+            return m == d.k0 ? v + qm : v;
+        });
+    }
+    if (threadIdx.x == 0) d.sA[R] = s;
+}
+
+// ---- the dense product ------------------------------------------------------------------
+__device__ __forceinline__ void ldsm4(unsigned (&r)[4], unsigned addr)
+{
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(addr));
+}
+__device__ __forceinline__ void mma_bf16(float (&c)[4], const unsigned (&a)[4], unsigned b0, unsigned b1)
+{
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+                 "{%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void cp16(unsigned dst, const void *src)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src));
+}
+
+// out(M, N) = A(M, K) B(N, K)^T from digits, WM x WN warps of 16 x 16 outputs.  A stage in
+// shared memory is one chunk of the tile's rows of both factors, kKC terms of every digit;
+// a row is 64 L + 16 bytes there, an odd number of 16-byte units, so ldmatrix meets no
+// bank conflict.  A warp holds its L digit fragments of A and walks the digits of B: 2 L
+// ldmatrix for L (L + 1) mma.
+template <int L, int WM, int WN, int ST>
+__global__ void __launch_bounds__(32 * WM * WN, 2) k_sep_gemm(const __nv_bfloat16 *__restrict__ A,
+                                                          const double *__restrict__ sA, int M,
+                                                          const __nv_bfloat16 *__restrict__ B,
+                                                          const double *__restrict__ sB, int N, int nch,
+                                                          double *__restrict__ out, int so_m, int so_n)
+{
+    constexpr int TM = 16 * WM, TN = 16 * WN, T = 32 * WM * WN;
+    constexpr int RB = 64 * L + 16;                // bytes of a row in a stage
+    constexpr int STAGE = (TM + TN) * RB;
+    extern __shared__ __align__(16) unsigned char smem[];
+    const unsigned sbase = (unsigned)__cvta_generic_to_shared(smem);
+    const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int wm = warp / WN, wn = warp % WN;
+    const size_t rowBytes = (size_t)nch * L * kKC * 2;
+
+    auto load = [&](int ch) {
+        const unsigned s = sbase + (ch % ST) * STAGE;
+        constexpr int U = 4 * L;  // 16-byte units of a row and chunk
+        for (int u = threadIdx.x; u < (TM + TN) * U; u += T) {
+            const int row = u / U, k = u - row * U;
+            const char *g = row < TM
+                                ? reinterpret_cast<const char *>(A) + (size_t)min(m0 + row, M - 1) * rowBytes
+                                : reinterpret_cast<const char *>(B) + (size_t)min(n0 + row - TM, N - 1) * rowBytes;
+            cp16(s + row * RB + k * 16, g + (size_t)ch * U * 16 + k * 16);
+        }
+    };
+
+    float acc[L][2][4];
+    long long tot[2][4];
+#pragma unroll
+    for (int t = 0; t < 2; ++t)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) tot[t][q] = 0;
+#pragma unroll
+    for (int d = 0; d < L; ++d)
+#pragma unroll
+        for (int t = 0; t < 2; ++t)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) acc[d][t][q] = 0.f;
+
+    for (int s = 0; s < ST - 1; ++s) {
+        if (s < nch) load(s);
+        asm volatile("cp.async.commit_group;");
+    }
+    const unsigned offA = (wm * 16 + (lane & 15)) * RB + (lane >> 4) * 16;
+    const unsigned offB = (TM + wn * 16 + (lane & 7) + ((lane >> 4) << 3)) * RB + ((lane >> 3) & 1) * 16;
+    for (int ch = 0; ch < nch; ++ch) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(ST - 2));
+        __syncthreads();
+        if (ch + ST - 1 < nch) load(ch + ST - 1);
+        asm volatile("cp.async.commit_group;");
+        const unsigned s = sbase + (ch % ST) * STAGE;
+#pragma unroll
+        for (int ks = 0; ks < 2; ++ks) {
+            unsigned a[L][4];
+#pragma unroll
+            for (int i = 0; i < L; ++i) ldsm4(a[i], s + offA + i * 64 + ks * 32);
+#pragma unroll
+            for (int j = 0; j < L; ++j) {
+                unsigned b[4];
+                ldsm4(b, s + offB + j * 64 + ks * 32);
+#pragma unroll
+                for (int i = 0; i < L - j; ++i) {
+                    mma_bf16(acc[i + j][0], a[i], b[0], b[1]);
+                    mma_bf16(acc[i + j][1], a[i], b[2], b[3]);
+                }
+            }
+        }
+        if ((ch % kFlush) == kFlush - 1 || ch == nch - 1) {
+            // whole numbers below 2^24: into units of 2^-36 of the leading digits' product
+#pragma unroll
+            for (int d = 0; d < L; ++d)
+#pragma unroll
+                for (int t = 0; t < 2; ++t)
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const int w = __float2int_rn(acc[d][t][q]);
+                        acc[d][t][q] = 0.f;
+                        const int sh = 36 - 8 * d;
+                        if (sh >= 0) tot[t][q] += (long long)w * (1ll << (sh >= 0 ? sh : 0));
+                        else tot[t][q] += (w + (1 << (-sh - 1 > 0 ? -sh - 1 : 0))) >> (sh < 0 ? -sh : 0);
+                    }
+        }
+    }
+    const int r0 = m0 + wm * 16 + (lane >> 2), c0 = n0 + wn * 16 + (lane & 3) * 2;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int r = r0 + (q >> 1) * 8;
+        if (r >= M) continue;
+        const double sa = sA[r];
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+            const int col = c0 + t * 8 + (q & 1);
+            if (col < N) out[(size_t)r * so_m + (size_t)col * so_n] = (double)tot[t][q] * (sa * sB[col]);
+        }
+    }
+}
+
+// ---- the tridiagonal solves -----------------------------------------------------------------
+// A block solves CB modes; kTriThreads / CB threads share a mode's rows, m = ceil(nr / that)
+// neighbouring rows each.  Forward d_J = r_J + l_J d_J-1 and backward x_J = inv_J d_J + c_J
+// x_J+1 are linear recurrences: each thread runs its rows from zero, the threads' ends are
+// joined by a scan of affine maps in shared memory (the factors' products over a thread's
+// rows are tables), and each thread runs its rows again from the true start.  922 rows in
+// sequence would be 1844 dependent FP64 operations; this way it is 4 x 15 and two scans of
+// 6 steps.
+template <int CB>
+__device__ __forceinline__ double tri_scan(double end, double prod, bool up, double *se, double *sp)
+{
+    // inclusive scan over q of x -> end + prod x, from q = 0 up or from the last down;
+    // returns the value that enters this thread's rows
+    constexpr int NQ = kTriThreads / CB;
+    const int tid = threadIdx.x, q = up ? tid / CB : NQ - 1 - tid / CB, step = up ? CB : -CB;
+    int cur = 0;
+    se[tid] = end;
+    sp[tid] = prod;
+    __syncthreads();
+#pragma unroll
+    for (int o = 1; o < NQ; o <<= 1) {
+        const double *e = se + cur * kTriThreads, *p = sp + cur * kTriThreads;
+        double *en = se + (cur ^ 1) * kTriThreads, *pn = sp + (cur ^ 1) * kTriThreads;
+        double ee = e[tid], pp = p[tid];
+        if (q >= o) {
+            const int from = tid - o * step;
+            ee += pp * e[from];
+            pp *= p[from];
+        }
+        en[tid] = ee;
+        pn[tid] = pp;
+        cur ^= 1;
+        __syncthreads();
+    }
+    const double in = q > 0 ? se[cur * kTriThreads + tid - step] : 0.0;
+    __syncthreads();
+    return in;
+}
+
+template <int CB>
+__global__ void __launch_bounds__(kTriThreads) k_sep_tri(SepDev d)
+{
+    constexpr int NQ = kTriThreads / CB;
+    extern __shared__ double row[];  // [m][thread]: r, then inv d
+    __shared__ double se[2 * kTriThreads], sp[2 * kTriThreads];
+    const int tid = threadIdx.x, n = d.nm;
+    const int k = blockIdx.x * CB + tid % CB, q = tid / CB, m = (d.nr + NQ - 1) / NQ;
+    const int J0 = min(q * m, d.nr), J1 = min(J0 + m, d.nr), cnt = k < n ? J1 - J0 : 0;
+    const size_t at = (size_t)J0 * n + k;
+    double x = 0;
+#pragma unroll 4
+    for (int t = 0; t < cnt; ++t) {
+        const double r = d.h[at + (size_t)t * n];
+        row[t * kTriThreads + tid] = r;
+        x = r + d.l[at + (size_t)t * n] * x;
+    }
+    x = tri_scan<CB>(x, k < n ? d.Pf[(size_t)q * n + k] : 0.0, true, se, sp);
+#pragma unroll 4
+    for (int t = 0; t < cnt; ++t) {
+        x = row[t * kTriThreads + tid] + d.l[at + (size_t)t * n] * x;
+        row[t * kTriThreads + tid] = x * d.inv[at + (size_t)t * n];
+    }
+    x = 0;
+#pragma unroll 4
+    for (int t = cnt - 1; t >= 0; --t) x = row[t * kTriThreads + tid] + d.c[at + (size_t)t * n] * x;
+    x = tri_scan<CB>(x, k < n ? d.Pb[(size_t)q * n + k] : 0.0, false, se, sp);
+#pragma unroll 4
+    for (int t = cnt - 1; t >= 0; --t) {
+        x = row[t * kTriThreads + tid] + d.c[at + (size_t)t * n] * x;
+        d.h[at + (size_t)t * n] = x;
+    }
+}
+
+// Wide blocks of modes (whole 64-byte segments) where enough of them fill the GPU and their
+// rows fit shared memory; kTriRows rows are what 4 modes a block can hold
+constexpr int kTriRows = 6400;
+static int tri_modes(int nm, int nr) { return nm >= 600 && nr <= kTriRows / 2 ? 8 : 4; }
+
+// the factors of Y + lambda_k, one thread a mode, and their products over each thread's
+// rows of k_sep_tri; the constant's mode gets reg on its first diagonal
+__global__ void k_sep_factor(int nm, int nr, int nq, const double *__restrict__ up, const double *__restrict__ dn,
+                             const double *__restrict__ lam, int k0, double reg, double *l, double *c, double *inv,
+                             double *Pf, double *Pb)
+{
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= nm) return;
+    double prev = 0;
+    for (int J = 0; J < nr; ++J) {
+        double dg = up[J] + dn[J] + lam[k];
+        if (k == k0 && J == 0) dg += reg;
+        const double lj = J ? dn[J] * prev : 0.0;
+        if (J) dg -= lj * up[J - 1];
+        prev = 1.0 / dg;
+        const size_t at = (size_t)J * nm + k;
+        l[at] = lj;
+        inv[at] = prev;
+        c[at] = J + 1 < nr ? up[J] * prev : 0.0;
+    }
+    const int m = (nr + nq - 1) / nq;
+    for (int q = 0; q < nq; ++q) {
+        double pf = 1, pb = 1;
+        for (int J = q * m; J < min((q + 1) * m, nr); ++J) {
+            pf *= l[(size_t)J * nm + k];
+            pb *= c[(size_t)J * nm + k];
+        }
+        Pf[(size_t)q * nm + k] = pf;
+        Pb[(size_t)q * nm + k] = pb;
+    }
+}
+
+// Q from the QR iteration's rotations: thread i holds row i of Q in shared memory (element
+// j at [j][thread]) and applies every rotation to it in order; a rotation changes elements
+// j and j + 1, ascending in a sweep, so one value is carried in a register
+struct Sweep {
+    int first, count;
+    long long at;
+};
+__global__ void k_sep_rotate(int n, const Sweep *__restrict__ sw, int nsw, const double2 *__restrict__ rot,
+                             double *__restrict__ Q)
+{
+    extern __shared__ double z[];
+    __shared__ double2 cs[64];
+    const int W = blockDim.x, t = threadIdx.x, i = blockIdx.x * W + t;
+    for (int j = 0; j < n; ++j) z[j * W + t] = j == i ? 1.0 : 0.0;
+    for (int s = 0; s < nsw; ++s) {
+        const Sweep S = sw[s];
+        double a = z[S.first * W + t];
+        for (int b0 = 0; b0 < S.count; b0 += 64) {
+            const int nb = min(64, S.count - b0);
+            __syncthreads();
+            for (int b = t; b < nb; b += W) cs[b] = rot[S.at + b0 + b];
+            __syncthreads();
+#pragma unroll 4
+            for (int b = 0; b < nb; ++b) {
+                const double2 r = cs[b];
+                const int j = S.first + b0 + b;
+                const double v = z[(j + 1) * W + t];
+                z[j * W + t] = r.x * a + r.y * v;
+                a = r.x * v - r.y * a;
+            }
+        }
+        z[(S.first + S.count) * W + t] = a;
+    }
+    if (i < n)
+        for (int j = 0; j < n; ++j) Q[(size_t)i * n + j] = z[j * W + t];
+}
+
+// column k0 of Q: the constant in exact form
+__global__ void k_sep_constant(int n, int k0, const double *__restrict__ v, double *Q)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) Q[(size_t)i * n + k0] = v[i];
+}
+
+// ---- Krylov kernels ---------------------------------------------------------------------
+// BiCGSTAB as in krylov.cu with two differences: the first half iteration takes r for its
+// shadow residual and direction (they are copies then), and x takes alpha M p in the half
+// step, so that a solve that ends there - the usual end - needs nothing more.
+template <class Op>
+__global__ void __launch_bounds__(256) k_sep_init(Op A, int n, const double *__restrict__ b, const double *x, double *r,
+                                                  double *partials, KrylovScalars *ks, int *err, int which)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    double v[2] = {0, 0}, t[2];
+    if (i < n) {
+        const double bi = b[i], ri = bi - A.row(i, PtrAccess{x});
+        r[i] = ri;
+        v[0] = ri * ri;
+        v[1] = bi * bi;
+    }
+    if (reduce_arrive<2>(v, partials, &ks->arrive, t) && threadIdx.x == 0) {
+        ks->rho = t[0];
+        ks->rnorm = sqrt(t[0]);
+        ks->bnorm = sqrt(t[1]);
+        ks->tol = ks->rtol * ks->bnorm;
+        ks->it = 0;
+        ks->s_done = 0;
+        ks->body_runs = 0;
+        ks->status = KS_RUNNING;
+        finish_status(ks, err, which);
+    }
+}
+
+template <class Op>
+__global__ void __launch_bounds__(256) k_sep_1(Op A, int n, const double *__restrict__ Mp, double *AMp,
+                                               const double *__restrict__ rs, double *partials, KrylovScalars *ks,
+                                               int first)
+{
+    if (ks->status != KS_RUNNING) return;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    double v[1] = {0}, t[1];
+    if (i < n) {
+        const double a = A.row(i, PtrAccess{Mp});
+        AMp[i] = a;
+        v[0] = rs[i] * a;
+    }
+    if (reduce_arrive<1>(v, partials, &ks->arrive, t) && threadIdx.x == 0) {
+        ks->alpha = ks->rho / t[0];
+        ks->s_done = 0;
+        if (!first) ks->body_runs += 1;
+    }
+}
+
+__global__ void __launch_bounds__(256) k_sep_2(int n, const double *__restrict__ r, const double *__restrict__ AMp,
+                                               const double *__restrict__ Mp, double *s, double *x, double *partials,
+                                               KrylovScalars *ks, int first, cudaGraphConditionalHandle h, int use_cond)
+{
+    if (ks->status != KS_RUNNING) return;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const double alpha = ks->alpha;
+    double v[1] = {0}, t[1];
+    if (i < n) {
+        const double si = r[i] - alpha * AMp[i];
+        s[i] = si;
+        x[i] += alpha * Mp[i];
+        v[0] = si * si;
+    }
+    if (reduce_arrive<1>(v, partials, &ks->arrive, t) && threadIdx.x == 0) {
+        ks->snorm = sqrt(t[0]);
+        if (ks->snorm <= ks->tol) {
+            ks->s_done = 1;
+            ks->rnorm = ks->snorm;
+            ks->status = KS_CONVERGED;
+        } else if (first) {
+            ks->body_runs = 1;
+        }
+        set_cond(h, use_cond, ks->status == KS_RUNNING);
+    }
+}
+
+template <class Op>
+__global__ void __launch_bounds__(256) k_sep_3(Op A, int n, const double *__restrict__ s,
+                                               const double *__restrict__ Ms, double *AMs, double *partials,
+                                               KrylovScalars *ks)
+{
+    if (ks->status != KS_RUNNING) return;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    double v[2] = {0, 0}, t[2];
+    if (i < n) {
+        const double a = A.row(i, PtrAccess{Ms});
+        AMs[i] = a;
+        v[0] = a * s[i];
+        v[1] = a * a;
+    }
+    if (reduce_arrive<2>(v, partials, &ks->arrive, t) && threadIdx.x == 0) ks->omega = t[0] / t[1];
+}
+
+// x += omega M s, r = s - omega A M s; the first time also rs = p = the residual the solve began with
+__global__ void __launch_bounds__(256) k_sep_4(int n, double *x, double *r, double *rs, double *p,
+                                               const double *__restrict__ s, const double *__restrict__ Ms,
+                                               const double *__restrict__ AMs, double *partials, KrylovScalars *ks,
+                                               int *err, int which, int first, cudaGraphConditionalHandle h,
+                                               int use_cond)
+{
+    if (ks->status != KS_RUNNING) return;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const double omega = ks->omega;
+    double v[2] = {0, 0}, t[2];
+    if (i < n) {
+        const double r0 = first ? r[i] : rs[i];
+        if (first) {
+            rs[i] = r0;
+            p[i] = r0;
+        }
+        x[i] += omega * Ms[i];
+        const double ri = s[i] - omega * AMs[i];
+        r[i] = ri;
+        v[0] = r0 * ri;
+        v[1] = ri * ri;
+    }
+    if (reduce_arrive<2>(v, partials, &ks->arrive, t) && threadIdx.x == 0) {
+        ks->beta = (t[0] / ks->rho) * (ks->alpha / omega);
+        ks->rho = t[0];
+        ks->it += 1;
+        ks->rnorm = sqrt(t[1]);
+        finish_status(ks, err, which);
+        set_cond(h, use_cond, ks->status == KS_RUNNING);
+    }
+}
+
+// CG's first iteration: p = z, q = A z, rho = r . z, alpha = rho / (z . q)
+template <class Op>
+__global__ void __launch_bounds__(256) k_sep_cg_1(Op A, int n, const double *__restrict__ r,
+                                                  const double *__restrict__ z, double *p, double *q,
+                                                  double *partials, KrylovScalars *ks)
+{
+    if (ks->status != KS_RUNNING) return;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    double v[2] = {0, 0}, t[2];
+    if (i < n) {
+        const double zi = z[i], qi = A.row(i, PtrAccess{z});
+        p[i] = zi;
+        q[i] = qi;
+        v[0] = r[i] * zi;
+        v[1] = zi * qi;
+    }
+    if (reduce_arrive<2>(v, partials, &ks->arrive, t) && threadIdx.x == 0) {
+        ks->rho = t[0];
+        ks->alpha = t[0] / t[1];
+    }
+}
+
+// ---- host side: set-up ------------------------------------------------------------------
+namespace {
+
+// Eigenvalues (d, on return) of the symmetric tridiagonal matrix with diagonal d and
+// off-diagonal e, by implicitly shifted QR sweeps; the rotations of every sweep are
+// recorded in order (element j and j + 1 of a row vector take c, s: [c a + s b, c b - s a]).
+// False: no convergence (non-finite entries).
+bool tridiagonal_qr(std::vector<double> &d, std::vector<double> e, std::vector<Sweep> &sweeps,
+                    std::vector<double2> &rot)
+{
+    const int n = (int)d.size();
+    const double eps = 2.220446049250313e-16;
+    int hi = n - 1;
+    for (long guard = 0; hi > 0; ++guard) {
+        if (guard > 60L * n) return false;
+        auto small = [&](int k) { return std::fabs(e[k]) <= eps * (std::fabs(d[k]) + std::fabs(d[k + 1])); };
+        if (small(hi - 1)) {
+            e[--hi] = 0;
+            continue;
+        }
+        int lo = hi - 1;
+        while (lo > 0 && !small(lo - 1)) --lo;
+        // Wilkinson's shift: the eigenvalue of the trailing 2 x 2 block nearer its last entry
+        const double g = 0.5 * (d[hi - 1] - d[hi]), b = e[hi - 1];
+        const double mu = d[hi] - b * (b / (g + std::copysign(std::hypot(g, b), g)));
+        if (!std::isfinite(mu)) return false;
+        sweeps.push_back({lo, hi - lo, (long long)rot.size()});
+        double x = d[lo] - mu, z = e[lo];
+        for (int k = lo; k < hi; ++k) {
+            const double r = std::sqrt(x * x + z * z);
+            const double cc = r > 0 ? x / r : 1.0, ss = r > 0 ? z / r : 0.0;
+            if (k > lo) e[k - 1] = r;
+            const double a = d[k], w = d[k + 1], f = e[k];
+            const double t = cc * ss * f * 2;
+            d[k] = cc * cc * a + t + ss * ss * w;
+            d[k + 1] = ss * ss * a - t + cc * cc * w;
+            e[k] = cc * ss * (w - a) + (cc * cc - ss * ss) * f;
+            if (k + 1 < hi) {
+                x = e[k];
+                z = ss * e[k + 1];
+                e[k + 1] *= cc;
+            }
+            rot.push_back(make_double2(cc, ss));
+        }
+    }
+    return true;
+}
+
+// the inverse of the leading n x n block (n <= 3) of K, rows of 3, by elimination with pivoting
+bool invert3(double *K, int n)
+{
+    double a[3][6] = {};
+    for (int i = 0; i < n; ++i) {
+        for (int j = 0; j < n; ++j) a[i][j] = K[3 * i + j];
+        a[i][n + i] = 1;
+    }
+    for (int k = 0; k < n; ++k) {
+        int p = k;
+        for (int i = k + 1; i < n; ++i)
+            if (std::fabs(a[i][k]) > std::fabs(a[p][k])) p = i;
+        if (!(std::fabs(a[p][k]) > 0)) return false;
+        for (int j = 0; j < 2 * n; ++j) std::swap(a[k][j], a[p][j]);
+        const double s = 1 / a[k][k];
+        for (int j = 0; j < 2 * n; ++j) a[k][j] *= s;
+        for (int i = 0; i < n; ++i)
+            if (i != k) {
+                const double f = a[i][k];
+                for (int j = 0; j < 2 * n; ++j) a[i][j] -= f * a[k][j];
+            }
+    }
+    for (int i = 0; i < n; ++i)
+        for (int j = 0; j < n; ++j) K[3 * i + j] = a[i][n + j];
+    return true;
+}
+
+}  // namespace
+
+template <int L, int WM, int WN, int ST>
+static void launch_gemm_t(Context &c, const __nv_bfloat16 *A, const double *sA, int M, const __nv_bfloat16 *B,
+                          const double *sB, int N, int nch, double *out, int so_m, int so_n)
+{
+    constexpr int smem = ST * 16 * (WM + WN) * (64 * L + 16);
+    const dim3 grid((N + 16 * WN - 1) / (16 * WN), (M + 16 * WM - 1) / (16 * WM));
+    k_sep_gemm<L, WM, WN, ST><<<grid, 32 * WM * WN, smem, c.stream>>>(A, sA, M, B, sB, N, nch, out, so_m, so_n);
+    CUIBM_TRY(cudaGetLastError());
+}
+
+template <class K>
+static void allow_smem(K *fn, size_t bytes)
+{
+    CUIBM_TRY(cudaFuncSetAttribute(reinterpret_cast<const void *>(fn), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)bytes));
+}
+
+// once per context (set-up): dynamic shared memory above 48 KB
+template <int L>
+static void allow_gemm()
+{
+    allow_smem(k_sep_gemm<L, 2, 2, 3>, 3 * 16 * 4 * (64 * L + 16));
+    allow_smem(k_sep_gemm<L, 2, 4, 2>, 2 * 16 * 6 * (64 * L + 16));
+}
+
+// Tiles of 32 x 64 (two blocks an SM) where there are enough of them for every SM, else 32
+// x 32: a 270 x 270 product is 81 small tiles or 45 large ones on 152 SMs
+template <int L>
+static void launch_gemm(Context &c, const SepPlan &P, const __nv_bfloat16 *B, const double *sB, double *out, int so_m,
+                        int so_n)
+{
+    const SepDev &d = P.d;
+    const int large = ((d.nr + 31) / 32) * ((d.nm + 63) / 64);
+    if (large >= 152)
+        launch_gemm_t<L, 2, 4, 2>(c, d.A, d.sA, d.nr, B, sB, d.nm, d.nch, out, so_m, so_n);
+    else
+        launch_gemm_t<L, 2, 2, 3>(c, d.A, d.sA, d.nr, B, sB, d.nm, d.nch, out, so_m, so_n);
+}
+
+template <int L, bool SPEC>
+static void launch_split(Context &c, const SepPlan &P, const double *in)
+{
+    const SepDev &d = P.d;
+    const int n = d.nch * kKC;
+    if (n <= 256) k_sep_split<L, 1, SPEC><<<d.nr, 128, 0, c.stream>>>(d, in);
+    else if (n <= 512) k_sep_split<L, 2, SPEC><<<d.nr, 128, 0, c.stream>>>(d, in);
+    else if (n <= 1024) k_sep_split<L, 4, SPEC><<<d.nr, 128, 0, c.stream>>>(d, in);
+    else k_sep_split<L, 8, SPEC><<<d.nr, 128, 0, c.stream>>>(d, in);
+    CUIBM_TRY(cudaGetLastError());
+}
+
+template <int L>
+static void split_table(Context &c, const double *src, int rows, int n, int nch, int ld_r, int ld_m,
+                        const double *extra, __nv_bfloat16 *out, double *scale)
+{
+    if (nch * kKC <= 512)
+        k_sep_split_table<L, 2><<<rows, 128, 0, c.stream>>>(src, n, nch, ld_r, ld_m, extra, out, scale);
+    else
+        k_sep_split_table<L, 8><<<rows, 128, 0, c.stream>>>(src, n, nch, ld_r, ld_m, extra, out, scale);
+    CUIBM_TRY(cudaGetLastError());
+}
+
+static void launch_tri(Context &c, const SepPlan &P)
+{
+    const SepDev &d = P.d;
+    const int cb = tri_modes(d.nm, d.nr), nq = kTriThreads / cb, m = (d.nr + nq - 1) / nq;
+    const size_t smem = (size_t)m * kTriThreads * sizeof(double);
+    const int nb = (d.nm + cb - 1) / cb;
+    if (cb == 8) k_sep_tri<8><<<nb, kTriThreads, smem, c.stream>>>(d);
+    else k_sep_tri<4><<<nb, kTriThreads, smem, c.stream>>>(d);
+    CUIBM_TRY(cudaGetLastError());
+}
+
+template <int L>
+static void apply_t(Context &c, const SepPlan &P, const double *in, double *out)
+{
+    const SepDev &d = P.d;
+    launch_split<L, false>(c, P, in);
+    launch_gemm<L>(c, P, d.B1, d.sB1, d.h, d.nm, 1);
+    launch_tri(c, P);
+    launch_split<L, true>(c, P, nullptr);
+    launch_gemm<L>(c, P, d.B2, d.sB2, out, d.sr, d.sm);
+}
+
+// out = M in: five kernels
+void launch_separable_apply(Context &c, LinearSystem &S, const double *in, double *out)
+{
+    const SepPlan &P = *static_cast<const SepPlan *>(S.sep);
+    if (P.digits == kDigits) apply_t<kDigits>(c, P, in, out);
+    else apply_t<kDigitsMixed>(c, P, in, out);
+}
+
+// Where the separable preconditioner takes the place of the smoothed-aggregation cycle: the
+// pressure system of the methods that leave its rows alone, unless the case asks for a form
+// of smoothed aggregation by name (-saStructured 0 or 1, strengthThreshold, -separable 0).
+// By itself (-separable -1) not where the pressure's level would move by more than 1e-9 of
+// it: with the external method one pinned cell in the domain's corner fixes the level, and
+// the smoothed-aggregation solves leave their stopping error in it (against a solve to
+// 1e-15: 1e-10 to 1e-7 of p at a relative residual of 1e-13 from 200k unknowns on, 1e-9 in
+// mixed precision and in batches at 1e-12, below 3e-10 elsewhere; the separable solves
+// 1e-11), so runs there keep the solver that they began with.  With the plain method the
+// centre cell is pinned too and the level agrees to 1e-12.
+constexpr int kLevelMax = 200000;
+
+static bool separable_applies(const Context &c, const LinearSystem &S)
+{
+    const int nx = c.g.nx, ny = c.g.ny;
+    const bool fits = S.which == 2 && S.precond == PC_SMOOTHED_AGGREGATION && c.P.saStructured == -1 &&
+                      c.P.poisson.strength < 0 &&
+                      (c.P.solverType == ST_NAVIERSTOKES || c.P.solverType == ST_LUO) &&
+                      std::min(nx, ny) <= kSepMax && std::max(nx, ny) <= kTriRows;
+    if (!fits || c.P.separable >= 0) return fits && c.P.separable == 1;
+    return c.P.solverType == ST_NAVIERSTOKES ||
+           (S.n < kLevelMax && S.precision == PRECISION_FP64 && c.P.solverPack != 2);
+}
+
+void setup_separable(Context &c, LinearSystem &S)
+{
+    S.sep = nullptr;
+    if (!separable_applies(c, S)) return;
+    const int nx = c.g.nx, ny = c.g.ny;
+    const bool alongx = nx <= ny;  // the shorter direction is transformed: n_m^2 n_r work
+    SepPlan *P = new SepPlan();
+    S.sep = P;
+    SepDev &d = P->d;
+    P->digits = S.precision == PRECISION_MIXED ? kDigitsMixed : kDigits;
+    const int L = P->digits, nm = alongx ? nx : ny, nr = alongx ? ny : nx;
+    d.nm = nm;
+    d.nr = nr;
+    d.sm = alongx ? 1 : nx;
+    d.sr = alongx ? nx : 1;
+    d.nch = (nm + kKC - 1) / kKC;
+    const double *t = c.htab.data();
+    auto tab = [&](const char *k, int n) { return std::vector<double>(t + c.hoff.at(k), t + c.hoff.at(k) + n); };
+    const std::vector<double> &wm = alongx ? c.gx.width : c.gy.width, &wr = alongx ? c.gy.width : c.gx.width;
+    const std::vector<double> um = tab(alongx ? "2E" : "2N", nm), dm = tab(alongx ? "2W" : "2S", nm);
+    const std::vector<double> ur = tab(alongx ? "2N" : "2E", nr), dr = tab(alongx ? "2S" : "2W", nr);
+
+    // eigenvalues of D^1/2 X D^-1/2 and the rotations that give its eigenvectors
+    std::vector<double> lam(nm), off(nm, 0.0);
+    for (int i = 0; i < nm; ++i) lam[i] = um[i] + dm[i];
+    for (int i = 0; i + 1 < nm; ++i) off[i] = -std::sqrt(um[i] * dm[i + 1]);
+    std::vector<Sweep> sweeps;
+    std::vector<double2> rot;
+    if (!tridiagonal_qr(lam, off, sweeps, rot)) {  // not a grid this can be built on
+        free_separable(S);
+        return;
+    }
+    const int k0 = (int)(std::min_element(lam.begin(), lam.end()) - lam.begin());
+    lam[k0] = 0;  // the constant: exactly the null vector of X
+    double len = 0;
+    for (double w : wm) len += w;
+    std::vector<double> cm(nm), cr(nr), em(nm), con(nm);
+    const bool sym = S.w != nullptr;  // CG: the system's rows carry the cell areas
+    for (int i = 0; i < nm; ++i) {
+        cm[i] = sym ? 1 / std::sqrt(wm[i]) : std::sqrt(wm[i]);
+        em[i] = 1 / std::sqrt(wm[i]);
+        con[i] = std::sqrt(wm[i] / len);
+    }
+    for (int J = 0; J < nr; ++J) cr[J] = sym ? 1 / wr[J] : 1.0;
+
+    // one allocation for all tables and work arrays
+    const int cb = tri_modes(nm, nr), nq = kTriThreads / cb;
+    const size_t n = (size_t)nm * nr, dig = (size_t)d.nch * L * kKC;
+    size_t need = 0;
+    auto reserve = [&](size_t bytes) {
+        const size_t at = need;
+        need += (bytes + 255) & ~size_t(255);
+        return at;
+    };
+    const size_t oB1 = reserve(nm * dig * 2), oB2 = reserve(nm * dig * 2), oA = reserve(nr * dig * 2);
+    const size_t osB1 = reserve(nm * 8), osB2 = reserve(nm * 8), osA = reserve(nr * 8);
+    const size_t oh = reserve(n * 8), ol = reserve(n * 8), oc = reserve(n * 8), oi = reserve(n * 8);
+    const size_t oPf = reserve((size_t)nq * nm * 8), oPb = reserve((size_t)nq * nm * 8);
+    const size_t ocm = reserve(nm * 8), ocr = reserve(nr * 8), oF0 = reserve(nm * 8), oF1 = reserve(nm * 8);
+    const size_t oG0 = reserve(n * 8), oG1 = reserve(c.l2.pinc >= 0 ? n * 8 : 8), ogm = reserve(nr * 8);
+    CUIBM_TRY(cudaMalloc(&P->block, need));
+    auto D = [&](size_t at) { return reinterpret_cast<double *>(P->block + at); };
+    auto H = [&](size_t at) { return reinterpret_cast<__nv_bfloat16 *>(P->block + at); };
+    auto put = [&](double *dst, const std::vector<double> &v) {
+        CUIBM_TRY(cudaMemcpyAsync(dst, v.data(), v.size() * 8, cudaMemcpyHostToDevice, c.stream));
+    };
+    // set-up scratch, freed at the end
+    char *tmp = nullptr;
+    const size_t bq = ((size_t)nm * nm * 8 + 255) & ~size_t(255), bs = (sweeps.size() * sizeof(Sweep) + 511) & ~size_t(255),
+                 br = (rot.size() * sizeof(double2) + 511) & ~size_t(255), bv = (size_t)(4 * nm + 4 * nr) * 8;
+    CUIBM_TRY(cudaMalloc(&tmp, bq + bs + br + bv));
+    struct Freed {
+        char *p;
+        ~Freed() { cudaFree(p); }
+    } freed{tmp};
+    double *Q = reinterpret_cast<double *>(tmp);
+    Sweep *sw = reinterpret_cast<Sweep *>(tmp + bq);
+    double2 *rt = reinterpret_cast<double2 *>(tmp + bq + bs);
+    double *vl = reinterpret_cast<double *>(tmp + bq + bs + br), *vcon = vl + nm, *vem = vcon + nm, *vur = vem + nm,
+           *vdr = vur + nr;
+    CUIBM_TRY(cudaMemcpyAsync(sw, sweeps.data(), sweeps.size() * sizeof(Sweep), cudaMemcpyHostToDevice, c.stream));
+    CUIBM_TRY(cudaMemcpyAsync(rt, rot.data(), rot.size() * sizeof(double2), cudaMemcpyHostToDevice, c.stream));
+    put(vl, lam);
+    put(vcon, con);
+    put(vem, em);
+    put(vur, ur);
+    put(vdr, dr);
+    put(D(ocm), cm);
+    put(D(ocr), cr);
+    // rows of Q a block: as many as shared memory holds, a warp at most
+    int W = 32;
+    while (W > 4 && (size_t)nm * W * 8 > 200 * 1024) W /= 2;
+    allow_smem(k_sep_rotate, (size_t)nm * W * 8);
+    k_sep_rotate<<<(nm + W - 1) / W, W, (size_t)nm * W * 8, c.stream>>>(nm, sw, (int)sweeps.size(), rt, Q);
+    k_sep_constant<<<blocks_for(nm), kBlock, 0, c.stream>>>(nm, k0, vcon, Q);
+    CUIBM_TRY(cudaGetLastError());
+    if (L == kDigits) {
+        allow_gemm<kDigits>();
+        split_table<kDigits>(c, Q, nm, nm, d.nch, 1, nm, nullptr, H(oB1), D(osB1));
+        split_table<kDigits>(c, Q, nm, nm, d.nch, nm, 1, vem, H(oB2), D(osB2));
+    } else {
+        allow_gemm<kDigitsMixed>();
+        split_table<kDigitsMixed>(c, Q, nm, nm, d.nch, 1, nm, nullptr, H(oB1), D(osB1));
+        split_table<kDigitsMixed>(c, Q, nm, nm, d.nch, nm, 1, vem, H(oB2), D(osB2));
+    }
+    allow_smem(k_sep_tri<8>, 200 * 1024);
+    allow_smem(k_sep_tri<4>, 200 * 1024);
+    const double reg = ur[0];
+    k_sep_factor<<<(nm + 31) / 32, 32, 0, c.stream>>>(nm, nr, nq, vur, vdr, vl, k0, reg, D(ol), D(oc), D(oi), D(oPf),
+                                                      D(oPb));
+    CUIBM_TRY(cudaGetLastError());
+    d.B1 = H(oB1);
+    d.B2 = H(oB2);
+    d.A = H(oA);
+    d.sB1 = D(osB1);
+    d.sB2 = D(osB2);
+    d.sA = D(osA);
+    d.h = D(oh);
+    d.l = D(ol);
+    d.c = D(oc);
+    d.inv = D(oi);
+    d.Pf = D(oPf);
+    d.Pb = D(oPb);
+    d.cm = D(ocm);
+    d.cr = sym ? D(ocr) : nullptr;
+    d.k0 = k0;
+    d.mean = 1 / std::sqrt(len);
+    d.gm = D(ogm);
+
+    // Pinned cells and the constant.  With B = A0 plus reg on the constant's mode in row 0,
+    // A = B + sum_p delta_p e_p e_p^T - reg u mean^T (u one on row 0, mean the average over
+    // it), so z = B^-1 r - sum_p q_p G_p + q_m G_m with q_p = delta_p z_p, q_m = reg mean(z)
+    std::vector<int> cell{c.l2.pin0};
+    if (c.l2.pinc >= 0) cell.push_back(c.l2.pinc);
+    d.pins = (int)cell.size();
+    std::vector<std::vector<double>> F(3, std::vector<double>(nm)), G0, q(nm);
+    std::vector<double> qrow(nm), resp((size_t)nm);
+    double *Gp[2] = {D(oG0), D(oG1)}, *Fp[2] = {D(oF0), D(oF1)};
+    int Rp[2] = {0, 0};
+    double delta[2] = {0, 0};
+    std::vector<std::vector<double>> at_pin(3, std::vector<double>(3, 0.0));  // functional a of response b
+    for (int p = 0; p < d.pins; ++p) {
+        const int I = cell[p] % nx, J = cell[p] / nx, m = alongx ? I : J;
+        Rp[p] = alongx ? J : I;
+        delta[p] = um[m] + dm[m] + ur[Rp[p]] + dr[Rp[p]];
+        CUIBM_TRY(cudaMemcpyAsync(qrow.data(), Q + (size_t)m * nm, nm * 8, cudaMemcpyDeviceToHost, c.stream));
+        CUIBM_TRY(cudaStreamSynchronize(c.stream));
+        std::vector<double> rhs(nm);
+        for (int k = 0; k < nm; ++k) {
+            rhs[k] = qrow[k] * std::sqrt(wm[m]);
+            F[p][k] = qrow[k] * em[m];
+        }
+        put(Fp[p], F[p]);
+        CUIBM_TRY(cudaMemsetAsync(d.h, 0, n * 8, c.stream));
+        CUIBM_TRY(cudaMemcpyAsync(d.h + (size_t)Rp[p] * nm, rhs.data(), nm * 8, cudaMemcpyHostToDevice, c.stream));
+        launch_tri(c, *P);
+        CUIBM_TRY(cudaMemcpyAsync(Gp[p], d.h, n * 8, cudaMemcpyDeviceToDevice, c.stream));
+        CUIBM_TRY(cudaStreamSynchronize(c.stream));
+        d.R[p] = Rp[p];
+        d.F[p] = Fp[p];
+        d.G[p] = Gp[p];
+    }
+    // the constant's response: mode k0 only, u = sqrt(len) there
+    CUIBM_TRY(cudaMemsetAsync(d.h, 0, n * 8, c.stream));
+    const double one = std::sqrt(len);
+    CUIBM_TRY(cudaMemcpyAsync(d.h + k0, &one, 8, cudaMemcpyHostToDevice, c.stream));
+    launch_tri(c, *P);
+    CUIBM_TRY(cudaMemcpy2DAsync(D(ogm), 8, d.h + k0, (size_t)nm * 8, 8, nr, cudaMemcpyDeviceToDevice, c.stream));
+    std::vector<double> row(nm);
+    for (int b = 0; b <= d.pins; ++b) {  // responses: the pins', then the constant's
+        const double *src = b < d.pins ? Gp[b] : d.h;
+        for (int a = 0; a <= d.pins; ++a) {
+            CUIBM_TRY(cudaMemcpyAsync(row.data(), src + (size_t)(a < d.pins ? Rp[a] : 0) * nm, nm * 8,
+                                      cudaMemcpyDeviceToHost, c.stream));
+            CUIBM_TRY(cudaStreamSynchronize(c.stream));
+            double v = 0;
+            if (a < d.pins)
+                for (int k = 0; k < nm; ++k) v += F[a][k] * row[k];
+            else
+                v = row[k0] * d.mean;
+            at_pin[a][b] = v;
+        }
+    }
+    const int m = d.pins;
+    for (int a = 0; a <= m; ++a)
+        for (int b = 0; b <= m; ++b) d.K[3 * a + b] = b == m ? -at_pin[a][b] : at_pin[a][b];
+    for (int p = 0; p < m; ++p) d.K[3 * p + p] += 1 / delta[p];
+    d.K[3 * m + m] += 1 / reg;
+    if (!invert3(d.K, m + 1)) throw CudaError("the separable preconditioner's pinned-cell correction is singular");
+    CUIBM_TRY(cudaStreamSynchronize(c.stream));
+}
+
+void free_separable(LinearSystem &S)
+{
+    SepPlan *P = static_cast<SepPlan *>(S.sep);
+    if (!P) return;
+    if (P->block) cudaFree(P->block);
+    delete P;
+    S.sep = nullptr;
+}
+
+// ---- host side: solves --------------------------------------------------------------------
+namespace {
+
+struct SepSolve {
+    Context &c;
+    LinearSystem &S;
+    const double *b;
+    double *x;
+
+    template <class F>
+    void with_op(const F &f) const
+    {
+        if (S.which == 1) f(op1(c, S.w));
+        else f(op2(c, S.w));
+    }
+    int nb() const { return blocks_for(S.n); }
+
+    void init() const
+    {
+        with_op([&](auto A) {
+            if (S.krylov == KRYLOV_CG)
+                k_cg_init<decltype(A), 2><<<nb(), kBlock, 0, c.stream>>>(A, S.n, b, S.w, x, S.r, S.z, S.p, S.dinv,
+                                                                        S.partials, S.ks, c.err_word, S.which, 0, 0);
+            else
+                k_sep_init<<<nb(), kBlock, 0, c.stream>>>(A, S.n, b, x, S.r, S.partials, S.ks, c.err_word, S.which);
+        });
+        CUIBM_TRY(cudaGetLastError());
+    }
+    // BiCGSTAB to the half step
+    void half(bool first, cudaGraphConditionalHandle h, int use) const
+    {
+        launch_separable_apply(c, S, first ? S.r : S.p, S.Mp);
+        with_op([&](auto A) {
+            k_sep_1<<<nb(), kBlock, 0, c.stream>>>(A, S.n, S.Mp, S.AMp, first ? S.r : S.rs, S.partials, S.ks, first);
+        });
+        k_sep_2<<<nb(), kBlock, 0, c.stream>>>(S.n, S.r, S.AMp, S.Mp, S.s, x, S.partials, S.ks, first, h, use);
+        CUIBM_TRY(cudaGetLastError());
+    }
+    // and from there
+    void rest(bool first, cudaGraphConditionalHandle h, int use) const
+    {
+        launch_separable_apply(c, S, S.s, S.Ms);
+        with_op([&](auto A) {
+            k_sep_3<<<nb(), kBlock, 0, c.stream>>>(A, S.n, S.s, S.Ms, S.AMs, S.partials, S.ks);
+        });
+        k_sep_4<<<nb(), kBlock, 0, c.stream>>>(S.n, x, S.r, S.rs, S.p, S.s, S.Ms, S.AMs, S.partials, S.ks, c.err_word,
+                                               S.which, first, h, use);
+        k_bicg_5<<<nb(), kBlock, 0, c.stream>>>(S.n, S.p, S.r, S.AMp, S.ks);
+        CUIBM_TRY(cudaGetLastError());
+    }
+    void cg(bool first, cudaGraphConditionalHandle h, int use) const
+    {
+        launch_separable_apply(c, S, S.r, S.z);
+        with_op([&](auto A) {
+            if (first) {
+                k_sep_cg_1<<<nb(), kBlock, 0, c.stream>>>(A, S.n, S.r, S.z, S.p, S.q, S.partials, S.ks);
+            } else {
+                k_cg_rz<<<nb(), kBlock, 0, c.stream>>>(S.n, S.r, S.z, S.partials, S.ks);
+                k_cg_3<<<nb(), kBlock, 0, c.stream>>>(S.n, S.p, S.z, S.ks);
+                k_cg_1<<<nb(), kBlock, 0, c.stream>>>(A, S.n, S.p, S.q, S.partials, S.ks);
+            }
+        });
+        k_cg_2<2><<<nb(), kBlock, 0, c.stream>>>(S.n, x, S.r, S.z, S.p, S.q, S.w, S.dinv, S.partials, S.ks, c.err_word,
+                                                 S.which, h, use);
+        CUIBM_TRY(cudaGetLastError());
+    }
+};
+
+// A conditional node after what c.stream has captured so far; its handle's value is 0 at
+// each launch of the graph.  make() creates the handle before the kernels that set it.
+struct CondNode {
+    Context &c;
+    cudaGraphConditionalHandle h{};
+
+    explicit CondNode(Context &c_) : c(c_)
+    {
+        cudaStreamCaptureStatus st;
+        cudaGraph_t graph;
+        CUIBM_TRY(cudaStreamGetCaptureInfo(c.stream, &st, nullptr, &graph, nullptr, nullptr, nullptr));
+        CUIBM_TRY(cudaGraphConditionalHandleCreate(&h, graph, 0, cudaGraphCondAssignDefault));
+    }
+    template <class F>
+    int add(cudaGraphConditionalNodeType type, const F &body)
+    {
+        cudaStreamCaptureStatus st;
+        cudaGraph_t graph;
+        const cudaGraphNode_t *deps = nullptr;
+        size_t ndeps = 0;
+        CUIBM_TRY(cudaStreamGetCaptureInfo(c.stream, &st, nullptr, &graph, &deps, nullptr, &ndeps));
+        cudaGraphNodeParams cp = {};
+        cp.type = cudaGraphNodeTypeConditional;
+        cp.conditional.handle = h;
+        cp.conditional.type = type;
+        cp.conditional.size = 1;
+        cudaGraphNode_t node;
+        CUIBM_TRY(cudaGraphAddNode(&node, graph, deps, nullptr, ndeps, &cp));
+        cudaStream_t main = c.stream, side = c.side_stream;
+        CUIBM_TRY(cudaStreamBeginCaptureToGraph(side, cp.conditional.phGraph_out[0], nullptr, nullptr, 0,
+                                                cudaStreamCaptureModeRelaxed));
+        c.stream = side;
+        try {
+            body();
+        } catch (...) {
+            c.stream = main;
+            cudaGraph_t dummy;
+            cudaStreamEndCapture(side, &dummy);
+            throw;
+        }
+        c.stream = main;
+        cudaGraph_t got;
+        CUIBM_TRY(cudaStreamEndCapture(side, &got));
+        CUIBM_TRY(cudaStreamUpdateCaptureDependencies(c.stream, &node, nullptr, 1, cudaStreamSetCaptureDependencies));
+        return count_kernel_nodes(got);
+    }
+};
+
+}  // namespace
+
+// A solve on c.stream.  Captured into the step's graph, the first half iteration (CG: the
+// first iteration) is plain nodes, the rest of it an IF node and further iterations a WHILE
+// node, both skipped by the solves that have converged; otherwise the host reads the
+// status after each.
+void launch_separable_solve(Context &c, LinearSystem &S, const double *b, double *x, bool in_graph)
+{
+    const SepSolve L{c, S, b, x};
+    SepPlan &P = *static_cast<SepPlan *>(S.sep);
+    const bool cg = S.krylov == KRYLOV_CG;
+    if (in_graph) {
+        L.init();
+        CondNode more(c);
+        if (cg) {
+            L.cg(true, more.h, 1);
+            S.body_kernels = more.add(cudaGraphCondTypeWhile, [&] { L.cg(false, more.h, 1); });
+            P.first_kernels = S.body_kernels;
+            return;
+        }
+        CondNode second(c);
+        L.half(true, second.h, 1);
+        P.first_kernels = second.add(cudaGraphCondTypeIf, [&] { L.rest(true, more.h, 1); });
+        S.body_kernels = more.add(cudaGraphCondTypeWhile, [&] {
+            L.half(false, more.h, 1);
+            L.rest(false, more.h, 1);
+        });
+        return;
+    }
+    KrylovScalars host{};
+    auto running = [&] {
+        CUIBM_TRY(cudaMemcpyAsync(&host, S.ks, sizeof(host), cudaMemcpyDeviceToHost, c.stream));
+        CUIBM_TRY(cudaStreamSynchronize(c.stream));
+        return host.status == KS_RUNNING;
+    };
+    L.init();
+    if (cg) {
+        L.cg(true, 0, 0);
+        while (running()) L.cg(false, 0, 0);
+        return;
+    }
+    L.half(true, 0, 0);
+    if (!running()) return;
+    L.rest(true, 0, 0);
+    while (running()) {
+        L.half(false, 0, 0);
+        L.rest(false, 0, 0);
+    }
+}
+
+// kernels that a solve's conditional bodies ran: the first execution is the rest of the
+// first iteration, the later ones whole iterations
+long long separable_body_launches(const LinearSystem &S, int runs)
+{
+    const SepPlan &P = *static_cast<const SepPlan *>(S.sep);
+    return runs > 0 ? P.first_kernels + (long long)(runs - 1) * S.body_kernels : 0;
+}
+
+// Algorithmic bytes of a solve with `it` iterations: the residual, and for each application
+// of the preconditioner its input, output, digits of one operand, the transform's two
+// tables and the tridiagonal factors, with the operator applied to the result
+double separable_bytes(const LinearSystem &S, int it)
+{
+    const SepPlan &P = *static_cast<const SepPlan *>(S.sep);
+    const double n = S.n, nm = P.d.nm, L = P.digits;
+    const double app = 8 * n * 2 + 2 * 2 * L * (n + nm * nm) + 8 * n * (2 + 3 + 2) + 8 * n * 5;
+    const double apps = S.krylov == KRYLOV_CG ? std::max(it, 1) : 1 + 2 * std::max(0.0, it - 0.5);
+    return 8 * n * 3 + apps * app;
+}
+
+}  // namespace cuibm

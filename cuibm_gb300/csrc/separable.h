@@ -1,0 +1,14 @@
+// The pressure system's separable preconditioner (separable.cu).
+#pragma once
+#include "solver.h"
+
+namespace cuibm {
+
+void setup_separable(Context &c, LinearSystem &S);  // S.sep stays null where it does not apply
+void launch_separable_apply(Context &c, LinearSystem &S, const double *in, double *out);
+void launch_separable_solve(Context &c, LinearSystem &S, const double *b, double *x, bool in_graph);
+long long separable_body_launches(const LinearSystem &S, int runs);
+double separable_bytes(const LinearSystem &S, int it);
+void free_separable(LinearSystem &S);
+
+}  // namespace cuibm

@@ -157,6 +157,7 @@ struct LinearSystem {
     bool sa_dynamic = false;
     std::vector<void *> sa_blocks;
     unsigned long long sa_key = 0;
+    void *sep = nullptr;    // the separable preconditioner (separable.cu), null where it does not apply
     void *mixed = nullptr;  // mixed precision: the float tables (fused_solve.cu)
     double *aedef = nullptr;                // A e (the operator's row sums), with wdef
     double *ym = nullptr, *wdef = nullptr;  // constant-mode correction of the SA cycle (Poisson):

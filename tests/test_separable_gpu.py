@@ -1,0 +1,98 @@
+"""The pressure system's separable preconditioner (csrc/separable.cu): pressure solves on
+grids at the edges of its tiles - chunks of 32 terms, product tiles of 32 x 32 and 32 x 64,
+the splitting kernels' 256, 512 and 1024 places, the tridiagonal blocks of 4 and 8 modes -
+along both transform directions, uniform and stretched, for both Krylov methods and
+precisions, against the residual of the assembled matrix.
+
+The bound: the solver stops at ||r|| <= tol ||b|| for the recursively updated r; x is the
+sum of at most a few updates, each rounded to half an ulp, and each application of A (five
+terms a row) rounds by at most 6 eps of |A| |x|, so the true residual is below
+tol ||b|| + 40 eps || |A| |x| + |b| ||."""
+import numpy as np
+import pytest
+
+cb = pytest.importorskip("cuibm_gb300")
+sp = pytest.importorskip("scipy.sparse")
+from cuibm_gb300 import cases  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-12
+
+
+def box(folder, nx, ny, ratio, krylov, precision, tol=TOL):
+    """nx x ny cells: uniform, or stretched away from the first corner (the counts of a
+    stretched axis follow from its length)."""
+    def axis(name, n):
+        if ratio == 1.0:
+            return cases.axis(name, 0.0, 0.01, [((n + 0.5) * 0.01, 1.0)])
+        return cases.axis(name, 0.0, 0.01, [(0.01 * (ratio ** (n + 0.5) - 1) / (ratio - 1), ratio)])
+    sim = {"type": "simulation", "dt": 0.003, "nt": 10, "nsave": 10, "SolverType": "NAVIER_STOKES_SOLVER",
+           "linearSolvers": cases.solvers("DIAGONAL", tol, "SMOOTHED_AGGREGATION", tol, pois_krylov=krylov,
+                                          precision=precision)}
+    flow = [{"type": "flow", "nu": 0.01, "initialVelocity": [0.0, 0.0], "initialPerturbation": [0.0, 0.0],
+             "boundaryConditions": cases.bcs((0, 0), (0, 0), (0, 0), (1.0, 0))}]
+    return cases.write_case(folder, [sim], flow, [axis("x", nx), axis("y", ny)], [])
+
+
+def solver(folder, args=()):
+    s = cb.NavierStokesSolver(folder, args)
+    s.set_option("write_output", 0)
+    s.initialise()
+    return s
+
+
+def check(s, b, p0):
+    n = s.info.numP
+    s.set("rhs2", b)
+    s.set("p", p0)
+    s.run("solve_poisson")
+    p = s.get("p")
+    A = sp.coo_matrix((s.matrix(2)[2], s.matrix(2)[:2]), shape=(n, n)).tocsr()
+    floor = np.linalg.norm(abs(A) @ np.abs(p) + np.abs(b))
+    res = np.linalg.norm(b - A @ p)
+    assert res <= TOL * np.linalg.norm(b) + 40 * np.finfo(float).eps * floor, (res, np.linalg.norm(b), floor)
+    return p
+
+
+SIZES = [(3, 3, 1.0), (5, 4, 1.3), (31, 40, 1.05), (32, 33, 1.0), (33, 32, 1.0), (64, 65, 1.02), (129, 63, 1.0),
+         (257, 90, 1.01), (700, 24, 1.0), (24, 700, 1.0), (290, 1100, 1.0), (521, 530, 1.004), (610, 601, 1.0),
+         (1033, 1040, 1.0)]
+
+
+@pytest.mark.parametrize("nx,ny,ratio", SIZES)
+@pytest.mark.parametrize("krylov,precision", [("BICGSTAB", None), ("CG", None), ("BICGSTAB", "MIXED")])
+def test_solves_meet_the_residual_bound(tmp_path, nx, ny, ratio, krylov, precision):
+    with solver(box(str(tmp_path / "c"), nx, ny, ratio, krylov, precision)) as s:
+        i = s.info
+        assert (i.nx, i.ny) == (nx, ny)
+        rng = np.random.default_rng(nx * 1000 + ny)
+        for b in (rng.standard_normal(i.numP), np.repeat(rng.standard_normal(ny), nx)):
+            check(s, b, rng.standard_normal(i.numP))
+            assert s.iterations()[1] <= 3  # the inverse to rounding (mixed precision: to 2^-31)
+
+
+def test_agrees_with_smoothed_aggregation_and_runs_in_steps(tmp_path):
+    f = box(str(tmp_path / "c"), 90, 71, 1.02, "BICGSTAB", None)
+    out = []
+    for flag, graph in (("1", 1), ("1", 0), ("0", 1)):
+        with solver(f, ["-separable", flag]) as s:
+            s.set_option("use_graph", graph)
+            s.stepTime(12)
+            out.append((s.get("u"), s.get("p"), s.iterations()[1]))
+    assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
+    (u, p, it), _, (us, ps, its) = out
+    assert it <= 2 < its
+    assert np.linalg.norm(u - us) <= 1e-9 * np.linalg.norm(us) and np.linalg.norm(p - ps) <= 1e-9 * np.linalg.norm(ps)
+
+
+def test_zero_and_non_finite_right_hand_sides(tmp_path):
+    with solver(box(str(tmp_path / "c"), 40, 36, 1.0, "BICGSTAB", None)) as s:
+        n = s.info.numP
+        assert np.all(check(s, np.zeros(n), np.zeros(n)) == 0)
+        b = np.ones(n)
+        b[77] = np.inf
+        s.set("rhs2", b)
+        with pytest.raises(cb.CuibmError) as e:
+            s.run("solve_poisson")
+        assert e.value.status == cb.ERR_NAN
+        check(s, np.random.default_rng(1).standard_normal(n), np.zeros(n))  # and is usable again
