@@ -22,6 +22,7 @@
 // system (W A) x = W b with W = diag(w) the row weights that make the staggered
 // operators symmetric (cell or face areas); convergence is still measured on the
 // original residual b - A x = W^-1 r_sym.
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -239,7 +240,7 @@ void setup_system(Context &c, LinearSystem &S)
     S.z = S.Ms;
     S.q = S.AMs;
     S.dinv = c.carve<double>(n);
-    S.partials = c.carve<double>(4 * (size_t)blocks_for(n) + 4);
+    S.partials = c.carve<double>(4 * (size_t)std::max(blocks_for(n) + 1, kRowBlocks));
     S.ks = c.carve<KrylovScalars>(1);
     {
         KrylovScalars hk{};

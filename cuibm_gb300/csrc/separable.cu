@@ -1,4 +1,5 @@
-// The pressure system's separable preconditioner and the Krylov solves that use it.
+// The separable preconditioner of the pressure and velocity systems and the Krylov solves
+// that use it.
 //
 // On the tensor-product pressure grid the operator of NavierStokes/kernels/LHS2.cu
 // (dt D G) is A0 = X (x) I + I (x) Y with tridiagonal X (entries of the column spacing)
@@ -20,7 +21,8 @@
 // after one application or two.  It stays a preconditioner of the same Krylov method, with
 // the same stopping rule on the FP64 residual, so what the dense products' rounding leaves
 // (about 1e-9 of the residual at 922 x 922, as FP64 products leave it) the iteration
-// removes.
+// removes.  The velocity operator (I - dt/2 nu L, LHS1.cu) is 1 + X (x) I + I (x) Y on the u
+// and on the v grid, without pinned cells; both grids go through the same launches.
 //
 // The dense products are 2 n_m^2 n_r multiply-adds each, which at GB300's FP64 rate
 // (1.25 TFLOP/s) would take 1.25 ms at 922 x 922.  They run on the tensor cores instead,
@@ -53,10 +55,11 @@ constexpr int kFlush = 4;        // chunks between flushes: 7 x 128 x 2^14 < 2^2
 constexpr int kSepMax = 2048;
 constexpr int kTriThreads = 512;
 
-// device view of the plan (a kernel argument)
+// Device view of one grid's plan.  The pressure system has one grid; the velocity system
+// two (u, v), which every kernel takes in one launch.
 struct SepDev {
     int nm, nr;            // modes (length of the transformed direction), rows (the other)
-    int sm, sr;            // strides of a field: element (row R, place m) at R sr + m sm
+    int sm, sr, base;      // a field's layout: element (row R, place m) at base + R sr + m sm
     int nch;               // chunks of kKC terms in a transform
     const __nv_bfloat16 *B1, *B2;  // digits of Q^T and of Q
     const double *sB1, *sB2;       // their row scales (and the output's D^-1/2)
@@ -66,16 +69,24 @@ struct SepDev {
     const double *l, *c, *inv;     // tridiagonal factors [row][mode]
     const double *Pf, *Pb;         // products of l and c over a thread's rows [thread row][mode]
     const double *cm, *cr;         // input scaling per place and per row (cr null: 1)
-    // pinned cells: functionals F (rows R0, R1), responses G, the constant's response gm
+    // pinned cells (the pressure system): functionals F (rows R0, R1), responses G, the
+    // constant's response gm
     int pins, R[2], k0;
     const double *F[2], *G[2], *gm;
     double K[9], mean;
 };
+struct SepArgs {
+    SepDev f[2];
+};
 
 struct SepPlan {
-    SepDev d{};
+    SepArgs a{};
+    int grids = 1;
     int digits = kDigits;
-    char *block = nullptr;  // one device allocation
+    char *block[2] = {nullptr, nullptr};  // one device allocation a grid
+    int tri_rows = 0;  // neighbouring rows a thread of k_sep_tri takes
+    int max_nm() const { return grids > 1 ? std::max(a.f[0].nm, a.f[1].nm) : a.f[0].nm; }
+    int max_nr() const { return grids > 1 ? std::max(a.f[0].nr, a.f[1].nr) : a.f[0].nr; }
     int first_kernels = 0;  // kernels of the conditional body after the first half iteration
 };
 
@@ -180,22 +191,30 @@ __device__ __forceinline__ double block_sum(double v)
 // makes the transform orthonormal); true: z^, with the pinned cells' correction.  A row of
 // 922 is 7 values a thread: bound by one round of loads, the conversion and the stores.
 template <int L, int NP, bool SPEC>
-__global__ void __launch_bounds__(128) k_sep_split(SepDev d, const double *__restrict__ in)
+__global__ void __launch_bounds__(128) k_sep_split(const __grid_constant__ SepArgs args, const double *__restrict__ in)
 {
+    const SepDev &d = args.f[blockIdx.y];
     const int R = blockIdx.x, n = d.nm;
+    if (R >= d.nr) return;
     __nv_bfloat16 *out = d.A + (size_t)R * d.nch * L * kKC;
     double s;
     if (!SPEC) {
-        const double *row = in + (size_t)R * d.sr;
+        const double *row = in + d.base + (size_t)R * d.sr;
         const double cr = d.cr ? d.cr[R] : 1.0;
         s = split_row<L, NP>(n, d.nch, out, [&](int m) { return row[(size_t)m * d.sm] * (d.cm[m] * cr); });
     } else {
+        const double *row = d.h + (size_t)R * n;
+        if (d.pins == 0) {
+            s = split_row<L, NP>(n, d.nch, out, [&](int m) { return row[m]; });
+            if (threadIdx.x == 0) d.sA[R] = s;
+            return;
+        }
         // q = K^-1 (values of z at the pinned cells, mean of row 0), the same in every block
         double f[3] = {0, 0, 0}, q[3] = {0, 0, 0};
         for (int p = 0; p < d.pins; ++p) {
             double v = 0;
-            const double *row = d.h + (size_t)d.R[p] * n;
-            for (int k = threadIdx.x; k < n; k += blockDim.x) v += d.F[p][k] * row[k];
+            const double *at = d.h + (size_t)d.R[p] * n;
+            for (int k = threadIdx.x; k < n; k += blockDim.x) v += d.F[p][k] * at[k];
             f[p] = block_sum(v);
         }
         const int nq = d.pins + 1;
@@ -203,7 +222,6 @@ __global__ void __launch_bounds__(128) k_sep_split(SepDev d, const double *__res
         for (int a = 0; a < nq; ++a)
             for (int b = 0; b < nq; ++b) q[a] += d.K[3 * a + b] * f[b];
         const double qm = q[d.pins] * d.gm[R];
-        const double *row = d.h + (size_t)R * n;
         const double *g0 = d.G[0] + (size_t)R * n, *g1 = d.pins > 1 ? d.G[1] + (size_t)R * n : nullptr;
         s = split_row<L, NP>(n, d.nch, out, [&](int m) {
             double v = row[m] - q[0] * g0[m];
@@ -239,18 +257,22 @@ __device__ __forceinline__ void cp16(unsigned dst, const void *src)
 // bank conflict.  A warp holds its L digit fragments of A and walks the digits of B: 2 L
 // ldmatrix for L (L + 1) mma.
 template <int L, int WM, int WN, int ST>
-__global__ void __launch_bounds__(32 * WM * WN, 2) k_sep_gemm(const __nv_bfloat16 *__restrict__ A,
-                                                          const double *__restrict__ sA, int M,
-                                                          const __nv_bfloat16 *__restrict__ B,
-                                                          const double *__restrict__ sB, int N, int nch,
-                                                          double *__restrict__ out, int so_m, int so_n)
+__global__ void __launch_bounds__(32 * WM * WN, 2) k_sep_gemm(const __grid_constant__ SepArgs args,
+                                                             double *__restrict__ field, int back)
 {
+    // forward: h = (digits of the field) Q; back: field = (digits of z^) Q^T
+    const SepDev &d = args.f[blockIdx.z];
+    const __nv_bfloat16 *__restrict__ A = d.A, *__restrict__ B = back ? d.B2 : d.B1;
+    const double *__restrict__ sA = d.sA, *__restrict__ sB = back ? d.sB2 : d.sB1;
+    const int M = d.nr, N = d.nm, nch = d.nch, so_m = back ? d.sr : d.nm, so_n = back ? d.sm : 1;
+    double *__restrict__ out = back ? field + d.base : d.h;
     constexpr int TM = 16 * WM, TN = 16 * WN, T = 32 * WM * WN;
     constexpr int RB = 64 * L + 16;                // bytes of a row in a stage
     constexpr int STAGE = (TM + TN) * RB;
     extern __shared__ __align__(16) unsigned char smem[];
     const unsigned sbase = (unsigned)__cvta_generic_to_shared(smem);
     const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
+    if (m0 >= M || n0 >= N) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int wm = warp / WN, wn = warp % WN;
     const size_t rowBytes = (size_t)nch * L * kKC * 2;
@@ -378,13 +400,13 @@ __device__ __forceinline__ double tri_scan(double end, double prod, bool up, dou
 }
 
 template <int CB>
-__global__ void __launch_bounds__(kTriThreads) k_sep_tri(SepDev d)
+__global__ void __launch_bounds__(kTriThreads) k_sep_tri(const __grid_constant__ SepArgs args, int m)
 {
-    constexpr int NQ = kTriThreads / CB;
+    const SepDev &d = args.f[blockIdx.y];
     extern __shared__ double row[];  // [m][thread]: r, then inv d
     __shared__ double se[2 * kTriThreads], sp[2 * kTriThreads];
     const int tid = threadIdx.x, n = d.nm;
-    const int k = blockIdx.x * CB + tid % CB, q = tid / CB, m = (d.nr + NQ - 1) / NQ;
+    const int k = blockIdx.x * CB + tid % CB, q = tid / CB;
     const int J0 = min(q * m, d.nr), J1 = min(J0 + m, d.nr), cnt = k < n ? J1 - J0 : 0;
     const size_t at = (size_t)J0 * n + k;
     double x = 0;
@@ -418,15 +440,15 @@ static int tri_modes(int nm, int nr) { return nm >= 600 && nr <= kTriRows / 2 ? 
 
 // the factors of Y + lambda_k, one thread a mode, and their products over each thread's
 // rows of k_sep_tri; the constant's mode gets reg on its first diagonal
-__global__ void k_sep_factor(int nm, int nr, int nq, const double *__restrict__ up, const double *__restrict__ dn,
-                             const double *__restrict__ lam, int k0, double reg, double *l, double *c, double *inv,
+__global__ void k_sep_factor(int nm, int nr, int nq, int m, const double *__restrict__ up, const double *__restrict__ dn,
+                             const double *__restrict__ lam, double shift, int k0, double reg, double *l, double *c, double *inv,
                              double *Pf, double *Pb)
 {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= nm) return;
     double prev = 0;
     for (int J = 0; J < nr; ++J) {
-        double dg = up[J] + dn[J] + lam[k];
+        double dg = shift + (up[J] + dn[J] + lam[k]);
         if (k == k0 && J == 0) dg += reg;
         const double lj = J ? dn[J] * prev : 0.0;
         if (J) dg -= lj * up[J - 1];
@@ -436,7 +458,6 @@ __global__ void k_sep_factor(int nm, int nr, int nq, const double *__restrict__ 
         inv[at] = prev;
         c[at] = J + 1 < nr ? up[J] * prev : 0.0;
     }
-    const int m = (nr + nq - 1) / nq;
     for (int q = 0; q < nq; ++q) {
         double pf = 1, pb = 1;
         for (int J = q * m; J < min((q + 1) * m, nr); ++J) {
@@ -448,41 +469,45 @@ __global__ void k_sep_factor(int nm, int nr, int nq, const double *__restrict__ 
     }
 }
 
-// Q from the QR iteration's rotations: thread i holds row i of Q in shared memory (element
-// j at [j][thread]) and applies every rotation to it in order; a rotation changes elements
-// j and j + 1, ascending in a sweep, so one value is carried in a register
+// Q from the QR iteration's rotations: every row of Q is a unit vector to which all
+// rotations are applied in order.  A warp takes a row and applies 32 sweeps at once as a
+// pipeline: lane l applies sweep l, two elements behind lane l - 1.  A rotation of elements
+// k, k + 1 takes the carried element a and the next one x to the finished c a + s x and the
+// carried c x - s a, so a lane is a shift register that hands its finished element to the
+// next lane a step later, and where its sweep has no rotation it passes elements on (c = 1,
+// s = 0).  922 x 922 in 7 ms; one thread a row, a rotation after another, took 120 ms.
 struct Sweep {
     int first, count;
     long long at;
 };
-__global__ void k_sep_rotate(int n, const Sweep *__restrict__ sw, int nsw, const double2 *__restrict__ rot,
-                             double *__restrict__ Q)
+constexpr int kRotWarps = 8;
+__global__ void __launch_bounds__(32 * kRotWarps) k_sep_rotate(int n, const Sweep *__restrict__ sw, int nsw,
+                                                               const double2 *__restrict__ rot,
+                                                               double *__restrict__ Q)
 {
-    extern __shared__ double z[];
-    __shared__ double2 cs[64];
-    const int W = blockDim.x, t = threadIdx.x, i = blockIdx.x * W + t;
-    for (int j = 0; j < n; ++j) z[j * W + t] = j == i ? 1.0 : 0.0;
-    for (int s = 0; s < nsw; ++s) {
-        const Sweep S = sw[s];
-        double a = z[S.first * W + t];
-        for (int b0 = 0; b0 < S.count; b0 += 64) {
-            const int nb = min(64, S.count - b0);
-            __syncthreads();
-            for (int b = t; b < nb; b += W) cs[b] = rot[S.at + b0 + b];
-            __syncthreads();
-#pragma unroll 4
-            for (int b = 0; b < nb; ++b) {
-                const double2 r = cs[b];
-                const int j = S.first + b0 + b;
-                const double v = z[(j + 1) * W + t];
-                z[j * W + t] = r.x * a + r.y * v;
-                a = r.x * v - r.y * a;
-            }
+    extern __shared__ double rows[];
+    const int lane = threadIdx.x & 31, i = blockIdx.x * kRotWarps + (threadIdx.x >> 5);
+    if (i >= n) return;
+    double *z = rows + (size_t)(threadIdx.x >> 5) * n;
+    for (int j = lane; j < n; j += 32) z[j] = j == i ? 1.0 : 0.0;
+    __syncwarp();
+    for (int s0 = 0; s0 < nsw; s0 += 32) {
+        const bool on = s0 + lane < nsw;
+        const int lo = on ? sw[s0 + lane].first : 0, cnt = on ? sw[s0 + lane].count : 0;
+        const double2 *r = rot + (on ? sw[s0 + lane].at : 0);
+        double a = 0, out = 0;
+        for (int t = 0; t < n + 63; ++t) {
+            const int k = t - 2 * lane - 1 - lo;  // this step's rotation in the sweep
+            double x = __shfl_up_sync(0xffffffffu, out, 1);
+            if (lane == 0) x = t < n ? z[t] : 0.0;
+            const double2 cs = k >= 0 && k < cnt ? r[k] : make_double2(1.0, 0.0);
+            out = fma(cs.y, x, cs.x * a);
+            a = fma(-cs.y, a, cs.x * x);
+            if (lane == 31 && t >= 63) z[t - 63] = out;
         }
-        z[(S.first + S.count) * W + t] = a;
+        __syncwarp();
     }
-    if (i < n)
-        for (int j = 0; j < n; ++j) Q[(size_t)i * n + j] = z[j * W + t];
+    for (int j = lane; j < n; j += 32) Q[(size_t)i * n + j] = z[j];
 }
 
 // column k0 of Q: the constant in exact form
@@ -493,6 +518,50 @@ __global__ void k_sep_constant(int n, int k0, const double *__restrict__ v, doub
 }
 
 // ---- Krylov kernels ---------------------------------------------------------------------
+// The rows of a grid of at most kRowBlocks blocks, and its sums: a block's partial sums go
+// to memory, and the last block to arrive adds them in a fixed order with one warp.  The
+// totals are valid in the last block's thread 0 (true there only).
+static int row_blocks(int n) { return std::min(kRowBlocks, blocks_for(n)); }
+#define SEP_ROWS(i, n) for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < (n); i += gridDim.x * blockDim.x)
+
+template <int NV>
+__device__ __forceinline__ bool row_sums(double (&v)[NV], double *partials, unsigned int *arrive)
+{
+    __shared__ double sh[NV][kBlock / 32];
+    __shared__ bool last;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+        for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
+        if (lane == 0) sh[k][w] = v[k];
+    }
+    __syncthreads();
+    if (w != 0) return false;
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+        v[k] = lane < kBlock / 32 ? sh[k][lane] : 0.0;
+        for (int o = kBlock / 64; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
+        if (lane == 0) partials[k * kRowBlocks + blockIdx.x] = v[k];
+    }
+    if (lane == 0) {
+        __threadfence();
+        last = atomicAdd(arrive, 1u) == gridDim.x - 1;
+        __threadfence();
+    }
+    __syncwarp();
+    if (!last) return false;
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+        double a = 0;
+#pragma unroll 4
+        for (int b = lane; b < (int)gridDim.x; b += 32) a += __ldcg(partials + k * kRowBlocks + b);
+        for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
+        v[k] = a;
+    }
+    if (lane == 0) *arrive = 0;
+    return lane == 0;
+}
+
 // BiCGSTAB as in krylov.cu with two differences: the first half iteration takes r for its
 // shadow residual and direction (they are copies then), and x takes alpha M p in the half
 // step, so that a solve that ends there - the usual end - needs nothing more.
@@ -500,18 +569,18 @@ template <class Op>
 __global__ void __launch_bounds__(256) k_sep_init(Op A, int n, const double *__restrict__ b, const double *x, double *r,
                                                   double *partials, KrylovScalars *ks, int *err, int which)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    double v[2] = {0, 0}, t[2];
-    if (i < n) {
+    double v[2] = {0, 0};
+    SEP_ROWS(i, n)
+    {
         const double bi = b[i], ri = bi - A.row(i, PtrAccess{x});
         r[i] = ri;
-        v[0] = ri * ri;
-        v[1] = bi * bi;
+        v[0] += ri * ri;
+        v[1] += bi * bi;
     }
-    if (reduce_arrive<2>(v, partials, &ks->arrive, t) && threadIdx.x == 0) {
-        ks->rho = t[0];
-        ks->rnorm = sqrt(t[0]);
-        ks->bnorm = sqrt(t[1]);
+    if (row_sums<2>(v, partials, &ks->arrive)) {
+        ks->rho = v[0];
+        ks->rnorm = sqrt(v[0]);
+        ks->bnorm = sqrt(v[1]);
         ks->tol = ks->rtol * ks->bnorm;
         ks->it = 0;
         ks->s_done = 0;
@@ -527,15 +596,15 @@ __global__ void __launch_bounds__(256) k_sep_1(Op A, int n, const double *__rest
                                                int first)
 {
     if (ks->status != KS_RUNNING) return;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    double v[1] = {0}, t[1];
-    if (i < n) {
+    double v[1] = {0};
+    SEP_ROWS(i, n)
+    {
         const double a = A.row(i, PtrAccess{Mp});
         AMp[i] = a;
-        v[0] = rs[i] * a;
+        v[0] += rs[i] * a;
     }
-    if (reduce_arrive<1>(v, partials, &ks->arrive, t) && threadIdx.x == 0) {
-        ks->alpha = ks->rho / t[0];
+    if (row_sums<1>(v, partials, &ks->arrive)) {
+        ks->alpha = ks->rho / v[0];
         ks->s_done = 0;
         if (!first) ks->body_runs += 1;
     }
@@ -546,17 +615,17 @@ __global__ void __launch_bounds__(256) k_sep_2(int n, const double *__restrict__
                                                KrylovScalars *ks, int first, cudaGraphConditionalHandle h, int use_cond)
 {
     if (ks->status != KS_RUNNING) return;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const double alpha = ks->alpha;
-    double v[1] = {0}, t[1];
-    if (i < n) {
+    double v[1] = {0};
+    SEP_ROWS(i, n)
+    {
         const double si = r[i] - alpha * AMp[i];
         s[i] = si;
         x[i] += alpha * Mp[i];
-        v[0] = si * si;
+        v[0] += si * si;
     }
-    if (reduce_arrive<1>(v, partials, &ks->arrive, t) && threadIdx.x == 0) {
-        ks->snorm = sqrt(t[0]);
+    if (row_sums<1>(v, partials, &ks->arrive)) {
+        ks->snorm = sqrt(v[0]);
         if (ks->snorm <= ks->tol) {
             ks->s_done = 1;
             ks->rnorm = ks->snorm;
@@ -574,15 +643,15 @@ __global__ void __launch_bounds__(256) k_sep_3(Op A, int n, const double *__rest
                                                KrylovScalars *ks)
 {
     if (ks->status != KS_RUNNING) return;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    double v[2] = {0, 0}, t[2];
-    if (i < n) {
+    double v[2] = {0, 0};
+    SEP_ROWS(i, n)
+    {
         const double a = A.row(i, PtrAccess{Ms});
         AMs[i] = a;
-        v[0] = a * s[i];
-        v[1] = a * a;
+        v[0] += a * s[i];
+        v[1] += a * a;
     }
-    if (reduce_arrive<2>(v, partials, &ks->arrive, t) && threadIdx.x == 0) ks->omega = t[0] / t[1];
+    if (row_sums<2>(v, partials, &ks->arrive)) ks->omega = v[0] / v[1];
 }
 
 // x += omega M s, r = s - omega A M s; the first time also rs = p = the residual the solve began with
@@ -593,10 +662,10 @@ __global__ void __launch_bounds__(256) k_sep_4(int n, double *x, double *r, doub
                                                int use_cond)
 {
     if (ks->status != KS_RUNNING) return;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const double omega = ks->omega;
-    double v[2] = {0, 0}, t[2];
-    if (i < n) {
+    double v[2] = {0, 0};
+    SEP_ROWS(i, n)
+    {
         const double r0 = first ? r[i] : rs[i];
         if (first) {
             rs[i] = r0;
@@ -605,14 +674,14 @@ __global__ void __launch_bounds__(256) k_sep_4(int n, double *x, double *r, doub
         x[i] += omega * Ms[i];
         const double ri = s[i] - omega * AMs[i];
         r[i] = ri;
-        v[0] = r0 * ri;
-        v[1] = ri * ri;
+        v[0] += r0 * ri;
+        v[1] += ri * ri;
     }
-    if (reduce_arrive<2>(v, partials, &ks->arrive, t) && threadIdx.x == 0) {
-        ks->beta = (t[0] / ks->rho) * (ks->alpha / omega);
-        ks->rho = t[0];
+    if (row_sums<2>(v, partials, &ks->arrive)) {
+        ks->beta = (v[0] / ks->rho) * (ks->alpha / omega);
+        ks->rho = v[0];
         ks->it += 1;
-        ks->rnorm = sqrt(t[1]);
+        ks->rnorm = sqrt(v[1]);
         finish_status(ks, err, which);
         set_cond(h, use_cond, ks->status == KS_RUNNING);
     }
@@ -625,18 +694,18 @@ __global__ void __launch_bounds__(256) k_sep_cg_1(Op A, int n, const double *__r
                                                   double *partials, KrylovScalars *ks)
 {
     if (ks->status != KS_RUNNING) return;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    double v[2] = {0, 0}, t[2];
-    if (i < n) {
+    double v[2] = {0, 0};
+    SEP_ROWS(i, n)
+    {
         const double zi = z[i], qi = A.row(i, PtrAccess{z});
         p[i] = zi;
         q[i] = qi;
-        v[0] = r[i] * zi;
-        v[1] = zi * qi;
+        v[0] += r[i] * zi;
+        v[1] += zi * qi;
     }
-    if (reduce_arrive<2>(v, partials, &ks->arrive, t) && threadIdx.x == 0) {
-        ks->rho = t[0];
-        ks->alpha = t[0] / t[1];
+    if (row_sums<2>(v, partials, &ks->arrive)) {
+        ks->rho = v[0];
+        ks->alpha = v[0] / v[1];
     }
 }
 
@@ -718,12 +787,11 @@ bool invert3(double *K, int n)
 }  // namespace
 
 template <int L, int WM, int WN, int ST>
-static void launch_gemm_t(Context &c, const __nv_bfloat16 *A, const double *sA, int M, const __nv_bfloat16 *B,
-                          const double *sB, int N, int nch, double *out, int so_m, int so_n)
+static void launch_gemm_t(Context &c, const SepPlan &P, double *field, int back)
 {
     constexpr int smem = ST * 16 * (WM + WN) * (64 * L + 16);
-    const dim3 grid((N + 16 * WN - 1) / (16 * WN), (M + 16 * WM - 1) / (16 * WM));
-    k_sep_gemm<L, WM, WN, ST><<<grid, 32 * WM * WN, smem, c.stream>>>(A, sA, M, B, sB, N, nch, out, so_m, so_n);
+    const dim3 grid((P.max_nm() + 16 * WN - 1) / (16 * WN), (P.max_nr() + 16 * WM - 1) / (16 * WM), P.grids);
+    k_sep_gemm<L, WM, WN, ST><<<grid, 32 * WM * WN, smem, c.stream>>>(P.a, field, back);
     CUIBM_TRY(cudaGetLastError());
 }
 
@@ -745,26 +813,23 @@ static void allow_gemm()
 // Tiles of 32 x 64 (two blocks an SM) where there are enough of them for every SM, else 32
 // x 32: a 270 x 270 product is 81 small tiles or 45 large ones on 152 SMs
 template <int L>
-static void launch_gemm(Context &c, const SepPlan &P, const __nv_bfloat16 *B, const double *sB, double *out, int so_m,
-                        int so_n)
+static void launch_gemm(Context &c, const SepPlan &P, double *field, int back)
 {
-    const SepDev &d = P.d;
-    const int large = ((d.nr + 31) / 32) * ((d.nm + 63) / 64);
-    if (large >= 152)
-        launch_gemm_t<L, 2, 4, 2>(c, d.A, d.sA, d.nr, B, sB, d.nm, d.nch, out, so_m, so_n);
+    if (P.grids * ((P.max_nr() + 31) / 32) * ((P.max_nm() + 63) / 64) >= 152)
+        launch_gemm_t<L, 2, 4, 2>(c, P, field, back);
     else
-        launch_gemm_t<L, 2, 2, 3>(c, d.A, d.sA, d.nr, B, sB, d.nm, d.nch, out, so_m, so_n);
+        launch_gemm_t<L, 2, 2, 3>(c, P, field, back);
 }
 
 template <int L, bool SPEC>
 static void launch_split(Context &c, const SepPlan &P, const double *in)
 {
-    const SepDev &d = P.d;
-    const int n = d.nch * kKC;
-    if (n <= 256) k_sep_split<L, 1, SPEC><<<d.nr, 128, 0, c.stream>>>(d, in);
-    else if (n <= 512) k_sep_split<L, 2, SPEC><<<d.nr, 128, 0, c.stream>>>(d, in);
-    else if (n <= 1024) k_sep_split<L, 4, SPEC><<<d.nr, 128, 0, c.stream>>>(d, in);
-    else k_sep_split<L, 8, SPEC><<<d.nr, 128, 0, c.stream>>>(d, in);
+    const int n = (P.max_nm() + kKC - 1) / kKC * kKC;
+    const dim3 grid(P.max_nr(), P.grids);
+    if (n <= 256) k_sep_split<L, 1, SPEC><<<grid, 128, 0, c.stream>>>(P.a, in);
+    else if (n <= 512) k_sep_split<L, 2, SPEC><<<grid, 128, 0, c.stream>>>(P.a, in);
+    else if (n <= 1024) k_sep_split<L, 4, SPEC><<<grid, 128, 0, c.stream>>>(P.a, in);
+    else k_sep_split<L, 8, SPEC><<<grid, 128, 0, c.stream>>>(P.a, in);
     CUIBM_TRY(cudaGetLastError());
 }
 
@@ -781,24 +846,23 @@ static void split_table(Context &c, const double *src, int rows, int n, int nch,
 
 static void launch_tri(Context &c, const SepPlan &P)
 {
-    const SepDev &d = P.d;
-    const int cb = tri_modes(d.nm, d.nr), nq = kTriThreads / cb, m = (d.nr + nq - 1) / nq;
+    const int nm = P.max_nm(), nr = P.max_nr();
+    const int cb = tri_modes(nm, nr), m = P.tri_rows;
     const size_t smem = (size_t)m * kTriThreads * sizeof(double);
-    const int nb = (d.nm + cb - 1) / cb;
-    if (cb == 8) k_sep_tri<8><<<nb, kTriThreads, smem, c.stream>>>(d);
-    else k_sep_tri<4><<<nb, kTriThreads, smem, c.stream>>>(d);
+    const dim3 grid((nm + cb - 1) / cb, P.grids);
+    if (cb == 8) k_sep_tri<8><<<grid, kTriThreads, smem, c.stream>>>(P.a, m);
+    else k_sep_tri<4><<<grid, kTriThreads, smem, c.stream>>>(P.a, m);
     CUIBM_TRY(cudaGetLastError());
 }
 
 template <int L>
 static void apply_t(Context &c, const SepPlan &P, const double *in, double *out)
 {
-    const SepDev &d = P.d;
     launch_split<L, false>(c, P, in);
-    launch_gemm<L>(c, P, d.B1, d.sB1, d.h, d.nm, 1);
+    launch_gemm<L>(c, P, nullptr, 0);
     launch_tri(c, P);
     launch_split<L, true>(c, P, nullptr);
-    launch_gemm<L>(c, P, d.B2, d.sB2, out, d.sr, d.sm);
+    launch_gemm<L>(c, P, out, 1);
 }
 
 // out = M in: five kernels
@@ -821,65 +885,89 @@ void launch_separable_apply(Context &c, LinearSystem &S, const double *in, doubl
 // centre cell is pinned too and the level agrees to 1e-12.
 constexpr int kLevelMax = 200000;
 
+// The velocity system (I - dt/2 nu L, two grids) has a far smaller condition number, and the
+// diagonally preconditioned iteration is good where it needs few steps.  Its matrix D^-1 A
+// has its spectrum in 1 +- s / (1 + s), s the largest sum of a row's coefficients, so a
+// BiCGSTAB step (two products) gains ((sqrt(1 + 2 s) - 1) / (sqrt(1 + 2 s) + 1))^2; the
+// prediction is 1.2 to 1.3 times the measured count (Re 40: 18 against 14, Re 550: 9
+// against 7).
+static double predicted_velocity_steps(const Context &c, double rtol)
+{
+    const double *t = c.htab.data();
+    const int nx = c.g.nx, ny = c.g.ny;
+    auto largest = [&](const char *a, const char *b, int n) {
+        double m = 0;
+        for (int i = 0; i < n; ++i) m = std::max(m, t[c.hoff.at(a) + i] + t[c.hoff.at(b) + i]);
+        return m;
+    };
+    const double s = std::max(largest("1uE", "1uW", nx - 1) + largest("1uN", "1uS", ny),
+                              largest("1vE", "1vW", nx) + largest("1vN", "1vS", ny - 1));
+    const double q = (std::sqrt(1 + 2 * s) - 1) / (std::sqrt(1 + 2 * s) + 1);
+    return q > 0 ? std::log(2 / rtol) / (2 * std::log(1 / q)) : 0.0;
+}
+constexpr double kVelocitySteps = 5;
+
 static bool separable_applies(const Context &c, const LinearSystem &S)
 {
     const int nx = c.g.nx, ny = c.g.ny;
-    const bool fits = S.which == 2 && S.precond == PC_SMOOTHED_AGGREGATION && c.P.saStructured == -1 &&
-                      c.P.poisson.strength < 0 &&
-                      (c.P.solverType == ST_NAVIERSTOKES || c.P.solverType == ST_LUO) &&
-                      std::min(nx, ny) <= kSepMax && std::max(nx, ny) <= kTriRows;
-    if (!fits || c.P.separable >= 0) return fits && c.P.separable == 1;
-    return c.P.solverType == ST_NAVIERSTOKES ||
-           (S.n < kLevelMax && S.precision == PRECISION_FP64 && c.P.solverPack != 2);
+    if (c.P.separable == 0 || std::min(nx, ny) > kSepMax || std::max(nx, ny) > kTriRows) return false;
+    if (S.which == 2) {
+        if (S.precond != PC_SMOOTHED_AGGREGATION || c.P.saStructured != -1 || c.P.poisson.strength >= 0) return false;
+    } else {
+        if (S.precond != PC_DIAGONAL || (c.P.solverType != ST_NAVIERSTOKES && c.P.solverType != ST_LUO)) return false;
+    }
+    if (c.P.separable == 1) return true;
+    const bool level = c.P.solverType == ST_NAVIERSTOKES ||
+                       (c.P.solverType == ST_LUO && c.g.nP < kLevelMax && c.P.solverPack != 2 &&
+                        c.P.poisson.precision == PRECISION_FP64);
+    return level && (S.which == 2 || predicted_velocity_steps(c, S.rtol) >= kVelocitySteps);
 }
 
-void setup_separable(Context &c, LinearSystem &S)
+// One grid's operator: shift + X + Y with the coefficients towards the next and the
+// previous node (um, dm along the transform, ur, dr along the rows; all of them in the
+// diagonal) and the weights that make X symmetric (wm; wr with them the rows of CG's system)
+struct SepGrid {
+    double shift;
+    std::vector<double> um, dm, wm, ur, dr, wr;
+    int sm, sr, base;
+    std::vector<int> pin_m, pin_r;
+};
+
+// The tables of grid g into P.a.f[k]; false where the eigenvalues do not converge.  cb: the
+// modes a block of k_sep_tri takes (the same for all grids of a launch).
+static bool build_grid(Context &c, SepPlan &P, int g, const SepGrid &G, bool sym, int cb)
 {
-    S.sep = nullptr;
-    if (!separable_applies(c, S)) return;
-    const int nx = c.g.nx, ny = c.g.ny;
-    const bool alongx = nx <= ny;  // the shorter direction is transformed: n_m^2 n_r work
-    SepPlan *P = new SepPlan();
-    S.sep = P;
-    SepDev &d = P->d;
-    P->digits = S.precision == PRECISION_MIXED ? kDigitsMixed : kDigits;
-    const int L = P->digits, nm = alongx ? nx : ny, nr = alongx ? ny : nx;
+    SepDev &d = P.a.f[g];
+    const int L = P.digits, nm = (int)G.um.size(), nr = (int)G.ur.size();
     d.nm = nm;
     d.nr = nr;
-    d.sm = alongx ? 1 : nx;
-    d.sr = alongx ? nx : 1;
+    d.sm = G.sm;
+    d.sr = G.sr;
+    d.base = G.base;
     d.nch = (nm + kKC - 1) / kKC;
-    const double *t = c.htab.data();
-    auto tab = [&](const char *k, int n) { return std::vector<double>(t + c.hoff.at(k), t + c.hoff.at(k) + n); };
-    const std::vector<double> &wm = alongx ? c.gx.width : c.gy.width, &wr = alongx ? c.gy.width : c.gx.width;
-    const std::vector<double> um = tab(alongx ? "2E" : "2N", nm), dm = tab(alongx ? "2W" : "2S", nm);
-    const std::vector<double> ur = tab(alongx ? "2N" : "2E", nr), dr = tab(alongx ? "2S" : "2W", nr);
-
+    d.pins = (int)G.pin_m.size();
     // eigenvalues of D^1/2 X D^-1/2 and the rotations that give its eigenvectors
     std::vector<double> lam(nm), off(nm, 0.0);
-    for (int i = 0; i < nm; ++i) lam[i] = um[i] + dm[i];
-    for (int i = 0; i + 1 < nm; ++i) off[i] = -std::sqrt(um[i] * dm[i + 1]);
+    for (int i = 0; i < nm; ++i) lam[i] = G.um[i] + G.dm[i];
+    for (int i = 0; i + 1 < nm; ++i) off[i] = -std::sqrt(G.um[i] * G.dm[i + 1]);
     std::vector<Sweep> sweeps;
     std::vector<double2> rot;
-    if (!tridiagonal_qr(lam, off, sweeps, rot)) {  // not a grid this can be built on
-        free_separable(S);
-        return;
-    }
-    const int k0 = (int)(std::min_element(lam.begin(), lam.end()) - lam.begin());
-    lam[k0] = 0;  // the constant: exactly the null vector of X
+    if (!tridiagonal_qr(lam, off, sweeps, rot)) return false;
+    // a system with pinned cells is singular without them: the constant is exactly X's null vector
+    const int k0 = d.pins ? (int)(std::min_element(lam.begin(), lam.end()) - lam.begin()) : -1;
+    if (d.pins) lam[k0] = 0;
     double len = 0;
-    for (double w : wm) len += w;
+    for (double w : G.wm) len += w;
     std::vector<double> cm(nm), cr(nr), em(nm), con(nm);
-    const bool sym = S.w != nullptr;  // CG: the system's rows carry the cell areas
     for (int i = 0; i < nm; ++i) {
-        cm[i] = sym ? 1 / std::sqrt(wm[i]) : std::sqrt(wm[i]);
-        em[i] = 1 / std::sqrt(wm[i]);
-        con[i] = std::sqrt(wm[i] / len);
+        cm[i] = sym ? 1 / std::sqrt(G.wm[i]) : std::sqrt(G.wm[i]);
+        em[i] = 1 / std::sqrt(G.wm[i]);
+        con[i] = std::sqrt(G.wm[i] / len);
     }
-    for (int J = 0; J < nr; ++J) cr[J] = sym ? 1 / wr[J] : 1.0;
+    for (int J = 0; J < nr; ++J) cr[J] = sym ? 1 / G.wr[J] : 1.0;
 
     // one allocation for all tables and work arrays
-    const int cb = tri_modes(nm, nr), nq = kTriThreads / cb;
+    const int nq = kTriThreads / cb;
     const size_t n = (size_t)nm * nr, dig = (size_t)d.nch * L * kKC;
     size_t need = 0;
     auto reserve = [&](size_t bytes) {
@@ -892,17 +980,18 @@ void setup_separable(Context &c, LinearSystem &S)
     const size_t oh = reserve(n * 8), ol = reserve(n * 8), oc = reserve(n * 8), oi = reserve(n * 8);
     const size_t oPf = reserve((size_t)nq * nm * 8), oPb = reserve((size_t)nq * nm * 8);
     const size_t ocm = reserve(nm * 8), ocr = reserve(nr * 8), oF0 = reserve(nm * 8), oF1 = reserve(nm * 8);
-    const size_t oG0 = reserve(n * 8), oG1 = reserve(c.l2.pinc >= 0 ? n * 8 : 8), ogm = reserve(nr * 8);
-    CUIBM_TRY(cudaMalloc(&P->block, need));
-    auto D = [&](size_t at) { return reinterpret_cast<double *>(P->block + at); };
-    auto H = [&](size_t at) { return reinterpret_cast<__nv_bfloat16 *>(P->block + at); };
+    const size_t oG0 = reserve(d.pins > 0 ? n * 8 : 8), oG1 = reserve(d.pins > 1 ? n * 8 : 8), ogm = reserve(nr * 8);
+    CUIBM_TRY(cudaMalloc(&P.block[g], need));
+    char *block = P.block[g];
+    auto D = [&](size_t at) { return reinterpret_cast<double *>(block + at); };
+    auto H = [&](size_t at) { return reinterpret_cast<__nv_bfloat16 *>(block + at); };
     auto put = [&](double *dst, const std::vector<double> &v) {
         CUIBM_TRY(cudaMemcpyAsync(dst, v.data(), v.size() * 8, cudaMemcpyHostToDevice, c.stream));
     };
     // set-up scratch, freed at the end
     char *tmp = nullptr;
     const size_t bq = ((size_t)nm * nm * 8 + 255) & ~size_t(255), bs = (sweeps.size() * sizeof(Sweep) + 511) & ~size_t(255),
-                 br = (rot.size() * sizeof(double2) + 511) & ~size_t(255), bv = (size_t)(4 * nm + 4 * nr) * 8;
+                 br = (rot.size() * sizeof(double2) + 511) & ~size_t(255), bv = (size_t)(3 * nm + 2 * nr) * 8;
     CUIBM_TRY(cudaMalloc(&tmp, bq + bs + br + bv));
     struct Freed {
         char *p;
@@ -913,21 +1002,21 @@ void setup_separable(Context &c, LinearSystem &S)
     double2 *rt = reinterpret_cast<double2 *>(tmp + bq + bs);
     double *vl = reinterpret_cast<double *>(tmp + bq + bs + br), *vcon = vl + nm, *vem = vcon + nm, *vur = vem + nm,
            *vdr = vur + nr;
-    CUIBM_TRY(cudaMemcpyAsync(sw, sweeps.data(), sweeps.size() * sizeof(Sweep), cudaMemcpyHostToDevice, c.stream));
-    CUIBM_TRY(cudaMemcpyAsync(rt, rot.data(), rot.size() * sizeof(double2), cudaMemcpyHostToDevice, c.stream));
+    if (!rot.empty()) {
+        CUIBM_TRY(cudaMemcpyAsync(sw, sweeps.data(), sweeps.size() * sizeof(Sweep), cudaMemcpyHostToDevice, c.stream));
+        CUIBM_TRY(cudaMemcpyAsync(rt, rot.data(), rot.size() * sizeof(double2), cudaMemcpyHostToDevice, c.stream));
+    }
     put(vl, lam);
     put(vcon, con);
     put(vem, em);
-    put(vur, ur);
-    put(vdr, dr);
+    put(vur, G.ur);
+    put(vdr, G.dr);
     put(D(ocm), cm);
     put(D(ocr), cr);
-    // rows of Q a block: as many as shared memory holds, a warp at most
-    int W = 32;
-    while (W > 4 && (size_t)nm * W * 8 > 200 * 1024) W /= 2;
-    allow_smem(k_sep_rotate, (size_t)nm * W * 8);
-    k_sep_rotate<<<(nm + W - 1) / W, W, (size_t)nm * W * 8, c.stream>>>(nm, sw, (int)sweeps.size(), rt, Q);
-    k_sep_constant<<<blocks_for(nm), kBlock, 0, c.stream>>>(nm, k0, vcon, Q);
+    const size_t smem = (size_t)nm * kRotWarps * 8;
+    allow_smem(k_sep_rotate, smem);
+    k_sep_rotate<<<(nm + kRotWarps - 1) / kRotWarps, 32 * kRotWarps, smem, c.stream>>>(nm, sw, (int)sweeps.size(), rt, Q);
+    if (d.pins) k_sep_constant<<<blocks_for(nm), kBlock, 0, c.stream>>>(nm, k0, vcon, Q);
     CUIBM_TRY(cudaGetLastError());
     if (L == kDigits) {
         allow_gemm<kDigits>();
@@ -940,9 +1029,9 @@ void setup_separable(Context &c, LinearSystem &S)
     }
     allow_smem(k_sep_tri<8>, 200 * 1024);
     allow_smem(k_sep_tri<4>, 200 * 1024);
-    const double reg = ur[0];
-    k_sep_factor<<<(nm + 31) / 32, 32, 0, c.stream>>>(nm, nr, nq, vur, vdr, vl, k0, reg, D(ol), D(oc), D(oi), D(oPf),
-                                                      D(oPb));
+    const double reg = d.pins ? G.ur[0] : 0.0;
+    k_sep_factor<<<(nm + 31) / 32, 32, 0, c.stream>>>(nm, nr, nq, P.tri_rows, vur, vdr, vl, G.shift, k0, reg, D(ol), D(oc),
+                                                      D(oi), D(oPf), D(oPb));
     CUIBM_TRY(cudaGetLastError());
     d.B1 = H(oB1);
     d.B2 = H(oB2);
@@ -961,75 +1050,128 @@ void setup_separable(Context &c, LinearSystem &S)
     d.k0 = k0;
     d.mean = 1 / std::sqrt(len);
     d.gm = D(ogm);
+    CUIBM_TRY(cudaStreamSynchronize(c.stream));
+    if (!d.pins) return true;
 
     // Pinned cells and the constant.  With B = A0 plus reg on the constant's mode in row 0,
     // A = B + sum_p delta_p e_p e_p^T - reg u mean^T (u one on row 0, mean the average over
     // it), so z = B^-1 r - sum_p q_p G_p + q_m G_m with q_p = delta_p z_p, q_m = reg mean(z)
-    std::vector<int> cell{c.l2.pin0};
-    if (c.l2.pinc >= 0) cell.push_back(c.l2.pinc);
-    d.pins = (int)cell.size();
-    std::vector<std::vector<double>> F(3, std::vector<double>(nm)), G0, q(nm);
-    std::vector<double> qrow(nm), resp((size_t)nm);
+    const int np = d.pins;
+    std::vector<std::vector<double>> F(2, std::vector<double>(nm));
+    std::vector<double> row(nm);
     double *Gp[2] = {D(oG0), D(oG1)}, *Fp[2] = {D(oF0), D(oF1)};
-    int Rp[2] = {0, 0};
-    double delta[2] = {0, 0};
-    std::vector<std::vector<double>> at_pin(3, std::vector<double>(3, 0.0));  // functional a of response b
-    for (int p = 0; p < d.pins; ++p) {
-        const int I = cell[p] % nx, J = cell[p] / nx, m = alongx ? I : J;
-        Rp[p] = alongx ? J : I;
-        delta[p] = um[m] + dm[m] + ur[Rp[p]] + dr[Rp[p]];
-        CUIBM_TRY(cudaMemcpyAsync(qrow.data(), Q + (size_t)m * nm, nm * 8, cudaMemcpyDeviceToHost, c.stream));
+    double delta[2] = {0, 0}, at_pin[3][3] = {};  // functional a of response b
+    for (int p = 0; p < np; ++p) {
+        const int m = G.pin_m[p], R = G.pin_r[p];
+        delta[p] = G.um[m] + G.dm[m] + G.ur[R] + G.dr[R];
+        CUIBM_TRY(cudaMemcpyAsync(row.data(), Q + (size_t)m * nm, nm * 8, cudaMemcpyDeviceToHost, c.stream));
         CUIBM_TRY(cudaStreamSynchronize(c.stream));
-        std::vector<double> rhs(nm);
-        for (int k = 0; k < nm; ++k) {
-            rhs[k] = qrow[k] * std::sqrt(wm[m]);
-            F[p][k] = qrow[k] * em[m];
-        }
+        for (int k = 0; k < nm; ++k) F[p][k] = row[k] * em[m];
+        for (int k = 0; k < nm; ++k) row[k] *= std::sqrt(G.wm[m]);
         put(Fp[p], F[p]);
         CUIBM_TRY(cudaMemsetAsync(d.h, 0, n * 8, c.stream));
-        CUIBM_TRY(cudaMemcpyAsync(d.h + (size_t)Rp[p] * nm, rhs.data(), nm * 8, cudaMemcpyHostToDevice, c.stream));
-        launch_tri(c, *P);
+        put(d.h + (size_t)R * nm, row);
+        launch_tri(c, P);
         CUIBM_TRY(cudaMemcpyAsync(Gp[p], d.h, n * 8, cudaMemcpyDeviceToDevice, c.stream));
         CUIBM_TRY(cudaStreamSynchronize(c.stream));
-        d.R[p] = Rp[p];
+        d.R[p] = R;
         d.F[p] = Fp[p];
         d.G[p] = Gp[p];
     }
     // the constant's response: mode k0 only, u = sqrt(len) there
     CUIBM_TRY(cudaMemsetAsync(d.h, 0, n * 8, c.stream));
-    const double one = std::sqrt(len);
-    CUIBM_TRY(cudaMemcpyAsync(d.h + k0, &one, 8, cudaMemcpyHostToDevice, c.stream));
-    launch_tri(c, *P);
+    put(d.h + k0, std::vector<double>(1, std::sqrt(len)));
+    launch_tri(c, P);
     CUIBM_TRY(cudaMemcpy2DAsync(D(ogm), 8, d.h + k0, (size_t)nm * 8, 8, nr, cudaMemcpyDeviceToDevice, c.stream));
-    std::vector<double> row(nm);
-    for (int b = 0; b <= d.pins; ++b) {  // responses: the pins', then the constant's
-        const double *src = b < d.pins ? Gp[b] : d.h;
-        for (int a = 0; a <= d.pins; ++a) {
-            CUIBM_TRY(cudaMemcpyAsync(row.data(), src + (size_t)(a < d.pins ? Rp[a] : 0) * nm, nm * 8,
+    for (int b = 0; b <= np; ++b) {  // responses: the pins', then the constant's
+        const double *src = b < np ? Gp[b] : d.h;
+        for (int a = 0; a <= np; ++a) {
+            CUIBM_TRY(cudaMemcpyAsync(row.data(), src + (size_t)(a < np ? d.R[a] : 0) * nm, nm * 8,
                                       cudaMemcpyDeviceToHost, c.stream));
             CUIBM_TRY(cudaStreamSynchronize(c.stream));
             double v = 0;
-            if (a < d.pins)
+            if (a < np)
                 for (int k = 0; k < nm; ++k) v += F[a][k] * row[k];
             else
                 v = row[k0] * d.mean;
             at_pin[a][b] = v;
         }
     }
-    const int m = d.pins;
-    for (int a = 0; a <= m; ++a)
-        for (int b = 0; b <= m; ++b) d.K[3 * a + b] = b == m ? -at_pin[a][b] : at_pin[a][b];
-    for (int p = 0; p < m; ++p) d.K[3 * p + p] += 1 / delta[p];
-    d.K[3 * m + m] += 1 / reg;
-    if (!invert3(d.K, m + 1)) throw CudaError("the separable preconditioner's pinned-cell correction is singular");
-    CUIBM_TRY(cudaStreamSynchronize(c.stream));
+    for (int a = 0; a <= np; ++a)
+        for (int b = 0; b <= np; ++b) d.K[3 * a + b] = b == np ? -at_pin[a][b] : at_pin[a][b];
+    for (int p = 0; p < np; ++p) d.K[3 * p + p] += 1 / delta[p];
+    d.K[3 * np + np] += 1 / reg;
+    if (!invert3(d.K, np + 1)) throw CudaError("the separable preconditioner's pinned-cell correction is singular");
+    return true;
+}
+
+void setup_separable(Context &c, LinearSystem &S)
+{
+    S.sep = nullptr;
+    if (!separable_applies(c, S)) return;
+    const int nx = c.g.nx, ny = c.g.ny;
+    const bool alongx = nx <= ny;  // the shorter direction is transformed: n_m^2 n_r work
+    const double *t = c.htab.data();
+    auto tab = [&](const char *k, int n) { return std::vector<double>(t + c.hoff.at(k), t + c.hoff.at(k) + n); };
+    const std::vector<double> &dx = c.gx.width, &dy = c.gy.width;
+    auto between = [](const std::vector<double> &w) {  // face nodes
+        std::vector<double> f(w.size() - 1);
+        for (size_t i = 0; i < f.size(); ++i) f[i] = 0.5 * (w[i] + w[i + 1]);
+        return f;
+    };
+    std::vector<SepGrid> grids;
+    auto add = [&](double shift, int mx, int my, int base, const char *e, const char *w, const char *n, const char *s,
+                   const std::vector<double> &wx, const std::vector<double> &wy) {
+        SepGrid G;
+        G.shift = shift;
+        G.base = base;
+        G.sm = alongx ? 1 : mx;
+        G.sr = alongx ? mx : 1;
+        G.um = alongx ? tab(e, mx) : tab(n, my);
+        G.dm = alongx ? tab(w, mx) : tab(s, my);
+        G.ur = alongx ? tab(n, my) : tab(e, mx);
+        G.dr = alongx ? tab(s, my) : tab(w, mx);
+        G.wm = alongx ? wx : wy;
+        G.wr = alongx ? wy : wx;
+        grids.push_back(G);
+    };
+    if (S.which == 1) {
+        add(1.0, nx - 1, ny, 0, "1uE", "1uW", "1uN", "1uS", between(dx), dy);
+        add(1.0, nx, ny - 1, c.g.nU, "1vE", "1vW", "1vN", "1vS", dx, between(dy));
+    } else {
+        add(0.0, nx, ny, 0, "2E", "2W", "2N", "2S", dx, dy);
+        for (int cell : {c.l2.pin0, c.l2.pinc}) {
+            if (cell < 0) continue;
+            grids[0].pin_m.push_back(alongx ? cell % nx : cell / nx);
+            grids[0].pin_r.push_back(alongx ? cell / nx : cell % nx);
+        }
+    }
+    SepPlan *P = new SepPlan();
+    S.sep = P;
+    P->digits = S.precision == PRECISION_MIXED ? kDigitsMixed : kDigits;
+    int nm = 0, nr = 0;
+    for (const SepGrid &G : grids) {
+        nm = std::max(nm, (int)G.um.size());
+        nr = std::max(nr, (int)G.ur.size());
+    }
+    const int cb = tri_modes(nm, nr), nq = kTriThreads / cb;
+    P->tri_rows = (nr + nq - 1) / nq;
+    for (size_t g = 0; g < grids.size(); ++g) {
+        P->grids = 1;
+        if (!build_grid(c, *P, (int)g, grids[g], S.w != nullptr, cb)) {
+            free_separable(S);
+            return;
+        }
+    }
+    P->grids = (int)grids.size();
 }
 
 void free_separable(LinearSystem &S)
 {
     SepPlan *P = static_cast<SepPlan *>(S.sep);
     if (!P) return;
-    if (P->block) cudaFree(P->block);
+    for (char *b : P->block)
+        if (b) cudaFree(b);
     delete P;
     S.sep = nullptr;
 }
@@ -1049,13 +1191,13 @@ struct SepSolve {
         if (S.which == 1) f(op1(c, S.w));
         else f(op2(c, S.w));
     }
-    int nb() const { return blocks_for(S.n); }
+    int nb() const { return row_blocks(S.n); }
 
     void init() const
     {
         with_op([&](auto A) {
             if (S.krylov == KRYLOV_CG)
-                k_cg_init<decltype(A), 2><<<nb(), kBlock, 0, c.stream>>>(A, S.n, b, S.w, x, S.r, S.z, S.p, S.dinv,
+                k_cg_init<decltype(A), 2><<<blocks_for(S.n), kBlock, 0, c.stream>>>(A, S.n, b, S.w, x, S.r, S.z, S.p, S.dinv,
                                                                         S.partials, S.ks, c.err_word, S.which, 0, 0);
             else
                 k_sep_init<<<nb(), kBlock, 0, c.stream>>>(A, S.n, b, x, S.r, S.partials, S.ks, c.err_word, S.which);
@@ -1081,7 +1223,7 @@ struct SepSolve {
         });
         k_sep_4<<<nb(), kBlock, 0, c.stream>>>(S.n, x, S.r, S.rs, S.p, S.s, S.Ms, S.AMs, S.partials, S.ks, c.err_word,
                                                S.which, first, h, use);
-        k_bicg_5<<<nb(), kBlock, 0, c.stream>>>(S.n, S.p, S.r, S.AMp, S.ks);
+        k_bicg_5<<<blocks_for(S.n), kBlock, 0, c.stream>>>(S.n, S.p, S.r, S.AMp, S.ks);
         CUIBM_TRY(cudaGetLastError());
     }
     void cg(bool first, cudaGraphConditionalHandle h, int use) const
@@ -1091,12 +1233,12 @@ struct SepSolve {
             if (first) {
                 k_sep_cg_1<<<nb(), kBlock, 0, c.stream>>>(A, S.n, S.r, S.z, S.p, S.q, S.partials, S.ks);
             } else {
-                k_cg_rz<<<nb(), kBlock, 0, c.stream>>>(S.n, S.r, S.z, S.partials, S.ks);
-                k_cg_3<<<nb(), kBlock, 0, c.stream>>>(S.n, S.p, S.z, S.ks);
-                k_cg_1<<<nb(), kBlock, 0, c.stream>>>(A, S.n, S.p, S.q, S.partials, S.ks);
+                k_cg_rz<<<blocks_for(S.n), kBlock, 0, c.stream>>>(S.n, S.r, S.z, S.partials, S.ks);
+                k_cg_3<<<blocks_for(S.n), kBlock, 0, c.stream>>>(S.n, S.p, S.z, S.ks);
+                k_cg_1<<<blocks_for(S.n), kBlock, 0, c.stream>>>(A, S.n, S.p, S.q, S.partials, S.ks);
             }
         });
-        k_cg_2<2><<<nb(), kBlock, 0, c.stream>>>(S.n, x, S.r, S.z, S.p, S.q, S.w, S.dinv, S.partials, S.ks, c.err_word,
+        k_cg_2<2><<<blocks_for(S.n), kBlock, 0, c.stream>>>(S.n, x, S.r, S.z, S.p, S.q, S.w, S.dinv, S.partials, S.ks, c.err_word,
                                                  S.which, h, use);
         CUIBM_TRY(cudaGetLastError());
     }
@@ -1214,7 +1356,7 @@ long long separable_body_launches(const LinearSystem &S, int runs)
 double separable_bytes(const LinearSystem &S, int it)
 {
     const SepPlan &P = *static_cast<const SepPlan *>(S.sep);
-    const double n = S.n, nm = P.d.nm, L = P.digits;
+    const double n = S.n, nm = P.a.f[0].nm, L = P.digits;
     const double app = 8 * n * 2 + 2 * 2 * L * (n + nm * nm) + 8 * n * (2 + 3 + 2) + 8 * n * 5;
     const double apps = S.krylov == KRYLOV_CG ? std::max(it, 1) : 1 + 2 * std::max(0.0, it - 0.5);
     return 8 * n * 3 + apps * app;

@@ -1,9 +1,10 @@
-// The pressure system's separable preconditioner (separable.cu).
+// The separable preconditioner of the pressure and velocity systems (separable.cu).
 #pragma once
 #include "solver.h"
 
 namespace cuibm {
 
+constexpr int kRowBlocks = 608;  // blocks of the Krylov kernels there at most (four an SM): S.partials holds 4 sums of each
 void setup_separable(Context &c, LinearSystem &S);  // S.sep stays null where it does not apply
 void launch_separable_apply(Context &c, LinearSystem &S, const double *in, double *out);
 void launch_separable_solve(Context &c, LinearSystem &S, const double *b, double *x, bool in_graph);

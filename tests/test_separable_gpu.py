@@ -1,4 +1,4 @@
-"""The pressure system's separable preconditioner (csrc/separable.cu): pressure solves on
+"""The separable preconditioner (csrc/separable.cu): pressure and velocity solves on
 grids at the edges of its tiles - chunks of 32 terms, product tiles of 32 x 32 and 32 x 64,
 the splitting kernels' 256, 512 and 1024 places, the tridiagonal blocks of 4 and 8 modes -
 along both transform directions, uniform and stretched, for both Krylov methods and
@@ -19,7 +19,7 @@ pytestmark = pytest.mark.gpu
 TOL = 1e-12
 
 
-def box(folder, nx, ny, ratio, krylov, precision, tol=TOL):
+def box(folder, nx, ny, ratio, krylov, precision, tol=TOL, nu=0.01):
     """nx x ny cells: uniform, or stretched away from the first corner (the counts of a
     stretched axis follow from its length)."""
     def axis(name, n):
@@ -28,8 +28,8 @@ def box(folder, nx, ny, ratio, krylov, precision, tol=TOL):
         return cases.axis(name, 0.0, 0.01, [(0.01 * (ratio ** (n + 0.5) - 1) / (ratio - 1), ratio)])
     sim = {"type": "simulation", "dt": 0.003, "nt": 10, "nsave": 10, "SolverType": "NAVIER_STOKES_SOLVER",
            "linearSolvers": cases.solvers("DIAGONAL", tol, "SMOOTHED_AGGREGATION", tol, pois_krylov=krylov,
-                                          precision=precision)}
-    flow = [{"type": "flow", "nu": 0.01, "initialVelocity": [0.0, 0.0], "initialPerturbation": [0.0, 0.0],
+                                          vel_krylov=krylov, precision=precision)}
+    flow = [{"type": "flow", "nu": nu, "initialVelocity": [0.0, 0.0], "initialPerturbation": [0.0, 0.0],
              "boundaryConditions": cases.bcs((0, 0), (0, 0), (0, 0), (1.0, 0))}]
     return cases.write_case(folder, [sim], flow, [axis("x", nx), axis("y", ny)], [])
 
@@ -41,13 +41,15 @@ def solver(folder, args=()):
     return s
 
 
-def check(s, b, p0):
-    n = s.info.numP
-    s.set("rhs2", b)
-    s.set("p", p0)
-    s.run("solve_poisson")
-    p = s.get("p")
-    A = sp.coo_matrix((s.matrix(2)[2], s.matrix(2)[:2]), shape=(n, n)).tocsr()
+def check(s, b, p0, system=2):
+    n, rhs, sol, op = ((s.info.numP, "rhs2", "p", "solve_poisson") if system == 2 else
+                       (s.info.numUV, "rhs1", "uhat", "solve_velocity"))
+    s.set(rhs, b)
+    s.set(sol, p0)
+    s.run(op)
+    p = s.get(sol)
+    r, c, v = s.matrix(system)
+    A = sp.coo_matrix((v, (r, c)), shape=(n, n)).tocsr()
     floor = np.linalg.norm(abs(A) @ np.abs(p) + np.abs(b))
     res = np.linalg.norm(b - A @ p)
     assert res <= TOL * np.linalg.norm(b) + 40 * np.finfo(float).eps * floor, (res, np.linalg.norm(b), floor)
@@ -69,6 +71,17 @@ def test_solves_meet_the_residual_bound(tmp_path, nx, ny, ratio, krylov, precisi
         for b in (rng.standard_normal(i.numP), np.repeat(rng.standard_normal(ny), nx)):
             check(s, b, rng.standard_normal(i.numP))
             assert s.iterations()[1] <= 3  # the inverse to rounding (mixed precision: to 2^-31)
+        check(s, rng.standard_normal(i.numUV), rng.standard_normal(i.numUV), system=1)
+
+
+@pytest.mark.parametrize("nx,ny,ratio", [(3, 3, 1.0), (33, 32, 1.0), (65, 31, 1.03), (120, 257, 1.0), (514, 130, 1.0)])
+@pytest.mark.parametrize("krylov,precision", [("BICGSTAB", None), ("CG", None), ("BICGSTAB", "MIXED")])
+def test_velocity_solves_meet_the_residual_bound(tmp_path, nx, ny, ratio, krylov, precision):
+    """nu large enough that the diagonal preconditioner would take tens of iterations."""
+    with solver(box(str(tmp_path / "c"), nx, ny, ratio, krylov, precision, nu=1.0)) as s:
+        rng = np.random.default_rng(nx + ny)
+        check(s, rng.standard_normal(s.info.numUV), rng.standard_normal(s.info.numUV), system=1)
+        assert s.iterations()[0] <= 2
 
 
 def test_agrees_with_smoothed_aggregation_and_runs_in_steps(tmp_path):
