@@ -84,6 +84,12 @@ struct SepPlan {
     int grids = 1;
     int digits = kDigits;
     char *block[2] = {nullptr, nullptr};  // one device allocation a grid
+    // rows that a body patches (a fixed body's): how many, their cells, each cell's place in
+    // that list (or -1), the inverse of the capacitance matrix, and work arrays
+    int patched = 0;
+    int *prow = nullptr, *pidx = nullptr;
+    double *cap = nullptr, *gap = nullptr, *q = nullptr, *y = nullptr, *rin = nullptr;
+    char *pblock = nullptr;
     int tri_rows = 0;  // neighbouring rows a thread of k_sep_tri takes
     int max_nm() const { return grids > 1 ? std::max(a.f[0].nm, a.f[1].nm) : a.f[0].nm; }
     int max_nr() const { return grids > 1 ? std::max(a.f[0].nr, a.f[1].nr) : a.f[0].nr; }
@@ -865,12 +871,176 @@ static void apply_t(Context &c, const SepPlan &P, const double *in, double *out)
     launch_gemm<L>(c, P, out, 1);
 }
 
-// out = M in: five kernels
+static void apply_grid(Context &c, const SepPlan &P, const double *in, double *out)
+{
+    if (P.digits == kDigits) apply_t<kDigits>(c, P, in, out);
+    else apply_t<kDigitsMixed>(c, P, in, out);
+}
+
+// ---- rows that a body patches -----------------------------------------------------------
+// With A = A0 + E P (E the m patched rows' unit vectors, P what those rows add to A0's),
+// A^-1 r = A0^-1 (r - E q) where (I + P A0^-1 E) q = P A0^-1 r.  The m x m capacitance matrix
+// is inverted once, at set-up, for a body whose rows stay; an application then is two of
+// A0^-1 and a dense m x m product.
+struct RowGap {  // (P y)_k at the patched cell i: its row less the row that A0 has there
+    Lhs2Coef full, plain;
+    Grid g;
+};
+__global__ void k_sep_gap(RowGap A, int m, const int *__restrict__ row, const double *__restrict__ y, double *gap)
+{
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < m) gap[k] = lhs2_row(A.full, A.g, row[k], y) - lhs2_row(A.plain, A.g, row[k], y);
+}
+
+// q = cap gap, a warp a row
+__global__ void k_sep_cap(int m, const double *__restrict__ cap, const double *__restrict__ gap, double *q)
+{
+    const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (k >= m) return;
+    double v = 0;
+#pragma unroll 4
+    for (int j = lane; j < m; j += 32) v += cap[(size_t)k * m + j] * gap[j];
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane == 0) q[k] = v;
+}
+
+__global__ void k_sep_less(int n, const double *__restrict__ in, const int *__restrict__ idx,
+                           const double *__restrict__ q, double *out)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) out[i] = in[i] - (idx[i] >= 0 ? q[idx[i]] : 0.0);
+}
+
+// set-up: a unit vector at cell `at`, the one before it cleared; a column of the capacitance
+// matrix beside the identity; Gauss-Jordan with row exchanges on [m][2 m]
+__global__ void k_sep_unit(double *v, int before, int at)
+{
+    if (before >= 0) v[before] = 0;
+    v[at] = 1;
+}
+__global__ void k_sep_column(int m, int j, const double *__restrict__ gap, double *W)
+{
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= m) return;
+    W[(size_t)k * 2 * m + j] = gap[k] + (k == j ? 1.0 : 0.0);
+    W[(size_t)k * 2 * m + m + j] = k == j ? 1.0 : 0.0;
+}
+__global__ void __launch_bounds__(256) k_sep_pivot(int m, int k, double *W, double *fac, int *bad)
+{
+    __shared__ double big[256];
+    __shared__ int who[256];
+    double v = -1;
+    int p = k;
+    for (int i = k + threadIdx.x; i < m; i += 256) {
+        const double a = fabs(W[(size_t)i * 2 * m + k]);
+        if (a > v) v = a, p = i;
+    }
+    big[threadIdx.x] = v;
+    who[threadIdx.x] = p;
+    __syncthreads();
+    for (int o = 128; o > 0; o >>= 1) {
+        if (threadIdx.x < o && big[threadIdx.x + o] > big[threadIdx.x]) {
+            big[threadIdx.x] = big[threadIdx.x + o];
+            who[threadIdx.x] = who[threadIdx.x + o];
+        }
+        __syncthreads();
+    }
+    p = who[0];
+    const double piv = W[(size_t)p * 2 * m + k];
+    __syncthreads();
+    if (!(fabs(piv) > 1e-300)) {  // zero or not a number
+        if (threadIdx.x == 0) *bad = 1;
+        return;
+    }
+    for (int j = threadIdx.x; j < 2 * m; j += 256) {
+        const double a = W[(size_t)p * 2 * m + j];
+        if (p != k) W[(size_t)p * 2 * m + j] = W[(size_t)k * 2 * m + j];
+        W[(size_t)k * 2 * m + j] = a / piv;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < m; i += 256) fac[i] = i == k ? 0.0 : W[(size_t)i * 2 * m + k];
+}
+__global__ void k_sep_eliminate(int m, int k, double *W, const double *__restrict__ fac)
+{
+    const int j = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y;
+    if (j < 2 * m && i != k) W[(size_t)i * 2 * m + j] -= fac[i] * W[(size_t)k * 2 * m + j];
+}
+
+constexpr int kPatchMax = 2048;  // patched rows: the capacitance matrix is 8 m^2 bytes, its set-up m applications
+
+// out = M in: five kernels, or thirteen with patched rows
 void launch_separable_apply(Context &c, LinearSystem &S, const double *in, double *out)
 {
     const SepPlan &P = *static_cast<const SepPlan *>(S.sep);
-    if (P.digits == kDigits) apply_t<kDigits>(c, P, in, out);
-    else apply_t<kDigitsMixed>(c, P, in, out);
+    if (!P.patched) {
+        apply_grid(c, P, in, out);
+        return;
+    }
+    apply_grid(c, P, in, P.y);
+    RowGap A{c.l2, c.l2, c.g};
+    A.plain.patch = RowPatch{};
+    k_sep_gap<<<blocks_for(P.patched), kBlock, 0, c.stream>>>(A, P.patched, P.prow, P.y, P.gap);
+    k_sep_cap<<<blocks_for(32L * P.patched), kBlock, 0, c.stream>>>(P.patched, P.cap, P.gap, P.q);
+    k_sep_less<<<blocks_for(S.n), kBlock, 0, c.stream>>>(S.n, in, P.pidx, P.q, P.rin);
+    CUIBM_TRY(cudaGetLastError());
+    apply_grid(c, P, P.rin, out);
+}
+
+// The capacitance matrix of a fixed body's patched rows and its inverse.  False where it
+// cannot be inverted or the body has too many rows for it.
+static bool build_patch(Context &c, LinearSystem &S, const std::vector<int> &pid)
+{
+    SepPlan &P = *static_cast<SepPlan *>(S.sep);
+    std::vector<int> rows, idx(S.n, -1);
+    for (int i = 0; i < S.n; ++i)
+        if (pid[i] >= 0) {
+            idx[i] = (int)rows.size();
+            rows.push_back(i);
+        }
+    const int m = (int)rows.size();
+    if (m == 0) return true;
+    if (m > kPatchMax) return false;
+    const size_t n = S.n, w = (size_t)2 * m * m;
+    const size_t bytes = (2 * n + (size_t)m * m + 2 * (size_t)m) * 8 + (n + (size_t)m) * 4;
+    CUIBM_TRY(cudaMalloc(&P.pblock, bytes));
+    P.y = reinterpret_cast<double *>(P.pblock);
+    P.rin = P.y + n;
+    P.cap = P.rin + n;
+    P.gap = P.cap + (size_t)m * m;
+    P.q = P.gap + m;
+    P.pidx = reinterpret_cast<int *>(P.q + m);
+    P.prow = P.pidx + n;
+    CUIBM_TRY(cudaMemcpyAsync(P.pidx, idx.data(), n * 4, cudaMemcpyHostToDevice, c.stream));
+    CUIBM_TRY(cudaMemcpyAsync(P.prow, rows.data(), m * 4, cudaMemcpyHostToDevice, c.stream));
+    char *tmp = nullptr;
+    CUIBM_TRY(cudaMalloc(&tmp, (w + m) * 8 + 256));
+    struct Freed {
+        char *p;
+        ~Freed() { cudaFree(p); }
+    } freed{tmp};
+    double *W = reinterpret_cast<double *>(tmp), *fac = W + w;
+    int *bad = reinterpret_cast<int *>(fac + m), hbad = 0;
+    CUIBM_TRY(cudaMemsetAsync(bad, 0, 4, c.stream));
+    CUIBM_TRY(cudaMemsetAsync(P.rin, 0, n * 8, c.stream));
+    RowGap A{c.l2, c.l2, c.g};
+    A.plain.patch = RowPatch{};
+    for (int j = 0; j < m; ++j) {
+        k_sep_unit<<<1, 1, 0, c.stream>>>(P.rin, j ? rows[j - 1] : -1, rows[j]);
+        apply_grid(c, P, P.rin, P.y);
+        k_sep_gap<<<blocks_for(m), kBlock, 0, c.stream>>>(A, m, P.prow, P.y, P.gap);
+        k_sep_column<<<blocks_for(m), kBlock, 0, c.stream>>>(m, j, P.gap, W);
+    }
+    for (int k = 0; k < m; ++k) {
+        k_sep_pivot<<<1, 256, 0, c.stream>>>(m, k, W, fac, bad);
+        k_sep_eliminate<<<dim3(blocks_for(2L * m), m), kBlock, 0, c.stream>>>(m, k, W, fac);
+    }
+    CUIBM_TRY(cudaGetLastError());
+    CUIBM_TRY(cudaMemcpy2DAsync(P.cap, (size_t)m * 8, W + m, (size_t)2 * m * 8, (size_t)m * 8, m,
+                                cudaMemcpyDeviceToDevice, c.stream));
+    CUIBM_TRY(cudaMemcpyAsync(&hbad, bad, 4, cudaMemcpyDeviceToHost, c.stream));
+    CUIBM_TRY(cudaStreamSynchronize(c.stream));
+    P.patched = m;
+    return !hbad;
 }
 
 // Where the separable preconditioner takes the place of the smoothed-aggregation cycle: the
@@ -912,12 +1082,15 @@ static bool separable_applies(const Context &c, const LinearSystem &S)
     const int nx = c.g.nx, ny = c.g.ny;
     if (c.P.separable == 0 || std::min(nx, ny) > kSepMax || std::max(nx, ny) > kTriRows) return false;
     if (S.which == 2) {
-        if (S.precond != PC_SMOOTHED_AGGREGATION || c.P.saStructured != -1 || c.P.poisson.strength >= 0) return false;
+        // the embedded method's rows change with its body
+        if (S.precond != PC_SMOOTHED_AGGREGATION || c.P.saStructured != -1 || c.P.poisson.strength >= 0 ||
+            c.P.solverType == ST_OSC)
+            return false;
     } else {
         if (S.precond != PC_DIAGONAL || (c.P.solverType != ST_NAVIERSTOKES && c.P.solverType != ST_LUO)) return false;
     }
     if (c.P.separable == 1) return true;
-    const bool level = c.P.solverType == ST_NAVIERSTOKES ||
+    const bool level = c.P.solverType == ST_NAVIERSTOKES || c.P.solverType == ST_FADLUN ||
                        (c.P.solverType == ST_LUO && c.g.nP < kLevelMax && c.P.solverPack != 2 &&
                         c.P.poisson.precision == PRECISION_FP64);
     return level && (S.which == 2 || predicted_velocity_steps(c, S.rtol) >= kVelocitySteps);
@@ -1164,12 +1337,14 @@ void setup_separable(Context &c, LinearSystem &S)
         }
     }
     P->grids = (int)grids.size();
+    if (S.which == 2 && c.l2.patch.pid && !build_patch(c, S, c.fadlun.pid2)) free_separable(S);
 }
 
 void free_separable(LinearSystem &S)
 {
     SepPlan *P = static_cast<SepPlan *>(S.sep);
     if (!P) return;
+    if (P->pblock) cudaFree(P->pblock);
     for (char *b : P->block)
         if (b) cudaFree(b);
     delete P;

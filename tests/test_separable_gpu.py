@@ -109,3 +109,15 @@ def test_zero_and_non_finite_right_hand_sides(tmp_path):
             s.run("solve_poisson")
         assert e.value.status == cb.ERR_NAN
         check(s, np.random.default_rng(1).standard_normal(n), np.zeros(n))  # and is usable again
+
+
+@pytest.mark.parametrize("h,points,precision", [(0.05, 48, None), (0.05, 48, "MIXED"), (0.021, 150, None)])
+def test_patched_rows_of_a_fixed_body(tmp_path, h, points, precision):
+    """The modified Fadlun method's rows at the body: the capacitance matrix makes the
+    preconditioner the patched operator's inverse, so one or two iterations are left."""
+    f = cases.cylinder(str(tmp_path / "c"), h=h, ratio=1.1, extent=3.0, core=0.6, points=points, nu=0.025, dt=0.01,
+                       nt=10, vel_tol=TOL, pois_tol=TOL, method="FADLUN", precision=precision)
+    with solver(f) as s:
+        rng = np.random.default_rng(points)
+        check(s, rng.standard_normal(s.info.numP), rng.standard_normal(s.info.numP))
+        assert s.iterations()[1] <= 3
