@@ -134,20 +134,13 @@ __device__ __forceinline__ long long block_max(long long v)
     return v;
 }
 
-// A row of n values (value(m)) to digits: [chunk][digit][kKC], zero from n on to the end
-// of the last chunk.  A thread takes pairs of neighbours, NP of them, kept in registers
-// between the search for the largest and the splitting.  Returns the row's scale.
-template <int L, int NP, class Value>
-__device__ __forceinline__ double split_row(int n, int nch, __nv_bfloat16 *out, const Value &value)
+// A row of n values to digits: [chunk][digit][kKC], zero from n on to the end of the last
+// chunk.  A thread holds pairs of neighbours, NP of them (places 2 (thread + q blockDim) and
+// the next; zero from n on).  Returns the row's scale.
+template <int L, int NP>
+__device__ __forceinline__ double split_values(int n, int nch, __nv_bfloat16 *out, const double (&v)[2 * NP])
 {
-    double v[2 * NP];
     long long mx = 0;
-#pragma unroll
-    for (int q = 0; q < NP; ++q) {
-        const int m = 2 * (threadIdx.x + q * blockDim.x);
-        v[2 * q] = m < n ? value(m) : 0.0;
-        v[2 * q + 1] = m + 1 < n ? value(m + 1) : 0.0;
-    }
 #pragma unroll
     for (int q = 0; q < 2 * NP; ++q) mx = max(mx, __double_as_longlong(fabs(v[q])));
     mx = block_max(mx);
@@ -169,6 +162,19 @@ __device__ __forceinline__ double split_row(int n, int nch, __nv_bfloat16 *out, 
     return finite ? pow2(e) : __longlong_as_double(0x7ff8000000000000ll);
 }
 
+template <int L, int NP, class Value>
+__device__ __forceinline__ double split_row(int n, int nch, __nv_bfloat16 *out, const Value &value)
+{
+    double v[2 * NP];
+#pragma unroll
+    for (int q = 0; q < NP; ++q) {
+        const int m = 2 * (threadIdx.x + q * blockDim.x);
+        v[2 * q] = m < n ? value(m) : 0.0;
+        v[2 * q + 1] = m + 1 < n ? value(m + 1) : 0.0;
+    }
+    return split_values<L, NP>(n, nch, out, v);
+}
+
 // rows of a table: src[r ld_r + m ld_m], the scale of row r times 2^-50 and extra[r]
 template <int L, int NP>
 __global__ void k_sep_split_table(const double *__restrict__ src, int n, int nch, int ld_r, int ld_m,
@@ -180,17 +186,22 @@ __global__ void k_sep_split_table(const double *__restrict__ src, int n, int nch
     if (threadIdx.x == 0) scale[r] = s * pow2(-50) * (extra ? extra[r] : 1.0);
 }
 
-__device__ __forceinline__ double block_sum(double v)
+// both sums over the block, in every thread
+__device__ __forceinline__ void block_sums(double &a, double &b)
 {
-    __shared__ double sh[32];
+    __shared__ double2 sh[32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    for (int o = 16; o > 0; o >>= 1) {
+        a += __shfl_xor_sync(0xffffffffu, a, o);
+        b += __shfl_xor_sync(0xffffffffu, b, o);
+    }
+    if (lane == 0) sh[w] = make_double2(a, b);
     __syncthreads();
-    if (lane == 0) sh[w] = v;
-    __syncthreads();
-    v = 0;
-    for (int k = 0; k < nw; ++k) v += sh[k];
-    return v;
+    a = b = 0;
+    for (int k = 0; k < nw; ++k) {
+        a += sh[k].x;
+        b += sh[k].y;
+    }
 }
 
 // One grid row to digits, a block a row.  SPEC false: a field (times the scaling that
@@ -215,25 +226,38 @@ __global__ void __launch_bounds__(128) k_sep_split(const __grid_constant__ SepAr
             if (threadIdx.x == 0) d.sA[R] = s;
             return;
         }
-        // q = K^-1 (values of z at the pinned cells, mean of row 0), the same in every block
-        double f[3] = {0, 0, 0}, q[3] = {0, 0, 0};
-        for (int p = 0; p < d.pins; ++p) {
-            double v = 0;
-            const double *at = d.h + (size_t)d.R[p] * n;
-            for (int k = threadIdx.x; k < n; k += blockDim.x) v += d.F[p][k] * at[k];
-            f[p] = block_sum(v);
+        // q = K^-1 (values of z at the pinned cells, mean of row 0), the same in every block;
+        // both sums in one pass, with the row's own loads in flight
+        const bool two = d.pins > 1;
+        const double *g0 = d.G[0] + (size_t)R * n, *g1 = two ? d.G[1] + (size_t)R * n : g0;
+        double own[2 * NP], r0[2 * NP], r1[2 * NP], f0 = 0, f1 = 0;
+#pragma unroll
+        for (int u = 0; u < 2 * NP; ++u) {
+            const int m = 2 * (threadIdx.x + (u >> 1) * blockDim.x) + (u & 1);
+            own[u] = m < n ? row[m] : 0.0;
+            r0[u] = m < n ? g0[m] : 0.0;
+            r1[u] = m < n && two ? g1[m] : 0.0;
         }
-        const int nq = d.pins + 1;
-        f[d.pins] = d.h[d.k0] * d.mean;
-        for (int a = 0; a < nq; ++a)
-            for (int b = 0; b < nq; ++b) q[a] += d.K[3 * a + b] * f[b];
-        const double qm = q[d.pins] * d.gm[R];
-        const double *g0 = d.G[0] + (size_t)R * n, *g1 = d.pins > 1 ? d.G[1] + (size_t)R * n : nullptr;
-        s = split_row<L, NP>(n, d.nch, out, [&](int m) {
-            double v = row[m] - q[0] * g0[m];
-            if (g1) v -= q[1] * g1[m];
-            return m == d.k0 ? v + qm : v;
-        });
+        const double *h0 = d.h + (size_t)d.R[0] * n, *h1 = d.h + (size_t)d.R[two] * n;
+        const double *F0 = d.F[0], *F1 = d.F[two];
+        for (int k = threadIdx.x; k < n; k += blockDim.x) {
+            f0 += F0[k] * h0[k];
+            f1 += F1[k] * h1[k];
+        }
+        const double fm = d.h[d.k0] * d.mean, gm = d.gm[R];
+        block_sums(f0, f1);
+        // f = (f0, f1, fm), without f1 for one pinned cell
+        const double a1 = two ? f1 : fm, a2 = two ? fm : 0.0;
+        const double q0 = d.K[0] * f0 + d.K[1] * a1 + d.K[2] * a2, q1 = d.K[3] * f0 + d.K[4] * a1 + d.K[5] * a2,
+                     q2 = d.K[6] * f0 + d.K[7] * a1 + d.K[8] * a2;
+        const double qm = (two ? q2 : q1) * gm, qg = two ? q1 : 0.0;
+#pragma unroll
+        for (int u = 0; u < 2 * NP; ++u) {
+            const int m = 2 * (threadIdx.x + (u >> 1) * blockDim.x) + (u & 1);
+            own[u] -= q0 * r0[u] + qg * r1[u];
+            if (m == d.k0) own[u] += qm;
+        }
+        s = split_values<L, NP>(n, d.nch, out, own);
     }
     if (threadIdx.x == 0) d.sA[R] = s;
 }
@@ -405,24 +429,61 @@ __device__ __forceinline__ double tri_scan(double end, double prod, bool up, dou
     return in;
 }
 
-template <int CB>
+// M: rows a thread holds in registers, every load of the kernel issued at its start (0: any
+// number, the rows in shared memory and the tables read as they are needed).  512 x 512: 15
+// us with the tables read in four rounds.
+template <int CB, int M>
 __global__ void __launch_bounds__(kTriThreads) k_sep_tri(const __grid_constant__ SepArgs args, int m)
 {
     const SepDev &d = args.f[blockIdx.y];
-    extern __shared__ double row[];  // [m][thread]: r, then inv d
+    extern __shared__ double row[];  // M = 0: [m][thread]: r, then inv d
     __shared__ double se[2 * kTriThreads], sp[2 * kTriThreads];
     const int tid = threadIdx.x, n = d.nm;
     const int k = blockIdx.x * CB + tid % CB, q = tid / CB;
     const int J0 = min(q * m, d.nr), J1 = min(J0 + m, d.nr), cnt = k < n ? J1 - J0 : 0;
     const size_t at = (size_t)J0 * n + k;
+    const double pf = k < n ? d.Pf[(size_t)q * n + k] : 0.0, pb = k < n ? d.Pb[(size_t)q * n + k] : 0.0;
     double x = 0;
+    if (M > 0) {
+        double r[M ? M : 1], l[M ? M : 1], iv[M ? M : 1], cc[M ? M : 1];
+#pragma unroll
+        for (int t = 0; t < M; ++t) {
+            const bool on = t < cnt;
+            const size_t j = at + (size_t)t * n;
+            r[t] = on ? d.h[j] : 0.0;
+            l[t] = on ? d.l[j] : 0.0;
+            iv[t] = on ? d.inv[j] : 0.0;
+            cc[t] = on ? d.c[j] : 0.0;
+        }
+#pragma unroll
+        for (int t = 0; t < M; ++t)
+            if (t < cnt) x = r[t] + l[t] * x;
+        x = tri_scan<CB>(x, pf, true, se, sp);
+#pragma unroll
+        for (int t = 0; t < M; ++t) {
+            x = r[t] + l[t] * x;
+            r[t] = x * iv[t];
+        }
+        x = 0;
+#pragma unroll
+        for (int t = M - 1; t >= 0; --t)
+            if (t < cnt) x = r[t] + cc[t] * x;
+        x = tri_scan<CB>(x, pb, false, se, sp);
+#pragma unroll
+        for (int t = M - 1; t >= 0; --t)
+            if (t < cnt) {
+                x = r[t] + cc[t] * x;
+                d.h[at + (size_t)t * n] = x;
+            }
+        return;
+    }
 #pragma unroll 4
     for (int t = 0; t < cnt; ++t) {
         const double r = d.h[at + (size_t)t * n];
         row[t * kTriThreads + tid] = r;
         x = r + d.l[at + (size_t)t * n] * x;
     }
-    x = tri_scan<CB>(x, k < n ? d.Pf[(size_t)q * n + k] : 0.0, true, se, sp);
+    x = tri_scan<CB>(x, pf, true, se, sp);
 #pragma unroll 4
     for (int t = 0; t < cnt; ++t) {
         x = row[t * kTriThreads + tid] + d.l[at + (size_t)t * n] * x;
@@ -431,7 +492,7 @@ __global__ void __launch_bounds__(kTriThreads) k_sep_tri(const __grid_constant__
     x = 0;
 #pragma unroll 4
     for (int t = cnt - 1; t >= 0; --t) x = row[t * kTriThreads + tid] + d.c[at + (size_t)t * n] * x;
-    x = tri_scan<CB>(x, k < n ? d.Pb[(size_t)q * n + k] : 0.0, false, se, sp);
+    x = tri_scan<CB>(x, pb, false, se, sp);
 #pragma unroll 4
     for (int t = cnt - 1; t >= 0; --t) {
         x = row[t * kTriThreads + tid] + d.c[at + (size_t)t * n] * x;
@@ -522,6 +583,49 @@ __global__ void k_sep_constant(int n, int k0, const double *__restrict__ v, doub
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) Q[(size_t)i * n + k0] = v[i];
 }
+
+// ---- the operators with their stored diagonal --------------------------------------------
+// five FP64 operations a row instead of nine (the Krylov kernels are FP64-issue bound)
+struct StoredOp2 {
+    Lhs2Coef c;
+    const double *diag, *w;
+    int nx, ny;
+    template <class X>
+    __device__ __forceinline__ double row(int i, const X &x) const
+    {
+        double y;
+        const int k = c.patch.pid ? c.patch.pid[i] : -1;
+        if (k >= 0) {
+            y = patch_row(c.patch, k, x(i), x);
+        } else {
+            const int J = i / nx, I = i - J * nx;
+            y = diag[i] * x(i);
+            if (I != nx - 1) y -= c.E[I] * x(i + 1);
+            if (I != 0) y -= c.W[I] * x(i - 1);
+            if (J != ny - 1) y -= c.N[J] * x(i + nx);
+            if (J != 0) y -= c.S[J] * x(i - nx);
+        }
+        return w ? w[i] * y : y;
+    }
+};
+struct StoredOp1 {  // without patched rows or row scales (the plain and external methods)
+    Lhs1Coef c;
+    const double *diag, *w;
+    int nx, ny, nU;
+    template <class X>
+    __device__ __forceinline__ double row(int i, const X &x) const
+    {
+        const bool u = i < nU;
+        const int n = u ? nx - 1 : nx, m = u ? ny : ny - 1, k = u ? i : i - nU, J = k / n, I = k - J * n;
+        const double *E = u ? c.uE : c.vE, *W = u ? c.uW : c.vW, *N = u ? c.uN : c.vN, *S = u ? c.uS : c.vS;
+        double y = diag[i] * x(i);
+        if (I != n - 1) y -= E[I] * x(i + 1);
+        if (I != 0) y -= W[I] * x(i - 1);
+        if (J != m - 1) y -= N[J] * x(i + n);
+        if (J != 0) y -= S[J] * x(i - n);
+        return w ? w[i] * y : y;
+    }
+};
 
 // ---- Krylov kernels ---------------------------------------------------------------------
 // The rows of a grid of at most kRowBlocks blocks, and its sums: a block's partial sums go
@@ -854,10 +958,11 @@ static void launch_tri(Context &c, const SepPlan &P)
 {
     const int nm = P.max_nm(), nr = P.max_nr();
     const int cb = tri_modes(nm, nr), m = P.tri_rows;
-    const size_t smem = (size_t)m * kTriThreads * sizeof(double);
     const dim3 grid((nm + cb - 1) / cb, P.grids);
-    if (cb == 8) k_sep_tri<8><<<grid, kTriThreads, smem, c.stream>>>(P.a, m);
-    else k_sep_tri<4><<<grid, kTriThreads, smem, c.stream>>>(P.a, m);
+    auto go = [&](auto *fn, size_t smem) { fn<<<grid, kTriThreads, smem, c.stream>>>(P.a, m); };
+    const size_t rows = (size_t)m * kTriThreads * sizeof(double);
+    if (cb == 8) m <= 4 ? go(k_sep_tri<8, 4>, 0) : m <= 8 ? go(k_sep_tri<8, 8>, 0) : m <= 16 ? go(k_sep_tri<8, 16>, 0) : go(k_sep_tri<8, 0>, rows);
+    else m <= 2 ? go(k_sep_tri<4, 2>, 0) : m <= 4 ? go(k_sep_tri<4, 4>, 0) : m <= 8 ? go(k_sep_tri<4, 8>, 0) : go(k_sep_tri<4, 0>, rows);
     CUIBM_TRY(cudaGetLastError());
 }
 
@@ -1200,8 +1305,8 @@ static bool build_grid(Context &c, SepPlan &P, int g, const SepGrid &G, bool sym
         split_table<kDigitsMixed>(c, Q, nm, nm, d.nch, 1, nm, nullptr, H(oB1), D(osB1));
         split_table<kDigitsMixed>(c, Q, nm, nm, d.nch, nm, 1, vem, H(oB2), D(osB2));
     }
-    allow_smem(k_sep_tri<8>, 200 * 1024);
-    allow_smem(k_sep_tri<4>, 200 * 1024);
+    allow_smem(k_sep_tri<8, 0>, 200 * 1024);
+    allow_smem(k_sep_tri<4, 0>, 200 * 1024);
     const double reg = d.pins ? G.ur[0] : 0.0;
     k_sep_factor<<<(nm + 31) / 32, 32, 0, c.stream>>>(nm, nr, nq, P.tri_rows, vur, vdr, vl, G.shift, k0, reg, D(ol), D(oc),
                                                       D(oi), D(oPf), D(oPb));
@@ -1281,7 +1386,7 @@ static bool build_grid(Context &c, SepPlan &P, int g, const SepGrid &G, bool sym
 void setup_separable(Context &c, LinearSystem &S)
 {
     S.sep = nullptr;
-    if (!separable_applies(c, S)) return;
+    if (!separable_applies(c, S) || !S.diag) return;  // (the stored diagonal comes with the persistent solver)
     const int nx = c.g.nx, ny = c.g.ny;
     const bool alongx = nx <= ny;  // the shorter direction is transformed: n_m^2 n_r work
     const double *t = c.htab.data();
@@ -1363,8 +1468,8 @@ struct SepSolve {
     template <class F>
     void with_op(const F &f) const
     {
-        if (S.which == 1) f(op1(c, S.w));
-        else f(op2(c, S.w));
+        if (S.which == 1) f(StoredOp1{c.l1, S.diag, S.w, c.g.nx, c.g.ny, c.g.nU});
+        else f(StoredOp2{c.l2, S.diag, S.w, c.g.nx, c.g.ny});
     }
     int nb() const { return row_blocks(S.n); }
 
