@@ -960,6 +960,8 @@ int cuibm_set_option(cuibm_ctx *h, const char *key, double value)
                 free_sa_hierarchy(*S);
                 build_sa_hierarchy(c, *S);
                 refresh_fused_hierarchy(c, *S);
+                if (want) setup_separable(c, *S);  // takes the cycle's place where it applies
+                else free_separable(*S);
                 refresh_system_diagonals(c, *S);  // level 0 smooths with the current rows
                 S->sa_key = read_rows_key(c);
             }

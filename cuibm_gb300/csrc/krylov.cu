@@ -548,7 +548,10 @@ static void transposed_iterations(Context &c, LinearSystem &S, Op A, const Trans
 {
     const int n = S.n, nb = blocks_for(n);
     const bool sa = S.precond == PC_SMOOTHED_AGGREGATION;
-    auto precond = [&](const double *in, double *out) { launch_vcycle_transposed(c, S, T, in, out); };
+    auto precond = [&](const double *in, double *out) {
+        if (S.sep) launch_separable_transposed(c, S, T, in, out);
+        else launch_vcycle_transposed(c, S, T, in, out);
+    };
     k_bicg_init<<<nb, kBlock, 0, c.stream>>>(A, n, b, x, S.r, S.rs, S.p, S.partials, S.ks, nullptr, S.which, 0, 0);
     CUIBM_TRY(cudaGetLastError());
     KrylovScalars host{};
@@ -586,7 +589,8 @@ int launch_solve_transposed(Context &c, LinearSystem &S, LinearSystem &F, const 
                             double *x, int *iterations)
 {
     S.amg = F.amg;  // the forward hierarchy (rebuilt for a moving body between steps)
-    if (S.precond == PC_SMOOTHED_AGGREGATION) ensure_transposed_levels(c, F);
+    S.sep = F.sep;  // so its preconditioner
+    if (S.precond == PC_SMOOTHED_AGGREGATION && !S.sep) ensure_transposed_levels(c, F);
     KrylovScalars hk{};
     CUIBM_TRY(cudaMemcpyAsync(&hk, S.ks, sizeof(hk), cudaMemcpyDeviceToHost, c.stream));
     CUIBM_TRY(cudaStreamSynchronize(c.stream));

@@ -69,6 +69,14 @@ struct SepDev {
     const double *l, *c, *inv;     // tridiagonal factors [row][mode]
     const double *Pf, *Pb;         // products of l and c over a thread's rows [thread row][mode]
     const double *cm, *cr;         // input scaling per place and per row (cr null: 1)
+    // the transposed inverse, W A0^-1 W^-1 with the cell areas W: its input scaling, the
+    // transform back and its output scaling per row
+    const double *cmt, *crt, *sB2t, *wr;
+    // a moving body's rows (null: none): r is scaled there by the ratio of A0's diagonal to
+    // the row's own
+    RowPatch patch;
+    const double *E, *W, *N, *S;
+    int nx;
     // pinned cells (the pressure system): functionals F (rows R0, R1), responses G, the
     // constant's response gm
     int pins, R[2], k0;
@@ -90,10 +98,54 @@ struct SepPlan {
     int *prow = nullptr, *pidx = nullptr;
     double *cap = nullptr, *gap = nullptr, *q = nullptr, *y = nullptr, *rin = nullptr;
     char *pblock = nullptr;
+    bool moving = false;  // a body's rows change: one Jacobi sweep on them beside A0^-1
     int tri_rows = 0;  // neighbouring rows a thread of k_sep_tri takes
     int max_nm() const { return grids > 1 ? std::max(a.f[0].nm, a.f[1].nm) : a.f[0].nm; }
     int max_nr() const { return grids > 1 ? std::max(a.f[0].nr, a.f[1].nr) : a.f[0].nr; }
     int first_kernels = 0;  // kernels of the conditional body after the first half iteration
+};
+
+// ---- the operators with their stored diagonal --------------------------------------------
+// five FP64 operations a row instead of nine (the Krylov kernels are FP64-issue bound)
+struct StoredOp2 {
+    Lhs2Coef c;
+    const double *diag, *w;
+    int nx, ny;
+    template <class X>
+    __device__ __forceinline__ double row(int i, const X &x) const
+    {
+        double y;
+        const int k = c.patch.pid ? c.patch.pid[i] : -1;
+        if (k >= 0) {
+            y = patch_row(c.patch, k, x(i), x);
+        } else {
+            const int J = i / nx, I = i - J * nx;
+            y = diag[i] * x(i);
+            if (I != nx - 1) y -= c.E[I] * x(i + 1);
+            if (I != 0) y -= c.W[I] * x(i - 1);
+            if (J != ny - 1) y -= c.N[J] * x(i + nx);
+            if (J != 0) y -= c.S[J] * x(i - nx);
+        }
+        return w ? w[i] * y : y;
+    }
+};
+struct StoredOp1 {  // without patched rows or row scales (the plain and external methods)
+    Lhs1Coef c;
+    const double *diag, *w;
+    int nx, ny, nU;
+    template <class X>
+    __device__ __forceinline__ double row(int i, const X &x) const
+    {
+        const bool u = i < nU;
+        const int n = u ? nx - 1 : nx, m = u ? ny : ny - 1, k = u ? i : i - nU, J = k / n, I = k - J * n;
+        const double *E = u ? c.uE : c.vE, *W = u ? c.uW : c.vW, *N = u ? c.uN : c.vN, *S = u ? c.uS : c.vS;
+        double y = diag[i] * x(i);
+        if (I != n - 1) y -= E[I] * x(i + 1);
+        if (I != 0) y -= W[I] * x(i - 1);
+        if (J != m - 1) y -= N[J] * x(i + n);
+        if (J != 0) y -= S[J] * x(i - n);
+        return w ? w[i] * y : y;
+    }
 };
 
 // ---- digits -------------------------------------------------------------------------
@@ -207,8 +259,18 @@ __device__ __forceinline__ void block_sums(double &a, double &b)
 // One grid row to digits, a block a row.  SPEC false: a field (times the scaling that
 // makes the transform orthonormal); true: z^, with the pinned cells' correction.  A row of
 // 922 is 7 values a thread: bound by one round of loads, the conversion and the stores.
+// the ratio of A0's diagonal to a patched row's own (1 for a row without one)
+__device__ __forceinline__ double row_ratio(const SepDev &d, int i, int k)
+{
+    const double own = d.patch.pdiag[k];
+    if (own == 0) return 1.0;
+    const int J = i / d.nx, I = i - J * d.nx;
+    return ((d.E[I] + d.W[I]) + (d.N[J] + d.S[J])) / own;
+}
+
 template <int L, int NP, bool SPEC>
-__global__ void __launch_bounds__(128) k_sep_split(const __grid_constant__ SepArgs args, const double *__restrict__ in)
+__global__ void __launch_bounds__(128) k_sep_split(const __grid_constant__ SepArgs args, const double *__restrict__ in,
+                                                   int transposed)
 {
     const SepDev &d = args.f[blockIdx.y];
     const int R = blockIdx.x, n = d.nm;
@@ -217,8 +279,16 @@ __global__ void __launch_bounds__(128) k_sep_split(const __grid_constant__ SepAr
     double s;
     if (!SPEC) {
         const double *row = in + d.base + (size_t)R * d.sr;
-        const double cr = d.cr ? d.cr[R] : 1.0;
-        s = split_row<L, NP>(n, d.nch, out, [&](int m) { return row[(size_t)m * d.sm] * (d.cm[m] * cr); });
+        const double *cm = transposed ? d.cmt : d.cm, *crp = transposed ? d.crt : d.cr;
+        const double cr = crp ? crp[R] : 1.0;
+        if (d.patch.pid && !transposed)
+            s = split_row<L, NP>(n, d.nch, out, [&](int m) {
+                const int i = d.base + R * d.sr + m * d.sm, k = d.patch.pid[i];
+                const double v = in[i] * (cm[m] * cr);
+                return k >= 0 ? v * row_ratio(d, i, k) : v;
+            });
+        else
+            s = split_row<L, NP>(n, d.nch, out, [&](int m) { return row[(size_t)m * d.sm] * (cm[m] * cr); });
     } else {
         const double *row = d.h + (size_t)R * n;
         if (d.pins == 0) {
@@ -290,10 +360,10 @@ template <int L, int WM, int WN, int ST>
 __global__ void __launch_bounds__(32 * WM * WN, 2) k_sep_gemm(const __grid_constant__ SepArgs args,
                                                              double *__restrict__ field, int back)
 {
-    // forward: h = (digits of the field) Q; back: field = (digits of z^) Q^T
+    // back 0: h = (digits of the field) Q; 1: field = (digits of z^) Q^T; 2: the transposed inverse's
     const SepDev &d = args.f[blockIdx.z];
     const __nv_bfloat16 *__restrict__ A = d.A, *__restrict__ B = back ? d.B2 : d.B1;
-    const double *__restrict__ sA = d.sA, *__restrict__ sB = back ? d.sB2 : d.sB1;
+    const double *__restrict__ sA = d.sA, *__restrict__ sB = back == 2 ? d.sB2t : back ? d.sB2 : d.sB1;
     const int M = d.nr, N = d.nm, nch = d.nch, so_m = back ? d.sr : d.nm, so_n = back ? d.sm : 1;
     double *__restrict__ out = back ? field + d.base : d.h;
     constexpr int TM = 16 * WM, TN = 16 * WN, T = 32 * WM * WN;
@@ -381,7 +451,7 @@ __global__ void __launch_bounds__(32 * WM * WN, 2) k_sep_gemm(const __grid_const
     for (int q = 0; q < 4; ++q) {
         const int r = r0 + (q >> 1) * 8;
         if (r >= M) continue;
-        const double sa = sA[r];
+        const double sa = back == 2 ? sA[r] * d.wr[r] : sA[r];
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
             const int col = c0 + t * 8 + (q & 1);
@@ -444,8 +514,8 @@ __global__ void __launch_bounds__(kTriThreads) k_sep_tri(const __grid_constant__
     const size_t at = (size_t)J0 * n + k;
     const double pf = k < n ? d.Pf[(size_t)q * n + k] : 0.0, pb = k < n ? d.Pb[(size_t)q * n + k] : 0.0;
     double x = 0;
-    if (M > 0) {
-        double r[M ? M : 1], l[M ? M : 1], iv[M ? M : 1], cc[M ? M : 1];
+    if constexpr (M > 0) {
+        double r[M], l[M], iv[M], cc[M];
 #pragma unroll
         for (int t = 0; t < M; ++t) {
             const bool on = t < cnt;
@@ -475,28 +545,28 @@ __global__ void __launch_bounds__(kTriThreads) k_sep_tri(const __grid_constant__
                 x = r[t] + cc[t] * x;
                 d.h[at + (size_t)t * n] = x;
             }
-        return;
-    }
+    } else {
 #pragma unroll 4
-    for (int t = 0; t < cnt; ++t) {
-        const double r = d.h[at + (size_t)t * n];
-        row[t * kTriThreads + tid] = r;
-        x = r + d.l[at + (size_t)t * n] * x;
-    }
-    x = tri_scan<CB>(x, pf, true, se, sp);
+        for (int t = 0; t < cnt; ++t) {
+            const double r = d.h[at + (size_t)t * n];
+            row[t * kTriThreads + tid] = r;
+            x = r + d.l[at + (size_t)t * n] * x;
+        }
+        x = tri_scan<CB>(x, pf, true, se, sp);
 #pragma unroll 4
-    for (int t = 0; t < cnt; ++t) {
-        x = row[t * kTriThreads + tid] + d.l[at + (size_t)t * n] * x;
-        row[t * kTriThreads + tid] = x * d.inv[at + (size_t)t * n];
-    }
-    x = 0;
+        for (int t = 0; t < cnt; ++t) {
+            x = row[t * kTriThreads + tid] + d.l[at + (size_t)t * n] * x;
+            row[t * kTriThreads + tid] = x * d.inv[at + (size_t)t * n];
+        }
+        x = 0;
 #pragma unroll 4
-    for (int t = cnt - 1; t >= 0; --t) x = row[t * kTriThreads + tid] + d.c[at + (size_t)t * n] * x;
-    x = tri_scan<CB>(x, pb, false, se, sp);
+        for (int t = cnt - 1; t >= 0; --t) x = row[t * kTriThreads + tid] + d.c[at + (size_t)t * n] * x;
+        x = tri_scan<CB>(x, pb, false, se, sp);
 #pragma unroll 4
-    for (int t = cnt - 1; t >= 0; --t) {
-        x = row[t * kTriThreads + tid] + d.c[at + (size_t)t * n] * x;
-        d.h[at + (size_t)t * n] = x;
+        for (int t = cnt - 1; t >= 0; --t) {
+            x = row[t * kTriThreads + tid] + d.c[at + (size_t)t * n] * x;
+            d.h[at + (size_t)t * n] = x;
+        }
     }
 }
 
@@ -583,49 +653,6 @@ __global__ void k_sep_constant(int n, int k0, const double *__restrict__ v, doub
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) Q[(size_t)i * n + k0] = v[i];
 }
-
-// ---- the operators with their stored diagonal --------------------------------------------
-// five FP64 operations a row instead of nine (the Krylov kernels are FP64-issue bound)
-struct StoredOp2 {
-    Lhs2Coef c;
-    const double *diag, *w;
-    int nx, ny;
-    template <class X>
-    __device__ __forceinline__ double row(int i, const X &x) const
-    {
-        double y;
-        const int k = c.patch.pid ? c.patch.pid[i] : -1;
-        if (k >= 0) {
-            y = patch_row(c.patch, k, x(i), x);
-        } else {
-            const int J = i / nx, I = i - J * nx;
-            y = diag[i] * x(i);
-            if (I != nx - 1) y -= c.E[I] * x(i + 1);
-            if (I != 0) y -= c.W[I] * x(i - 1);
-            if (J != ny - 1) y -= c.N[J] * x(i + nx);
-            if (J != 0) y -= c.S[J] * x(i - nx);
-        }
-        return w ? w[i] * y : y;
-    }
-};
-struct StoredOp1 {  // without patched rows or row scales (the plain and external methods)
-    Lhs1Coef c;
-    const double *diag, *w;
-    int nx, ny, nU;
-    template <class X>
-    __device__ __forceinline__ double row(int i, const X &x) const
-    {
-        const bool u = i < nU;
-        const int n = u ? nx - 1 : nx, m = u ? ny : ny - 1, k = u ? i : i - nU, J = k / n, I = k - J * n;
-        const double *E = u ? c.uE : c.vE, *W = u ? c.uW : c.vW, *N = u ? c.uN : c.vN, *S = u ? c.uS : c.vS;
-        double y = diag[i] * x(i);
-        if (I != n - 1) y -= E[I] * x(i + 1);
-        if (I != 0) y -= W[I] * x(i - 1);
-        if (J != m - 1) y -= N[J] * x(i + n);
-        if (J != 0) y -= S[J] * x(i - n);
-        return w ? w[i] * y : y;
-    }
-};
 
 // ---- Krylov kernels ---------------------------------------------------------------------
 // The rows of a grid of at most kRowBlocks blocks, and its sums: a block's partial sums go
@@ -797,6 +824,21 @@ __global__ void __launch_bounds__(256) k_sep_4(int n, double *x, double *r, doub
     }
 }
 
+// A last correction x += M r for the residual that the solve ends with (a moving body's
+// solves): where the iteration stops, the level of the pressure - fixed by one pinned cell -
+// carries up to 2e-9 of it at a relative residual of 1e-12; M resolves it exactly
+__global__ void k_sep_pick(int n, const double *__restrict__ r, const double *__restrict__ s, double *out,
+                           const KrylovScalars *ks)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) out[i] = ks->s_done ? s[i] : r[i];
+}
+__global__ void k_sep_correct(int n, const double *__restrict__ z, double *x, const KrylovScalars *ks)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n && ks->status == KS_CONVERGED) x[i] += z[i];
+}
+
 // CG's first iteration: p = z, q = A z, rho = r . z, alpha = rho / (z . q)
 template <class Op>
 __global__ void __launch_bounds__(256) k_sep_cg_1(Op A, int n, const double *__restrict__ r,
@@ -932,14 +974,14 @@ static void launch_gemm(Context &c, const SepPlan &P, double *field, int back)
 }
 
 template <int L, bool SPEC>
-static void launch_split(Context &c, const SepPlan &P, const double *in)
+static void launch_split(Context &c, const SepPlan &P, const double *in, int tr = 0)
 {
     const int n = (P.max_nm() + kKC - 1) / kKC * kKC;
     const dim3 grid(P.max_nr(), P.grids);
-    if (n <= 256) k_sep_split<L, 1, SPEC><<<grid, 128, 0, c.stream>>>(P.a, in);
-    else if (n <= 512) k_sep_split<L, 2, SPEC><<<grid, 128, 0, c.stream>>>(P.a, in);
-    else if (n <= 1024) k_sep_split<L, 4, SPEC><<<grid, 128, 0, c.stream>>>(P.a, in);
-    else k_sep_split<L, 8, SPEC><<<grid, 128, 0, c.stream>>>(P.a, in);
+    if (n <= 256) k_sep_split<L, 1, SPEC><<<grid, 128, 0, c.stream>>>(P.a, in, tr);
+    else if (n <= 512) k_sep_split<L, 2, SPEC><<<grid, 128, 0, c.stream>>>(P.a, in, tr);
+    else if (n <= 1024) k_sep_split<L, 4, SPEC><<<grid, 128, 0, c.stream>>>(P.a, in, tr);
+    else k_sep_split<L, 8, SPEC><<<grid, 128, 0, c.stream>>>(P.a, in, tr);
     CUIBM_TRY(cudaGetLastError());
 }
 
@@ -967,19 +1009,19 @@ static void launch_tri(Context &c, const SepPlan &P)
 }
 
 template <int L>
-static void apply_t(Context &c, const SepPlan &P, const double *in, double *out)
+static void apply_t(Context &c, const SepPlan &P, const double *in, double *out, int tr)
 {
-    launch_split<L, false>(c, P, in);
+    launch_split<L, false>(c, P, in, tr);
     launch_gemm<L>(c, P, nullptr, 0);
     launch_tri(c, P);
     launch_split<L, true>(c, P, nullptr);
-    launch_gemm<L>(c, P, out, 1);
+    launch_gemm<L>(c, P, out, 1 + tr);
 }
 
-static void apply_grid(Context &c, const SepPlan &P, const double *in, double *out)
+static void apply_grid(Context &c, const SepPlan &P, const double *in, double *out, int transposed = 0)
 {
-    if (P.digits == kDigits) apply_t<kDigits>(c, P, in, out);
-    else apply_t<kDigitsMixed>(c, P, in, out);
+    if (P.digits == kDigits) apply_t<kDigits>(c, P, in, out, transposed);
+    else apply_t<kDigitsMixed>(c, P, in, out, transposed);
 }
 
 // ---- rows that a body patches -----------------------------------------------------------
@@ -1071,12 +1113,61 @@ __global__ void k_sep_eliminate(int m, int k, double *W, const double *__restric
     if (j < 2 * m && i != k) W[(size_t)i * 2 * m + j] -= fac[i] * W[(size_t)k * 2 * m + j];
 }
 
+// A moving body's rows change every step, so nothing of theirs is inverted ahead.  Scaled to
+// A0's diagonal before A0^-1 and swept once by Jacobi after it, z = y + D^-1 (r - A y) on the
+// patched rows, they leave 8 to 11 iterations (embedded cylinder, 186 patched rows of 96100:
+// 29 without either, 16 with the scaling alone; exact local solves of the rows' region: 10).
+__global__ void k_sep_sweep(StoredOp2 A, int n, const double *__restrict__ r, const double *__restrict__ z, double *dz)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int k = A.c.patch.pid[i];
+    if (k < 0) return;
+    const double own = A.c.patch.pdiag[k];
+    dz[i] = own != 0 ? (r[i] - A.row(i, PtrAccess{z})) / own : 0.0;
+}
+__global__ void k_sep_add(int n, const int *__restrict__ pid, const double *__restrict__ dz, double *z)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n && pid[i] >= 0) z[i] += dz[i];
+}
+// the transposed form: y = D^-1 r on the patched rows, then z = y + S A0^-T (r - A^T y)
+__global__ void k_sep_first(RowPatch P, int n, const double *__restrict__ r, double *y)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int k = P.pid[i];
+    const double own = k >= 0 ? P.pdiag[k] : 0.0;
+    y[i] = own != 0 ? r[i] / own : 0.0;
+}
+__global__ void k_sep_residual(Op2T A, int n, const double *__restrict__ r, const double *__restrict__ y, double *out)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) out[i] = r[i] - A.row(i, PtrAccess{y});
+}
+__global__ void k_sep_last(const __grid_constant__ SepArgs args, int n, const double *__restrict__ y, double *z)
+{
+    const SepDev &d = args.f[0];
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int k = d.patch.pid[i];
+    if (k >= 0) z[i] = y[i] + z[i] * row_ratio(d, i, k);
+}
+
 constexpr int kPatchMax = 2048;  // patched rows: the capacitance matrix is 8 m^2 bytes, its set-up m applications
 
 // out = M in: five kernels, or thirteen with patched rows
 void launch_separable_apply(Context &c, LinearSystem &S, const double *in, double *out)
 {
     const SepPlan &P = *static_cast<const SepPlan *>(S.sep);
+    if (P.moving) {
+        apply_grid(c, P, in, out);
+        const StoredOp2 A{c.l2, S.diag, nullptr, c.g.nx, c.g.ny};
+        k_sep_sweep<<<blocks_for(S.n), kBlock, 0, c.stream>>>(A, S.n, in, out, P.y);
+        k_sep_add<<<blocks_for(S.n), kBlock, 0, c.stream>>>(S.n, c.l2.patch.pid, P.y, out);
+        CUIBM_TRY(cudaGetLastError());
+        return;
+    }
     if (!P.patched) {
         apply_grid(c, P, in, out);
         return;
@@ -1089,6 +1180,19 @@ void launch_separable_apply(Context &c, LinearSystem &S, const double *in, doubl
     k_sep_less<<<blocks_for(S.n), kBlock, 0, c.stream>>>(S.n, in, P.pidx, P.q, P.rin);
     CUIBM_TRY(cudaGetLastError());
     apply_grid(c, P, P.rin, out);
+}
+
+// out = M^T in for the transposed solves of the embedded method's adjoint
+void launch_separable_transposed(Context &c, LinearSystem &S, const TransposeList &T, const double *in, double *out)
+{
+    const SepPlan &P = *static_cast<const SepPlan *>(S.sep);
+    const int n = S.n, nb = blocks_for(n);
+    k_sep_first<<<nb, kBlock, 0, c.stream>>>(c.l2.patch, n, in, P.y);
+    k_sep_residual<<<nb, kBlock, 0, c.stream>>>(Op2T{c.l2, c.g, T}, n, in, P.y, P.rin);
+    CUIBM_TRY(cudaGetLastError());
+    apply_grid(c, P, P.rin, out, 1);
+    k_sep_last<<<nb, kBlock, 0, c.stream>>>(P.a, n, P.y, out);
+    CUIBM_TRY(cudaGetLastError());
 }
 
 // The capacitance matrix of a fixed body's patched rows and its inverse.  False where it
@@ -1152,12 +1256,14 @@ static bool build_patch(Context &c, LinearSystem &S, const std::vector<int> &pid
 // pressure system of the methods that leave its rows alone, unless the case asks for a form
 // of smoothed aggregation by name (-saStructured 0 or 1, strengthThreshold, -separable 0).
 // By itself (-separable -1) not where the pressure's level would move by more than 1e-9 of
-// it: with the external method one pinned cell in the domain's corner fixes the level, and
+// it: with the external and embedded methods one pinned cell in the domain's corner fixes the level, and
 // the smoothed-aggregation solves leave their stopping error in it (against a solve to
 // 1e-15: 1e-10 to 1e-7 of p at a relative residual of 1e-13 from 200k unknowns on, 1e-9 in
 // mixed precision and in batches at 1e-12, below 3e-10 elsewhere; the separable solves
-// 1e-11), so runs there keep the solver that they began with.  With the plain method the
-// centre cell is pinned too and the level agrees to 1e-12.
+// 1e-11; embedded, 470k unknowns at 1e-12: up to 1.0e-9 against 4e-10), so runs there keep
+// the solver that they began with unless they ask (-separable 1: Re 550, 922 x 922, 101 to
+// 2.8 ms a step, the oscillating cylinder 686 x 686 34.5 to 10.1 ms).  With the plain and
+// Fadlun methods the centre cell is pinned too and the level agrees to 1e-10.
 constexpr int kLevelMax = 200000;
 
 // The velocity system (I - dt/2 nu L, two grids) has a far smaller condition number, and the
@@ -1187,16 +1293,13 @@ static bool separable_applies(const Context &c, const LinearSystem &S)
     const int nx = c.g.nx, ny = c.g.ny;
     if (c.P.separable == 0 || std::min(nx, ny) > kSepMax || std::max(nx, ny) > kTriRows) return false;
     if (S.which == 2) {
-        // the embedded method's rows change with its body
-        if (S.precond != PC_SMOOTHED_AGGREGATION || c.P.saStructured != -1 || c.P.poisson.strength >= 0 ||
-            c.P.solverType == ST_OSC)
-            return false;
+        if (S.precond != PC_SMOOTHED_AGGREGATION || c.P.saStructured != -1 || c.P.poisson.strength >= 0) return false;
     } else {
         if (S.precond != PC_DIAGONAL || (c.P.solverType != ST_NAVIERSTOKES && c.P.solverType != ST_LUO)) return false;
     }
     if (c.P.separable == 1) return true;
     const bool level = c.P.solverType == ST_NAVIERSTOKES || c.P.solverType == ST_FADLUN ||
-                       (c.P.solverType == ST_LUO && c.g.nP < kLevelMax && c.P.solverPack != 2 &&
+                       (c.g.nP < kLevelMax && c.P.solverPack != 2 &&
                         c.P.poisson.precision == PRECISION_FP64);
     return level && (S.which == 2 || predicted_velocity_steps(c, S.rtol) >= kVelocitySteps);
 }
@@ -1236,8 +1339,10 @@ static bool build_grid(Context &c, SepPlan &P, int g, const SepGrid &G, bool sym
     if (d.pins) lam[k0] = 0;
     double len = 0;
     for (double w : G.wm) len += w;
-    std::vector<double> cm(nm), cr(nr), em(nm), con(nm);
+    std::vector<double> cm(nm), cr(nr), em(nm), con(nm), et(nm), crt(nr);
+    for (int J = 0; J < nr; ++J) crt[J] = 1 / G.wr[J];
     for (int i = 0; i < nm; ++i) {
+        et[i] = std::sqrt(G.wm[i]);
         cm[i] = sym ? 1 / std::sqrt(G.wm[i]) : std::sqrt(G.wm[i]);
         em[i] = 1 / std::sqrt(G.wm[i]);
         con[i] = std::sqrt(G.wm[i] / len);
@@ -1257,6 +1362,7 @@ static bool build_grid(Context &c, SepPlan &P, int g, const SepGrid &G, bool sym
     const size_t osB1 = reserve(nm * 8), osB2 = reserve(nm * 8), osA = reserve(nr * 8);
     const size_t oh = reserve(n * 8), ol = reserve(n * 8), oc = reserve(n * 8), oi = reserve(n * 8);
     const size_t oPf = reserve((size_t)nq * nm * 8), oPb = reserve((size_t)nq * nm * 8);
+    const size_t ocmt = reserve(nm * 8), ocrt = reserve(nr * 8), osB2t = reserve(nm * 8), owr = reserve(nr * 8);
     const size_t ocm = reserve(nm * 8), ocr = reserve(nr * 8), oF0 = reserve(nm * 8), oF1 = reserve(nm * 8);
     const size_t oG0 = reserve(d.pins > 0 ? n * 8 : 8), oG1 = reserve(d.pins > 1 ? n * 8 : 8), ogm = reserve(nr * 8);
     CUIBM_TRY(cudaMalloc(&P.block[g], need));
@@ -1269,7 +1375,7 @@ static bool build_grid(Context &c, SepPlan &P, int g, const SepGrid &G, bool sym
     // set-up scratch, freed at the end
     char *tmp = nullptr;
     const size_t bq = ((size_t)nm * nm * 8 + 255) & ~size_t(255), bs = (sweeps.size() * sizeof(Sweep) + 511) & ~size_t(255),
-                 br = (rot.size() * sizeof(double2) + 511) & ~size_t(255), bv = (size_t)(3 * nm + 2 * nr) * 8;
+                 br = (rot.size() * sizeof(double2) + 511) & ~size_t(255), bv = (size_t)(4 * nm + 2 * nr) * 8;
     CUIBM_TRY(cudaMalloc(&tmp, bq + bs + br + bv));
     struct Freed {
         char *p;
@@ -1278,8 +1384,8 @@ static bool build_grid(Context &c, SepPlan &P, int g, const SepGrid &G, bool sym
     double *Q = reinterpret_cast<double *>(tmp);
     Sweep *sw = reinterpret_cast<Sweep *>(tmp + bq);
     double2 *rt = reinterpret_cast<double2 *>(tmp + bq + bs);
-    double *vl = reinterpret_cast<double *>(tmp + bq + bs + br), *vcon = vl + nm, *vem = vcon + nm, *vur = vem + nm,
-           *vdr = vur + nr;
+    double *vl = reinterpret_cast<double *>(tmp + bq + bs + br), *vcon = vl + nm, *vem = vcon + nm, *vet = vem + nm,
+           *vur = vet + nm, *vdr = vur + nr;
     if (!rot.empty()) {
         CUIBM_TRY(cudaMemcpyAsync(sw, sweeps.data(), sweeps.size() * sizeof(Sweep), cudaMemcpyHostToDevice, c.stream));
         CUIBM_TRY(cudaMemcpyAsync(rt, rot.data(), rot.size() * sizeof(double2), cudaMemcpyHostToDevice, c.stream));
@@ -1291,6 +1397,10 @@ static bool build_grid(Context &c, SepPlan &P, int g, const SepGrid &G, bool sym
     put(vdr, G.dr);
     put(D(ocm), cm);
     put(D(ocr), cr);
+    put(vet, et);
+    put(D(ocmt), em);
+    put(D(ocrt), crt);
+    put(D(owr), G.wr);
     const size_t smem = (size_t)nm * kRotWarps * 8;
     allow_smem(k_sep_rotate, smem);
     k_sep_rotate<<<(nm + kRotWarps - 1) / kRotWarps, 32 * kRotWarps, smem, c.stream>>>(nm, sw, (int)sweeps.size(), rt, Q);
@@ -1299,10 +1409,12 @@ static bool build_grid(Context &c, SepPlan &P, int g, const SepGrid &G, bool sym
     if (L == kDigits) {
         allow_gemm<kDigits>();
         split_table<kDigits>(c, Q, nm, nm, d.nch, 1, nm, nullptr, H(oB1), D(osB1));
+        split_table<kDigits>(c, Q, nm, nm, d.nch, nm, 1, vet, H(oB2), D(osB2t));
         split_table<kDigits>(c, Q, nm, nm, d.nch, nm, 1, vem, H(oB2), D(osB2));
     } else {
         allow_gemm<kDigitsMixed>();
         split_table<kDigitsMixed>(c, Q, nm, nm, d.nch, 1, nm, nullptr, H(oB1), D(osB1));
+        split_table<kDigitsMixed>(c, Q, nm, nm, d.nch, nm, 1, vet, H(oB2), D(osB2t));
         split_table<kDigitsMixed>(c, Q, nm, nm, d.nch, nm, 1, vem, H(oB2), D(osB2));
     }
     allow_smem(k_sep_tri<8, 0>, 200 * 1024);
@@ -1325,6 +1437,10 @@ static bool build_grid(Context &c, SepPlan &P, int g, const SepGrid &G, bool sym
     d.Pb = D(oPb);
     d.cm = D(ocm);
     d.cr = sym ? D(ocr) : nullptr;
+    d.cmt = D(ocmt);
+    d.crt = D(ocrt);
+    d.sB2t = D(osB2t);
+    d.wr = D(owr);
     d.k0 = k0;
     d.mean = 1 / std::sqrt(len);
     d.gm = D(ogm);
@@ -1442,7 +1558,22 @@ void setup_separable(Context &c, LinearSystem &S)
         }
     }
     P->grids = (int)grids.size();
-    if (S.which == 2 && c.l2.patch.pid && !build_patch(c, S, c.fadlun.pid2)) free_separable(S);
+    if (S.which != 2 || !c.l2.patch.pid) return;
+    if (c.P.solverType == ST_OSC) {
+        SepDev &d = P->a.f[0];
+        d.patch = c.l2.patch;
+        d.E = c.l2.E;
+        d.W = c.l2.W;
+        d.N = c.l2.N;
+        d.S = c.l2.S;
+        d.nx = nx;
+        P->moving = true;
+        CUIBM_TRY(cudaMalloc(&P->pblock, 2 * (size_t)S.n * sizeof(double)));
+        P->y = reinterpret_cast<double *>(P->pblock);
+        P->rin = P->y + S.n;
+    } else if (!build_patch(c, S, c.fadlun.pid2)) {
+        free_separable(S);
+    }
 }
 
 void free_separable(LinearSystem &S)
@@ -1504,6 +1635,14 @@ struct SepSolve {
         k_sep_4<<<nb(), kBlock, 0, c.stream>>>(S.n, x, S.r, S.rs, S.p, S.s, S.Ms, S.AMs, S.partials, S.ks, c.err_word,
                                                S.which, first, h, use);
         k_bicg_5<<<blocks_for(S.n), kBlock, 0, c.stream>>>(S.n, S.p, S.r, S.AMp, S.ks);
+        CUIBM_TRY(cudaGetLastError());
+    }
+    void correct() const
+    {
+        const int nb = blocks_for(S.n);
+        k_sep_pick<<<nb, kBlock, 0, c.stream>>>(S.n, S.r, S.s, S.p, S.ks);
+        launch_separable_apply(c, S, S.p, S.Mp);
+        k_sep_correct<<<nb, kBlock, 0, c.stream>>>(S.n, S.Mp, x, S.ks);
         CUIBM_TRY(cudaGetLastError());
     }
     void cg(bool first, cudaGraphConditionalHandle h, int use) const
@@ -1599,6 +1738,7 @@ void launch_separable_solve(Context &c, LinearSystem &S, const double *b, double
             L.half(false, more.h, 1);
             L.rest(false, more.h, 1);
         });
+        if (P.moving) L.correct();
         return;
     }
     KrylovScalars host{};
@@ -1614,12 +1754,11 @@ void launch_separable_solve(Context &c, LinearSystem &S, const double *b, double
         return;
     }
     L.half(true, 0, 0);
-    if (!running()) return;
-    L.rest(true, 0, 0);
-    while (running()) {
-        L.half(false, 0, 0);
-        L.rest(false, 0, 0);
+    for (bool first = true; running(); first = false) {
+        if (!first) L.half(false, 0, 0);
+        L.rest(first, 0, 0);
     }
+    if (P.moving) L.correct();
 }
 
 // kernels that a solve's conditional bodies ran: the first execution is the rest of the
