@@ -45,6 +45,10 @@ struct TagRecords {
     double *bi;      // [idx][5 slots][4]: bix, biy, ipx, ipy
     double *distA, *distB;
     int nrec;
+    // the body segments that cross each row and each column of the box, in order
+    int *cross_count, *cross;  // [line], [line][total]: rows first, then columns
+    double *cross_at, *cross_uv;  // where each crosses, and the body velocity there
+    int lines;
 };
 
 struct TagGeom {
@@ -54,6 +58,82 @@ struct TagGeom {
     int nx, ny, total;
     double midX, midY;
     const double *motion;  // moving body: the centre is motion[0], motion[1] (set on the device)
+    int nxc, nyc;          // lengths of xc, yc
+};
+
+// The segments (k, l = k + 1 around the body) whose ends lie on both sides of a row's
+// ordinate (line < rows) or a column's abscissa, in increasing l, a warp a line.  The tests
+// are those of the reference's node loops, as are the point where a segment crosses and the body
+// velocity there (FP64 divisions: about a microsecond of dependent instructions each); every
+// node of a line shares them, so a node visits the few segments of its row and column
+// instead of all of them.
+__global__ void k_tag_lines(TagGeom G, TagRecords R, int rows)
+{
+    const int line = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (line >= rows + G.width) return;
+    const bool row = line < rows;
+    const int at = row ? G.j0 + line : G.i0 + line - rows;
+    int n = 0;
+    if (at < (row ? G.nyc : G.nxc)) {
+        const double c = row ? G.yc[at] : G.xc[at], *b = row ? G.by : G.bx, *o = row ? G.bx : G.by, *vel = G.vel;
+        const size_t first = (size_t)line * G.total;
+        for (int l0 = 0; l0 < G.total; l0 += 32) {
+            const int l = l0 + lane, k = l > 0 ? l - 1 : G.total - 1;
+            bool hit = false;
+            if (l < G.total) {
+                const double lo = b[k] > b[l] ? b[l] : b[k], hi = b[k] > b[l] ? b[k] : b[l];
+                hit = lo - IB_EPS < c && hi - IB_EPS > c;
+            }
+            const unsigned m = __ballot_sync(0xffffffffu, hit);
+            if (hit) {
+                const size_t e = first + n + __popc(m & ((1u << lane) - 1));
+                R.cross[e] = l;
+                if (fabs(b[l] - b[k]) > IB_EPS) {
+                    R.cross_at[e] = o[k] + (o[l] - o[k]) * (c - b[k]) / (b[l] - b[k]);
+                    R.cross_uv[e] = vel[k] + (vel[l] - vel[k]) * (c - b[k]) / (b[l] - b[k]);
+                }
+            }
+            n += __popc(m);
+        }
+    }
+    if (lane == 0) R.cross_count[line] = n;
+}
+
+// the crossings of a node's row and column, merged in increasing l
+struct Crossings {
+    const TagRecords &R;
+    size_t row, col;
+    int nr, nc, l, k;
+    bool x, y;  // l crosses the row; the column
+    double ax, ay, ux, uy;  // where, and the body velocity there
+    __device__ Crossings(const TagGeom &G, const TagRecords &R_, int idx) : R(R_)
+    {
+        const int rows = (G.nthreads + G.width - 1) / G.width, j = idx / G.width, i = rows + idx % G.width;
+        row = (size_t)j * G.total;
+        col = (size_t)i * G.total;
+        nr = R.cross_count[j];
+        nc = R.cross_count[i];
+    }
+    __device__ bool next(int total)
+    {
+        const int lr = nr > 0 ? R.cross[row] : total, lc = nc > 0 ? R.cross[col] : total;
+        l = min(lr, lc);
+        if (l == total) return false;
+        k = l > 0 ? l - 1 : total - 1;
+        x = lr == l;
+        y = lc == l;
+        if (x) {
+            ax = R.cross_at[row];
+            ux = R.cross_uv[row];
+            ++row, --nr;
+        }
+        if (y) {
+            ay = R.cross_at[col];
+            uy = R.cross_uv[col];
+            ++col, --nc;
+        }
+        return true;
+    }
 };
 
 // Foot of the perpendicular from (px, py) onto the line through body points k and l.
@@ -108,23 +188,21 @@ __global__ void k_tag_velocity_records(TagGeom G, TagRecords R)
         R.flags[idx] = 0;
         return;
     }
-    const double *bx = G.bx, *by = G.by, *vel = G.vel, *xc = G.xc, *yc = G.yc;
+    const double *bx = G.bx, *by = G.by, *xc = G.xc, *yc = G.yc;
     const double midX = G.motion ? G.motion[0] : G.midX, midY = G.motion ? G.motion[1] : G.midY;
-    int k = G.total - 1, l = 0;
     bool outsideX = true, outsideY = true, flag = false;
     int fX = -1, fY = -1, f2X = -1, f2Y = -1;
     double uvX = 0.0, uvY = 0.0, Xa = 1.0, Ya = 1.0, Xb = 1.0, Yb = 1.0, x = 0.0, y = 0.0;
     double distA = 0, distB = 0;
     if (KIND == 0) flags_extra |= 1 << 17;  // dist_u_body[ip] = 0 at thread start
     double ix, iy;
-    while (l < G.total && (KIND == 1 || !flag)) {
-        int bottom, top, left, right;
-        if (by[k] > by[l]) { bottom = l; top = k; } else { bottom = k; top = l; }
-        if (bx[k] > bx[l]) { left = l; right = k; } else { left = k; right = l; }
-        if (by[bottom] - IB_EPS < yc[J] && by[top] - IB_EPS > yc[J] && (KIND == 0 || !flag)) {
+    // (once flag is set the reference's remaining segments do nothing)
+    for (Crossings cr(G, R, idx); !flag && cr.next(G.total);) {
+        const int k = cr.k, l = cr.l;
+        if (cr.x) {
             if (fabs(by[l] - by[k]) > IB_EPS) {
-                x = bx[k] + (bx[l] - bx[k]) * (yc[J] - by[k]) / (by[l] - by[k]);
-                uvX = vel[k] + (vel[l] - vel[k]) * (yc[J] - by[k]) / (by[l] - by[k]);
+                x = cr.ax;
+                uvX = cr.ux;
                 if (x > xc[I] + IB_EPS) outsideX = !outsideX;
                 if (x > xc[I - 1] + IB_EPS && x < xc[I] - IB_EPS) {
                     fX = n;
@@ -178,10 +256,10 @@ __global__ void k_tag_velocity_records(TagGeom G, TagRecords R)
                 }
             }
         }
-        if (bx[left] - IB_EPS < xc[I] && bx[right] - IB_EPS > xc[I] && (KIND == 0 || !flag)) {
+        if (cr.y && (KIND == 0 || !flag)) {
             if (fabs(bx[l] - bx[k]) > IB_EPS) {
-                y = by[k] + (by[l] - by[k]) * (xc[I] - bx[k]) / (bx[l] - bx[k]);
-                uvY = vel[k] + (vel[l] - vel[k]) * (xc[I] - bx[k]) / (bx[l] - bx[k]);
+                y = cr.ay;
+                uvY = cr.uy;
                 if (y > yc[J] + IB_EPS) outsideY = !outsideY;
                 if (y > yc[J - 1] + IB_EPS && y < yc[J] - IB_EPS) {
                     fY = n;
@@ -239,8 +317,6 @@ __global__ void k_tag_velocity_records(TagGeom G, TagRecords R)
                 }
             }
         }
-        k = l;
-        l = l + 1;
     }
     const bool useX = outsideX && fX >= 0, useY = outsideY && fY >= 0;
     int hy = -1, hy2 = -1;
@@ -289,16 +365,13 @@ __global__ void k_tag_pressure_records(TagGeom G, TagRecords R)
     }
     const double *bx = G.bx, *by = G.by, *xv = G.xc, *yu = G.yc;
     const double midX = G.motion ? G.motion[0] : G.midX, midY = G.motion ? G.motion[1] : G.midY;
-    int k = G.total - 1, l = 0;
     bool flag = false;
     double x, y, ix, iy;
-    while (l < G.total) {
-        int bottom, top, left, right;
-        if (by[k] > by[l]) { bottom = l; top = k; } else { bottom = k; top = l; }
-        if (bx[k] > bx[l]) { left = l; right = k; } else { left = k; right = l; }
-        if (by[bottom] - IB_EPS < yu[J] && by[top] - IB_EPS > yu[J] && !flag) {
+    for (Crossings cr(G, R, idx); !flag && cr.next(G.total);) {
+        const int k = cr.k, l = cr.l;
+        if (cr.x) {
             if (fabs(by[l] - by[k]) > IB_EPS) {
-                x = bx[k] + (bx[l] - bx[k]) * (yu[J] - by[k]) / (by[l] - by[k]);
+                x = cr.ax;
                 bool g1 = x > midX + IB_EPS && x > xv[I] + IB_EPS + IB_EPS && x < xv[I + 1] - IB_EPS;
                 bool g2 = x < midX + IB_EPS && x < xv[I] - IB_EPS && x > xv[I - 1] + IB_EPS;
                 if (g1 || g2) {
@@ -328,9 +401,9 @@ __global__ void k_tag_pressure_records(TagGeom G, TagRecords R)
                 }
             }
         }
-        if (bx[left] - IB_EPS < xv[I] && bx[right] - IB_EPS > xv[I] && !flag) {
+        if (cr.y && !flag) {
             if (fabs(bx[l] - bx[k]) > IB_EPS) {
-                y = by[k] + (by[l] - by[k]) * (xv[I] - bx[k]) / (bx[l] - bx[k]);
+                y = cr.ay;
                 bool g1 = y > midY + IB_EPS && y > yu[J] + IB_EPS && y < yu[J + 1] - IB_EPS;
                 bool g2 = y < midY + IB_EPS && y < yu[J] - IB_EPS && y > yu[J - 1] + IB_EPS;
                 if (g1 || g2) {
@@ -361,8 +434,6 @@ __global__ void k_tag_pressure_records(TagGeom G, TagRecords R)
                 }
             }
         }
-        k = l;
-        l = l + 1;
     }
     R.flags[idx] = w.flags | extra;
     for (int s = 0; s < 5; ++s)
@@ -452,32 +523,54 @@ __global__ void k_tag_resolve(TagGeom G, TagRecords R, TagOut O)
     if (have_d) O.dist[ip] = dv;
 }
 
-// zero_pressure_luo / zero_x_luo / zero_y_luo: one thread per row, left to right
-__global__ void k_zero_rows(int *tags, int stride, int i0, int i1, int j0, int j1, int rows, int scan_end)
+// zero_pressure_luo / zero_x_luo / zero_y_luo: a row left to right, a warp a row (blockIdx.y:
+// which of the three arrays).  The warp loads the row and finds the last tagged node up to
+// scan_end (the place the reference's inner loop looks for: nodes right of i still hold their
+// tags when the walk is at i); one lane walks the row in shared memory.  A thread a row with
+// the tags in memory took 410 us an array on the 500-node rows of the KC 10 box.
+struct ZeroRows {
+    int *tags[3];
+    int stride[3], scan_end[3];
+    int i0, i1, j0, j1, rows;
+};
+__global__ void __launch_bounds__(32) k_zero_rows(ZeroRows Z)
 {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= rows) return;
-    const int J = j0 + j;
-    if (J > j1) return;
-    bool rowIsntDone = true, flag = false;
-    for (int i = i0; i < i1; ++i) {
-        const int I = J * stride + i;
-        if (tags[I - 1] >= 0) {
-            if (tags[I] != -1 && tags[I - 1] == 0) rowIsntDone = false;
-            if (tags[I] == -1 && rowIsntDone) tags[I] = 0;
-            if (tags[I] == 0 && tags[I - 1] != 0) {
-                int k = i;
-                while (k < scan_end) {
-                    k++;
-                    if (tags[J * stride + k] != -1) flag = true;
+    extern __shared__ int t[];  // the row from i0 - 1 to i1 - 1
+    const int a = blockIdx.y, j = blockIdx.x, lane = threadIdx.x, J = Z.j0 + j;
+    if (j >= Z.rows || J > Z.j1) return;
+    int *row = Z.tags[a] + (size_t)J * Z.stride[a];
+    const int end = Z.scan_end[a], n = Z.i1 - Z.i0;
+    int last = -1;
+    for (int i = Z.i0 - 1 + lane; i <= max(end, Z.i1 - 1); i += 32) {
+        const int v = row[i];
+        if (i < Z.i1) t[i - Z.i0 + 1] = v;
+        if (i <= end && v != -1) last = i;
+    }
+    for (int o = 16; o > 0; o >>= 1) last = max(last, __shfl_xor_sync(0xffffffffu, last, o));
+    __syncwarp();
+    if (lane == 0) {
+        bool rowIsntDone = true, flag = false;
+        int before = t[0];
+        for (int q = 1; q <= n; ++q) {
+            int v = t[q];
+            if (before >= 0) {
+                const int old = v;
+                if (v != -1 && before == 0) rowIsntDone = false;
+                if (v == -1 && rowIsntDone) v = 0;
+                if (v == 0 && before != 0) {
+                    if (last > Z.i0 + q - 1) flag = true;
+                    if (!flag) {
+                        v = -1;
+                        rowIsntDone = false;
+                    }
                 }
-                if (!flag) {
-                    tags[I] = -1;
-                    rowIsntDone = false;
-                }
+                if (v != old) t[q] = v;
             }
+            before = v;
         }
     }
+    __syncwarp();
+    for (int q = 1 + lane; q <= n; q += 32) row[Z.i0 + q - 1] = t[q];
 }
 
 __global__ void k_tag_fill(int nUV, int nP, int *gUV, int *hUV, int *h2UV, double *dn, double *db, double *bix,
@@ -1361,6 +1454,11 @@ void setup_ib(Context &c)
     H.rec.nrec = ref_threads(w, h);
     const size_t nr = H.rec.nrec;
     H.rec.flags = c.carve<int>(nr);
+    H.rec.lines = (int)((nr + w - 1) / w) + w;
+    H.rec.cross_count = c.carve<int>(H.rec.lines);
+    H.rec.cross = c.carve<int>((size_t)H.rec.lines * c.body.total);
+    H.rec.cross_at = c.carve<double>((size_t)H.rec.lines * c.body.total);
+    H.rec.cross_uv = c.carve<double>((size_t)H.rec.lines * c.body.total);
     H.rec.hyb = c.carve<int>(nr);
     H.rec.hyb2 = c.carve<int>(nr);
     H.rec.dnode = c.carve<double>(nr);
@@ -1474,24 +1572,36 @@ void launch_tag_points(Context &c)
              b.distU};
     const int rows = (nthreads + w - 1) / w;
     const int nres = (w + 2) * (rows + 2);
+    if (rows + w > H.rec.lines) throw InputError("the body's box outgrew the tagging records");
+    auto lines = [&] {
+        k_tag_lines<<<blocks_for(32L * (rows + w)), kBlock, 0, c.stream>>>(G, H.rec, rows);
+    };
+    G.nxc = nx - 1;
+    G.nyc = ny;
+    lines();
     k_tag_velocity_records<0><<<blocks_for(nthreads), kBlock, 0, c.stream>>>(G, H.rec);
     k_tag_resolve<0><<<blocks_for(nres), kBlock, 0, c.stream>>>(G, H.rec, O);
     G.vel = b.vB;
     G.xc = c.xv;
     G.yc = c.yv;
+    G.nxc = nx;
+    G.nyc = ny - 1;
+    lines();
     O.dist = b.distV;
     k_tag_velocity_records<1><<<blocks_for(nthreads), kBlock, 0, c.stream>>>(G, H.rec);
     k_tag_resolve<1><<<blocks_for(nres), kBlock, 0, c.stream>>>(G, H.rec, O);
     G.xc = c.xv;
     G.yc = c.yu;
+    G.nyc = ny;
+    lines();
     TagOut OP{b.ghostP, b.hybridP, nullptr, nullptr, nullptr, nullptr, b.bipX, b.bipY, b.ippX, b.ippY, nullptr};
     k_tag_pressure_records<<<blocks_for(nthreads), kBlock, 0, c.stream>>>(G, H.rec);
     k_tag_resolve<2><<<blocks_for(nres), kBlock, 0, c.stream>>>(G, H.rec, OP);
     const int i0 = c.bb_tag.i0, i1 = c.bb_tag.i0 + w, j0 = c.bb_tag.j0, j1 = c.bb_tag.j0 + h;
     const int zrows = ref_threads(i1 - i0, 1);
-    k_zero_rows<<<blocks_for(zrows), kBlock, 0, c.stream>>>(b.ghostP, nx, i0, i1, j0, j1, zrows, nx);
-    k_zero_rows<<<blocks_for(zrows), kBlock, 0, c.stream>>>(b.ghostUV, nx - 1, i0, i1, j0, j1, zrows, nx - 1);
-    k_zero_rows<<<blocks_for(zrows), kBlock, 0, c.stream>>>(b.ghostUV + c.g.nU, nx, i0, i1, j0, j1, zrows, nx - 1);
+    const ZeroRows Z{{b.ghostP, b.ghostUV, b.ghostUV + c.g.nU}, {nx, nx - 1, nx}, {nx, nx - 1, nx - 1},
+                     i0, i1, j0, j1, zrows};
+    k_zero_rows<<<dim3(std::min(zrows, j1 - j0 + 1), 3), 32, (size_t)(w + 1) * sizeof(int), c.stream>>>(Z);
     // the interpolation plan of these tags
     IbPlan &P = H.plan;
     BoxLaunch B = box(c);
