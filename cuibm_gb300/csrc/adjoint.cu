@@ -1003,6 +1003,8 @@ void free_adjoint(Context &c)
 {
     if (!c.adj) return;
     AdjointState *A = static_cast<AdjointState *>(c.adj);
+    free_transposed_graph(A->S1T);
+    free_transposed_graph(A->S2T);
     for (void *p : A->allocs) cudaFree(p);
     delete A;
     c.adj = nullptr;

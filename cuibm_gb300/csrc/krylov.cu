@@ -542,9 +542,11 @@ void setup_transposed_system(Context &c, const LinearSystem &F, LinearSystem &S,
     S.amg = F.amg;
 }
 
+// One BiCGSTAB iteration of a transposed system; the kernel that tests convergence sets the
+// condition of the graph's loop
 template <class Op>
-static void transposed_iterations(Context &c, LinearSystem &S, Op A, const TransposeList &T, const double *b,
-                                  double *x)
+static void transposed_iteration(Context &c, LinearSystem &S, Op A, const TransposeList &T, double *x,
+                                 cudaGraphConditionalHandle h, int use)
 {
     const int n = S.n, nb = blocks_for(n);
     const bool sa = S.precond == PC_SMOOTHED_AGGREGATION;
@@ -552,55 +554,80 @@ static void transposed_iterations(Context &c, LinearSystem &S, Op A, const Trans
         if (S.sep) launch_separable_transposed(c, S, T, in, out);
         else launch_vcycle_transposed(c, S, T, in, out);
     };
-    k_bicg_init<<<nb, kBlock, 0, c.stream>>>(A, n, b, x, S.r, S.rs, S.p, S.partials, S.ks, nullptr, S.which, 0, 0);
-    CUIBM_TRY(cudaGetLastError());
-    KrylovScalars host{};
-    const int chunk = 4;
-    for (int done = 0; done <= S.maxit + chunk; done += chunk) {
-        for (int k = 0; k < chunk; ++k) {
-            if (sa) {
-                precond(S.p, S.Mp);
-                k_bicg_1<Op, 2><<<nb, kBlock, 0, c.stream>>>(A, n, S.p, S.dinv, S.Mp, S.AMp, S.rs, S.partials, S.ks);
-            } else {
-                k_bicg_1<Op, 1><<<nb, kBlock, 0, c.stream>>>(A, n, S.p, S.dinv, S.Mp, S.AMp, S.rs, S.partials, S.ks);
-            }
-            k_bicg_2<<<nb, kBlock, 0, c.stream>>>(n, S.r, S.AMp, S.s, S.partials, S.ks);
-            if (sa) {
-                precond(S.s, S.Ms);
-                k_bicg_3<Op, 2><<<nb, kBlock, 0, c.stream>>>(A, n, S.s, S.dinv, S.Ms, S.AMs, S.partials, S.ks);
-            } else {
-                k_bicg_3<Op, 1><<<nb, kBlock, 0, c.stream>>>(A, n, S.s, S.dinv, S.Ms, S.AMs, S.partials, S.ks);
-            }
-            k_bicg_4<<<nb, kBlock, 0, c.stream>>>(n, x, S.r, S.rs, S.s, S.Mp, S.Ms, S.AMs, S.partials, S.ks,
-                                                  nullptr, S.which, 0, 0);
-            k_bicg_5<<<nb, kBlock, 0, c.stream>>>(n, S.p, S.r, S.AMp, S.ks);
-        }
-        CUIBM_TRY(cudaGetLastError());
-        CUIBM_TRY(cudaMemcpyAsync(&host, S.ks, sizeof(host), cudaMemcpyDeviceToHost, c.stream));
-        CUIBM_TRY(cudaStreamSynchronize(c.stream));
-        if (host.status != KS_RUNNING) break;
+    if (sa) {
+        precond(S.p, S.Mp);
+        k_bicg_1<Op, 2><<<nb, kBlock, 0, c.stream>>>(A, n, S.p, S.dinv, S.Mp, S.AMp, S.rs, S.partials, S.ks);
+    } else {
+        k_bicg_1<Op, 1><<<nb, kBlock, 0, c.stream>>>(A, n, S.p, S.dinv, S.Mp, S.AMp, S.rs, S.partials, S.ks);
     }
+    k_bicg_2<<<nb, kBlock, 0, c.stream>>>(n, S.r, S.AMp, S.s, S.partials, S.ks);
+    if (sa) {
+        precond(S.s, S.Ms);
+        k_bicg_3<Op, 2><<<nb, kBlock, 0, c.stream>>>(A, n, S.s, S.dinv, S.Ms, S.AMs, S.partials, S.ks);
+    } else {
+        k_bicg_3<Op, 1><<<nb, kBlock, 0, c.stream>>>(A, n, S.s, S.dinv, S.Ms, S.AMs, S.partials, S.ks);
+    }
+    k_bicg_4<<<nb, kBlock, 0, c.stream>>>(n, x, S.r, S.rs, S.s, S.Mp, S.Ms, S.AMs, S.partials, S.ks, nullptr, S.which,
+                                          h, use);
+    k_bicg_5<<<nb, kBlock, 0, c.stream>>>(n, S.p, S.r, S.AMp, S.ks);
+    CUIBM_TRY(cudaGetLastError());
+}
+
+void free_transposed_graph(LinearSystem &S)
+{
+    if (S.t_exec) cudaGraphExecDestroy(S.t_exec);
+    if (S.t_graph) cudaGraphDestroy(S.t_graph);
+    S.t_exec = nullptr;
+    S.t_graph = nullptr;
+}
+
+// The whole solve as one graph - the residual and a WHILE node of iterations - so that a
+// solve is one launch and one wait.  With a launch per kernel and a look at the status every
+// four iterations, the reduced adjoint (59 x 59) spent more than half its time on the host.
+template <class Op>
+static void transposed_solve(Context &c, LinearSystem &S, Op A, const TransposeList &T, const double *b, double *x)
+{
+    const int n = S.n, nb = blocks_for(n);
+    const void *key[6] = {b, x, T.cnt, T.ent, S.sep, S.amg.empty() ? nullptr : S.amg[0]};
+    if (!S.t_exec || !std::equal(key, key + 6, S.t_key)) {
+        free_transposed_graph(S);
+        CUIBM_TRY(cudaStreamBeginCapture(c.stream, cudaStreamCaptureModeRelaxed));
+        try {
+            CondNode loop(c);
+            k_bicg_init<<<nb, kBlock, 0, c.stream>>>(A, n, b, x, S.r, S.rs, S.p, S.partials, S.ks, nullptr, S.which,
+                                                     loop.h, 1);
+            CUIBM_TRY(cudaGetLastError());
+            loop.add(cudaGraphCondTypeWhile, [&] { transposed_iteration(c, S, A, T, x, loop.h, 1); });
+        } catch (...) {
+            cudaGraph_t g = nullptr;
+            cudaStreamEndCapture(c.stream, &g);
+            if (g) cudaGraphDestroy(g);
+            throw;
+        }
+        CUIBM_TRY(cudaStreamEndCapture(c.stream, &S.t_graph));
+        CUIBM_TRY(cudaGraphInstantiate(&S.t_exec, S.t_graph, 0));
+        std::copy(key, key + 6, S.t_key);
+    }
+    CUIBM_TRY(cudaGraphLaunch(S.t_exec, c.stream));
 }
 
 // A^T x = b for system S.which, warm-started from x; returns the KStatus and the
-// iteration count.  The Poisson system's preconditioner is the transposed cycle of the
-// forward SA hierarchy (the same aggregates and prolongators, transposed level matrices).
+// iteration count.  The Poisson system's preconditioner is the transpose of the forward
+// one: the separable inverse with the body's sweep, or the transposed cycle of the forward
+// SA hierarchy (the same aggregates and prolongators, transposed level matrices).
 int launch_solve_transposed(Context &c, LinearSystem &S, LinearSystem &F, const TransposeList &T, const double *b,
                             double *x, int *iterations)
 {
     S.amg = F.amg;  // the forward hierarchy (rebuilt for a moving body between steps)
     S.sep = F.sep;  // so its preconditioner
     if (S.precond == PC_SMOOTHED_AGGREGATION && !S.sep) ensure_transposed_levels(c, F);
-    KrylovScalars hk{};
-    CUIBM_TRY(cudaMemcpyAsync(&hk, S.ks, sizeof(hk), cudaMemcpyDeviceToHost, c.stream));
-    CUIBM_TRY(cudaStreamSynchronize(c.stream));
-    hk.rtol = S.rtol;
-    hk.maxit = S.maxit;
-    CUIBM_TRY(cudaMemcpyAsync(S.ks, &hk, sizeof(hk), cudaMemcpyHostToDevice, c.stream));
+    // (both values are read before the calls return)
+    CUIBM_TRY(cudaMemcpyAsync(&S.ks->rtol, &S.rtol, sizeof(double), cudaMemcpyHostToDevice, c.stream));
+    CUIBM_TRY(cudaMemcpyAsync(&S.ks->maxit, &S.maxit, sizeof(int), cudaMemcpyHostToDevice, c.stream));
     if (S.which == 1)
-        transposed_iterations(c, S, Op1T{c.l1, c.g, T}, T, b, x);
+        transposed_solve(c, S, Op1T{c.l1, c.g, T}, T, b, x);
     else
-        transposed_iterations(c, S, Op2T{c.l2, c.g, T}, T, b, x);
+        transposed_solve(c, S, Op2T{c.l2, c.g, T}, T, b, x);
     KrylovScalars host{};
     CUIBM_TRY(cudaMemcpyAsync(&host, S.ks, sizeof(host), cudaMemcpyDeviceToHost, c.stream));
     CUIBM_TRY(cudaStreamSynchronize(c.stream));

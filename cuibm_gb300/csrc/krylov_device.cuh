@@ -229,4 +229,52 @@ static __global__ void __launch_bounds__(256) k_cg_3(int n, double *p, const dou
 inline Op1 op1(Context &c, const double *w) { return Op1{c.l1, c.g, w}; }
 inline Op2 op2(Context &c, const double *w) { return Op2{c.l2, c.g, w}; }
 
+// A conditional node after what c.stream has captured so far; its handle's value is 0 at
+// each launch of the graph.  make() creates the handle before the kernels that set it.
+struct CondNode {
+    Context &c;
+    cudaGraphConditionalHandle h{};
+
+    explicit CondNode(Context &c_) : c(c_)
+    {
+        cudaStreamCaptureStatus st;
+        cudaGraph_t graph;
+        CUIBM_TRY(cudaStreamGetCaptureInfo(c.stream, &st, nullptr, &graph, nullptr, nullptr, nullptr));
+        CUIBM_TRY(cudaGraphConditionalHandleCreate(&h, graph, 0, cudaGraphCondAssignDefault));
+    }
+    template <class F>
+    int add(cudaGraphConditionalNodeType type, const F &body)
+    {
+        cudaStreamCaptureStatus st;
+        cudaGraph_t graph;
+        const cudaGraphNode_t *deps = nullptr;
+        size_t ndeps = 0;
+        CUIBM_TRY(cudaStreamGetCaptureInfo(c.stream, &st, nullptr, &graph, &deps, nullptr, &ndeps));
+        cudaGraphNodeParams cp = {};
+        cp.type = cudaGraphNodeTypeConditional;
+        cp.conditional.handle = h;
+        cp.conditional.type = type;
+        cp.conditional.size = 1;
+        cudaGraphNode_t node;
+        CUIBM_TRY(cudaGraphAddNode(&node, graph, deps, nullptr, ndeps, &cp));
+        cudaStream_t main = c.stream, side = c.side_stream;
+        CUIBM_TRY(cudaStreamBeginCaptureToGraph(side, cp.conditional.phGraph_out[0], nullptr, nullptr, 0,
+                                                cudaStreamCaptureModeRelaxed));
+        c.stream = side;
+        try {
+            body();
+        } catch (...) {
+            c.stream = main;
+            cudaGraph_t dummy;
+            cudaStreamEndCapture(side, &dummy);
+            throw;
+        }
+        c.stream = main;
+        cudaGraph_t got;
+        CUIBM_TRY(cudaStreamEndCapture(side, &got));
+        CUIBM_TRY(cudaStreamUpdateCaptureDependencies(c.stream, &node, nullptr, 1, cudaStreamSetCaptureDependencies));
+        return count_kernel_nodes(got);
+    }
+};
+
 }  // namespace cuibm

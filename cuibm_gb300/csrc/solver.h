@@ -162,6 +162,11 @@ struct LinearSystem {
     double *aedef = nullptr;                // A e (the operator's row sums), with wdef
     double *ym = nullptr, *wdef = nullptr;  // constant-mode correction of the SA cycle (Poisson):
     double Edef = 0;                        // cycle output, A^T e, e^T A e
+    // a transposed system's whole solve as a graph (its right-hand side, solution and lists
+    // are the adjoint's own arrays): launched per solve, rebuilt when one of them changes
+    cudaGraphExec_t t_exec = nullptr;
+    cudaGraph_t t_graph = nullptr;
+    const void *t_key[6] = {};
     FusedSyncState *fsync = nullptr;
     void *fargs = nullptr;  // device copy of the solver arguments
 };
@@ -335,6 +340,7 @@ void refresh_system_diagonals(Context &c, LinearSystem &S);  // after the operat
 void setup_transposed_system(Context &c, const LinearSystem &F, LinearSystem &S, std::vector<void *> &allocs);
 int launch_solve_transposed(Context &c, LinearSystem &S, LinearSystem &F, const TransposeList &T, const double *b,
                             double *x, int *iterations);
+void free_transposed_graph(LinearSystem &S);
 void launch_apply_transposed(Context &c, int which, const TransposeList &T, const double *x, double *y);
 
 // fused_solve.cu
