@@ -390,13 +390,18 @@ static __device__ bool grid_sync(FusedSyncState *st, unsigned long long *trace, 
     __syncthreads();
     if (threadIdx.x == 0) {
         int good = 1;
-        __threadfence();
         const unsigned long long nb = gridDim.x;
-        const unsigned long long old = atomicAdd(&st->arrivals, 1ull);
+        // the block's writes before the barrier (ordered by __syncthreads) are released by
+        // the arrival and acquired by the wait: one release-add and one acquire-load a block
+        // where two sequentially consistent fences stood
+        unsigned long long old;
+        asm volatile("atom.add.release.gpu.u64 %0, [%1], %2;" : "=l"(old) : "l"(&st->arrivals), "l"(1ull) : "memory");
         const unsigned long long target = (old / nb + 1) * nb;
         unsigned long long t0 = 0;
         for (unsigned int spin = 0;; ++spin) {
-            if (*(volatile unsigned long long *)&st->arrivals >= target) break;
+            unsigned long long seen;
+            asm volatile("ld.acquire.gpu.u64 %0, [%1];" : "=l"(seen) : "l"(&st->arrivals) : "memory");
+            if (seen >= target) break;
             if ((spin & 127) == 127) {
                 if (*(volatile int *)&st->abort) {
                     good = 0;
@@ -412,7 +417,6 @@ static __device__ bool grid_sync(FusedSyncState *st, unsigned long long *trace, 
                 }
             }
         }
-        __threadfence();
         ok = good;
     }
     trace_stamp(trace, site);
