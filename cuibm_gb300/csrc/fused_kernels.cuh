@@ -525,9 +525,35 @@ __device__ __forceinline__ void vcycle_residual0_row(const Op &A, const FLevel<T
 // inverse has entries of order 1/lambda_min, and an FP32 product of it is noise.
 constexpr int kDenseMax = 1536;  // the coarsest level's size limit (kCoarse in amg.cu is below it)
 
+// The inverse is the same in every cycle: where a block's rows of it fit the launch's
+// dynamic shared memory (S.fused_smem in fused_solve.cu), the kernel loads them once at its
+// start (stage_inverse) and a coarsest solve then waits for b alone.  Streaming the rows from
+// L2 in each cycle took 7 us of a 50 us cycle at 1346 unknowns (five rounds of loads).
+__device__ __forceinline__ bool inverse_staged(int n)
+{
+    unsigned bytes;
+    asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(bytes));
+    const unsigned rows = (n + gridDim.x - 1) / gridDim.x;
+    return bytes > 0 && rows * (unsigned)n * 8u <= bytes;
+}
+template <class T>
+__device__ __forceinline__ void stage_inverse(const FArgs<T> &a)
+{
+    extern __shared__ double s_inv[];
+    if (a.nlev == 0) return;
+    const FLevel<T> &C = a.lev[a.nlev - 1];
+    const int n = C.n;
+    if (!inverse_staged(n)) return;
+    int q = 0;
+    for (int row = blockIdx.x; row < n; row += gridDim.x, ++q)
+        for (int k = threadIdx.x; k < n; k += blockDim.x) s_inv[q * n + k] = C.inv[(size_t)row * n + k];
+    // (the solve's first grid barrier comes before its first use)
+}
+
 template <class T>
 __device__ __forceinline__ void dense_solve(const FLevel<T> &C, const T *b, T *x)
 {
+    extern __shared__ double s_inv[];
     __shared__ double sb[kDenseMax];
     const int n = C.n;
     for (int k = threadIdx.x; k < n; k += blockDim.x) sb[k] = (double)__ldcg(b + k);
@@ -536,8 +562,7 @@ __device__ __forceinline__ void dense_solve(const FLevel<T> &C, const T *b, T *x
     // rows dealt to the blocks in turn (row r to block r mod grid), so that every SM
     // streams its share of the inverse rather than the first n / 16 blocks all of it
     const int nw = blockDim.x >> 5;
-    for (int row = blockIdx.x + gridDim.x * (threadIdx.x >> 5); row < n; row += gridDim.x * nw) {
-        const double *a = C.inv + (size_t)row * n;
+    auto dot = [&](const double *a) {
         double acc0 = 0, acc1 = 0;
         int k = lane;
 #pragma unroll 8
@@ -548,6 +573,12 @@ __device__ __forceinline__ void dense_solve(const FLevel<T> &C, const T *b, T *x
         if (k < n) acc0 += a[k] * sb[k];
         double s = acc0 + acc1;
         for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+        return s;
+    };
+    const bool staged = inverse_staged(n);
+    int q = threadIdx.x >> 5;
+    for (int row = blockIdx.x + gridDim.x * q; row < n; row += gridDim.x * nw, q += nw) {
+        const double s = staged ? dot(s_inv + q * n) : dot(C.inv + (size_t)row * n);
         if (lane == 0) x[row] = (T)s;
     }
 }
@@ -1480,6 +1511,7 @@ __global__ void __launch_bounds__(kFT, MINB) k_fused_solve(Op A, const FArgs<dou
         a.trace[0] = 1;
         a.trace[1] = global_ns() & 0xffffffffffffull;  // the start (site 0)
     }
+    if (PC == 2) stage_inverse(a);
     double res[4];
     int it = 0, status = KS_RUNNING, parity = 0;
     // rows taken four at a time, one at a time where the kernel is built for two blocks per
@@ -1519,6 +1551,7 @@ __global__ void __launch_bounds__(kFT, 1) k_fused_mixed(Op64 A, Op32 A32, const 
         a.trace[0] = 1;
         a.trace[1] = global_ns() & 0xffffffffffffull;  // the start (site 0)
     }
+    stage_inverse(*fp);
     double res[4];
     int it = 0, status = KS_RUNNING, parity = 0;
     const bool ok = bicg_solve<Op64, 2, double, true, Op32>(A, a, b, x, a.ks->rtol, a.ks->maxit, parity, res, it,
@@ -1555,6 +1588,7 @@ __global__ void __launch_bounds__(kFT, 1) k_fused_ir(Op64 A, Op32 A32, const FAr
         a.trace[0] = 1;
         a.trace[1] = global_ns() & 0xffffffffffffull;  // the start (site 0)
     }
+    if (PC == 2) stage_inverse(f);
     const double rtol = a.ks->rtol, floor_in = a.ks->inner_rtol;
     const int maxit = a.ks->maxit, maxit_in = a.ks->inner_maxit;
     int parity = 0, its = 0, status = KS_RUNNING;

@@ -97,7 +97,7 @@ static cudaLaunchConfig_t coop_config(Context &c, LinearSystem &S, cudaLaunchAtt
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(S.fused_grid);
     cfg.blockDim = dim3(S.fused_threads);
-    cfg.dynamicSmemBytes = 0;
+    cfg.dynamicSmemBytes = S.fused_smem;
     cfg.stream = c.stream;
     attr[0].id = cudaLaunchAttributeCooperative;
     attr[0].val.cooperative = 1;
@@ -440,13 +440,23 @@ void refresh_fused_hierarchy(Context &c, LinearSystem &S)
     if (!S.fused_fn) return;
     if (S.amg.empty() || (int)S.amg.size() > kMaxLevels || sa_coarsest_size(S) > kDenseMax)
         throw InputError("the rebuilt smoothed-aggregation hierarchy does not fit the persistent solver");
+    set_fused_grid(S, c.P.solverBlocks);  // (its coarsest size may have changed)
     upload_fargs(c, S);
 }
+
+constexpr int kInverseSmem = 160 * 1024;
 
 void set_fused_grid(LinearSystem &S, int blocks)
 {
     if (!S.fused_fn) return;
     S.fused_grid = blocks > 0 ? std::min(S.fused_grid_max, blocks) : S.fused_grid_default;
+    // the coarsest inverse's rows in shared memory (dense_solve) where a block's share fits
+    // beside the static arrays; batched solves share their SMs and keep none
+    S.fused_smem = 0;
+    if (S.precond == PC_SMOOTHED_AGGREGATION && S.fused_smem_max > 0) {
+        const size_t n = sa_coarsest_size(S), rows = (n + S.fused_grid - 1) / S.fused_grid;
+        if (rows * n * sizeof(double) <= S.fused_smem_max) S.fused_smem = (int)(rows * n * sizeof(double));
+    }
 }
 
 void setup_fused(Context &c, LinearSystem &S)
@@ -474,6 +484,11 @@ void setup_fused(Context &c, LinearSystem &S)
     S.fused_grid_default = sms * std::min(per_sm, want);
     S.fused_grid_max = sms * per_sm;
     S.fused_fn = fn;
+    S.fused_smem_max = 0;
+    if (S.precond == PC_SMOOTHED_AGGREGATION && c.P.solverPack != 2 && want == 1) {
+        CUIBM_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kInverseSmem));
+        S.fused_smem_max = kInverseSmem;
+    }
     set_fused_grid(S, c.P.solverBlocks);
     const int n = S.n;
     S.p2 = c.carve<double>(n);
