@@ -38,7 +38,7 @@
 
 #include <algorithm>
 #include <cmath>
-#include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "krylov_device.cuh"
@@ -98,6 +98,10 @@ struct SepPlan {
     int *prow = nullptr, *pidx = nullptr;
     double *cap = nullptr, *gap = nullptr, *q = nullptr, *y = nullptr, *rin = nullptr;
     char *pblock = nullptr;
+    // sums of the row kernels (k_row_*): four arrays of sums_cap, and the grid of one block a row
+    double *sums = nullptr;
+    int sums_cap = 0;
+    bool rows = false;    // their layout applies
     bool moving = false;  // a body's rows change: one Jacobi sweep on them beside A0^-1
     int tri_rows = 0;  // neighbouring rows a thread of k_sep_tri takes
     int max_nm() const { return grids > 1 ? std::max(a.f[0].nm, a.f[1].nm) : a.f[0].nm; }
@@ -824,6 +828,309 @@ __global__ void __launch_bounds__(256) k_sep_4(int n, double *x, double *r, doub
     }
 }
 
+// ---- the first iteration by rows ------------------------------------------------------------
+// Where the transform runs along a field's contiguous direction, the first iteration's vector
+// kernels take a block a row, as the splitting into digits does, and hand the digits of the
+// vector they form straight on.  Their sums and those of the operator kernels between them
+// stay partial: the kernel that needs a total adds the partials itself, in every block and in
+// the same order (about 1 us, in place of a fence, an atomic and a last block's sum at the
+// end of the kernel before: 4 to 6 us of a 10 us kernel at 270 x 270).  Only the kernels that
+// decide how the solve goes on end with a last block.
+struct RowSums {
+    double *sums;
+    int cap, ns, nr;  // partials of the starting kernel, of the operator kernels
+};
+template <int NV>
+__device__ __forceinline__ void partial_total(const double *p, int cap, int n, double (&t)[NV])
+{
+    __shared__ double sh[NV][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+        t[k] = 0;
+        for (int i = threadIdx.x; i < n; i += blockDim.x) t[k] += p[k * cap + i];
+    }
+    __syncthreads();  // (sh may be in use by an earlier call)
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+        for (int o = 16; o > 0; o >>= 1) t[k] += __shfl_xor_sync(0xffffffffu, t[k], o);
+        if (lane == 0) sh[k][w] = t[k];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+        t[k] = 0;
+        for (int q = 0; q < nw; ++q) t[k] += sh[k][q];
+    }
+}
+// a block's sums in every thread's v; thread 0 stores them
+template <int NV>
+__device__ __forceinline__ void partial_store(double (&v)[NV], double *p, int cap, int slot)
+{
+    __shared__ double sh[NV][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+        for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+        if (lane == 0) sh[k][w] = v[k];
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+#pragma unroll
+        for (int k = 0; k < NV; ++k) {
+            double a = 0;
+            for (int q = 0; q < nw; ++q) a += sh[k][q];
+            p[k * cap + slot] = a;
+        }
+}
+// the same, and the last block of the grid gets the totals (true in its thread 0)
+template <int NV>
+__device__ __forceinline__ bool partial_last(double (&v)[NV], double *p, int cap, int slot, int n, unsigned int *arrive)
+{
+    __shared__ bool last;
+    partial_store<NV>(v, p, cap, slot);
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicAdd(arrive, 1u) == (unsigned)n - 1;
+        __threadfence();
+    }
+    __syncthreads();
+    if (!last || threadIdx.x >= 32) return false;
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+        double a = 0;
+#pragma unroll 4
+        for (int b = threadIdx.x; b < n; b += 32) a += __ldcg(p + k * cap + b);
+        for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+        v[k] = a;
+    }
+    if (threadIdx.x == 0) *arrive = 0;
+    return threadIdx.x == 0;
+}
+
+#define ROW_PLACES(u, m) \
+    _Pragma("unroll") for (int u = 0, m = 2 * threadIdx.x; u < 2 * NP; ++u, m = 2 * (threadIdx.x + (u >> 1) * 128) + (u & 1))
+
+// r = b - A x (CG: of the system with the cell areas), its digits and ||r||^2, ||b||^2
+template <class Op, int L, int NP, bool CG>
+__global__ void __launch_bounds__(128) k_row_start(const __grid_constant__ SepArgs args, Op A,
+                                                   const double *__restrict__ b, const double *x, double *r, RowSums S)
+{
+    const SepDev &d = args.f[blockIdx.y];
+    const int R = blockIdx.x, n = d.nm;
+    if (R >= d.nr) return;  // (its partials stay the zeros they are set to)
+    const double cr = d.cr ? d.cr[R] : 1.0;
+    double v[2 * NP], t[2] = {0, 0};
+    ROW_PLACES(u, m)
+    {
+        v[u] = 0;
+        if (m < n) {
+            const int i = d.base + R * d.sr + m;
+            const double bi = b[i], ri = (CG ? A.w[i] * bi : bi) - A.row(i, PtrAccess{x});
+            const double ro = CG ? ri / A.w[i] : ri;
+            r[i] = ri;
+            t[0] += ro * ro;
+            t[1] += bi * bi;
+            v[u] = ri * (d.cm[m] * cr);
+        }
+    }
+    partial_store<2>(t, S.sums, S.cap, blockIdx.y * gridDim.x + R);
+    const double e = split_values<L, NP>(n, d.nch, d.A + (size_t)R * d.nch * L * kKC, v);
+    if (threadIdx.x == 0) d.sA[R] = e;
+}
+
+// a = A z and the partial sums y . a (TWO: and a . a; CG: and z . a with p = z)
+template <class Op, int KIND>
+__global__ void __launch_bounds__(256) k_row_apply(Op A, int n, const double *__restrict__ z, double *a,
+                                                   const double *__restrict__ y, double *p, RowSums S, int at)
+{
+    double v[2] = {0, 0};
+    SEP_ROWS(i, n)
+    {
+        const double ai = A.row(i, PtrAccess{z}), yi = y[i];
+        a[i] = ai;
+        if (KIND == 2) {
+            const double zi = z[i];
+            p[i] = zi;
+            v[0] += yi * zi;
+            v[1] += zi * ai;
+        } else {
+            v[0] += yi * ai;
+            if (KIND == 1) v[1] += ai * ai;
+        }
+    }
+    partial_store<2>(v, S.sums + (size_t)at * S.cap, S.cap, blockIdx.x);
+}
+
+// what a solve starts with, from the starting kernel's sums; false: it ends there
+__device__ __forceinline__ bool row_begin(const KrylovScalars *ks, const double (&t)[2], KrylovScalars &k)
+{
+    k = *ks;
+    k.rho = t[0];
+    k.rnorm = sqrt(t[0]);
+    k.bnorm = sqrt(t[1]);
+    k.tol = k.rtol * k.bnorm;
+    k.it = k.s_done = k.body_runs = 0;
+    k.status = KS_RUNNING;
+    return isfinite(k.rnorm) && isfinite(k.tol) && k.rnorm > k.tol && k.maxit > 0;
+}
+__device__ __forceinline__ void row_keep(KrylovScalars *ks, const KrylovScalars &k)
+{
+    ks->rho = k.rho;
+    ks->alpha = k.alpha;
+    ks->rnorm = k.rnorm;
+    ks->bnorm = k.bnorm;
+    ks->tol = k.tol;
+    ks->snorm = k.snorm;
+    ks->it = k.it;
+    ks->s_done = k.s_done;
+    ks->body_runs = k.body_runs;
+    ks->status = k.status;
+}
+
+// s = r - alpha A M p, x += alpha M p, the digits of s; the solve may end here
+template <int L, int NP>
+__global__ void __launch_bounds__(128) k_row_half(const __grid_constant__ SepArgs args, const double *__restrict__ r,
+                                                  const double *__restrict__ AMp, const double *__restrict__ Mp,
+                                                  double *s, double *x, RowSums S, KrylovScalars *ks, int *err,
+                                                  int which, cudaGraphConditionalHandle h, int use_cond)
+{
+    const SepDev &d = args.f[blockIdx.y];
+    const int R = blockIdx.x, n = R < d.nr ? d.nm : 0;
+    double t[2], a[1];
+    KrylovScalars k;
+    partial_total<2>(S.sums, S.cap, S.ns, t);
+    const bool on = row_begin(ks, t, k);
+    if (!on) {
+        if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
+            row_keep(ks, k);
+            finish_status(ks, err, which);
+            set_cond(h, use_cond, 0);
+        }
+        return;
+    }
+    partial_total<1>(S.sums + 2 * (size_t)S.cap, S.cap, S.nr, a);
+    k.alpha = k.rho / a[0];
+    const double cr = d.cr && n ? d.cr[R] : 1.0;
+    double v[2 * NP], q[1] = {0};
+    ROW_PLACES(u, m)
+    {
+        v[u] = 0;
+        if (m < n) {
+            const int i = d.base + R * d.sr + m;
+            const double si = r[i] - k.alpha * AMp[i];
+            s[i] = si;
+            x[i] += k.alpha * Mp[i];
+            q[0] += si * si;
+            v[u] = si * (d.cm[m] * cr);
+        }
+    }
+    if (n) {
+        const double e = split_values<L, NP>(n, d.nch, d.A + (size_t)R * d.nch * L * kKC, v);
+        if (threadIdx.x == 0) d.sA[R] = e;
+    }
+    if (partial_last<1>(q, S.sums + 4 * (size_t)S.cap, S.cap, blockIdx.y * gridDim.x + R, gridDim.x * gridDim.y,
+                        &ks->arrive)) {
+        k.snorm = sqrt(q[0]);
+        if (k.snorm <= k.tol) {
+            k.s_done = 1;
+            k.rnorm = k.snorm;
+            k.status = KS_CONVERGED;
+        } else {
+            k.body_runs = 1;
+        }
+        row_keep(ks, k);
+        set_cond(h, use_cond, k.status == KS_RUNNING);
+    }
+}
+
+// x += omega M s, r = s - omega A M s, rs = p = the residual the solve began with
+__global__ void __launch_bounds__(256) k_row_end(int n, double *x, double *r, double *rs, double *p,
+                                                 const double *__restrict__ s, const double *__restrict__ Ms,
+                                                 const double *__restrict__ AMs, RowSums S, KrylovScalars *ks, int *err,
+                                                 int which, cudaGraphConditionalHandle h, int use_cond)
+{
+    double o[2], v[2] = {0, 0};
+    partial_total<2>(S.sums + 2 * (size_t)S.cap, S.cap, S.nr, o);
+    const double omega = o[0] / o[1];
+    SEP_ROWS(i, n)
+    {
+        const double r0 = r[i];
+        rs[i] = r0;
+        p[i] = r0;
+        x[i] += omega * Ms[i];
+        const double ri = s[i] - omega * AMs[i];
+        r[i] = ri;
+        v[0] += r0 * ri;
+        v[1] += ri * ri;
+    }
+    if (partial_last<2>(v, S.sums + 4 * (size_t)S.cap, S.cap, blockIdx.x, gridDim.x, &ks->arrive)) {
+        ks->omega = omega;
+        ks->beta = (v[0] / ks->rho) * (ks->alpha / omega);
+        ks->rho = v[0];
+        ks->it += 1;
+        ks->rnorm = sqrt(v[1]);
+        finish_status(ks, err, which);
+        set_cond(h, use_cond, ks->status == KS_RUNNING);
+    }
+}
+
+// CG: x += alpha p, r -= alpha q, the digits of r; first: alpha from the sums before it
+template <int L, int NP>
+__global__ void __launch_bounds__(128) k_row_cg(const __grid_constant__ SepArgs args, const double *__restrict__ w,
+                                                const double *__restrict__ p, const double *__restrict__ q, double *r,
+                                                double *x, RowSums S, KrylovScalars *ks, int *err, int which, int first,
+                                                cudaGraphConditionalHandle h, int use_cond)
+{
+    const SepDev &d = args.f[blockIdx.y];
+    const int R = blockIdx.x, n = R < d.nr ? d.nm : 0;
+    KrylovScalars k;
+    if (first) {
+        double t[2], a[2];
+        partial_total<2>(S.sums, S.cap, S.ns, t);
+        if (!row_begin(ks, t, k)) {
+            if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
+                row_keep(ks, k);
+                finish_status(ks, err, which);
+                set_cond(h, use_cond, 0);
+            }
+            return;
+        }
+        partial_total<2>(S.sums + 2 * (size_t)S.cap, S.cap, S.nr, a);
+        k.rho = a[0];
+        k.alpha = a[0] / a[1];
+    } else {
+        k = *ks;
+        if (k.status != KS_RUNNING) return;
+    }
+    const double cr = d.cr && n ? d.cr[R] : 1.0;
+    double v[2 * NP], t[1] = {0};
+    ROW_PLACES(u, m)
+    {
+        v[u] = 0;
+        if (m < n) {
+            const int i = d.base + R * d.sr + m;
+            x[i] += k.alpha * p[i];
+            const double ri = r[i] - k.alpha * q[i], ro = ri / w[i];
+            r[i] = ri;
+            t[0] += ro * ro;
+            v[u] = ri * (d.cm[m] * cr);
+        }
+    }
+    if (n) {
+        const double e = split_values<L, NP>(n, d.nch, d.A + (size_t)R * d.nch * L * kKC, v);
+        if (threadIdx.x == 0) d.sA[R] = e;
+    }
+    if (partial_last<1>(t, S.sums + 4 * (size_t)S.cap, S.cap, blockIdx.y * gridDim.x + R, gridDim.x * gridDim.y,
+                        &ks->arrive)) {
+        k.it += 1;
+        k.rnorm = sqrt(t[0]);
+        row_keep(ks, k);
+        finish_status(ks, err, which);
+        set_cond(h, use_cond, ks->status == KS_RUNNING);
+    }
+}
+
 // A last correction x += M r for the residual that the solve ends with (a moving body's
 // solves): where the iteration stops, the level of the pressure - fixed by one pinned cell -
 // carries up to 2e-9 of it at a relative residual of 1e-12; M resolves it exactly
@@ -1011,7 +1318,7 @@ static void launch_tri(Context &c, const SepPlan &P)
 template <int L>
 static void apply_t(Context &c, const SepPlan &P, const double *in, double *out, int tr)
 {
-    launch_split<L, false>(c, P, in, tr);
+    if (in) launch_split<L, false>(c, P, in, tr);  // (null: the digits are there already)
     launch_gemm<L>(c, P, nullptr, 0);
     launch_tri(c, P);
     launch_split<L, true>(c, P, nullptr);
@@ -1157,7 +1464,7 @@ __global__ void k_sep_last(const __grid_constant__ SepArgs args, int n, const do
 constexpr int kPatchMax = 2048;  // patched rows: the capacitance matrix is 8 m^2 bytes, its set-up m applications
 
 // out = M in: five kernels, or thirteen with patched rows
-void launch_separable_apply(Context &c, LinearSystem &S, const double *in, double *out)
+void launch_separable_apply(Context &c, LinearSystem &S, const double *in, double *out, bool digits)
 {
     const SepPlan &P = *static_cast<const SepPlan *>(S.sep);
     if (P.moving) {
@@ -1169,10 +1476,10 @@ void launch_separable_apply(Context &c, LinearSystem &S, const double *in, doubl
         return;
     }
     if (!P.patched) {
-        apply_grid(c, P, in, out);
+        apply_grid(c, P, digits ? nullptr : in, out);
         return;
     }
-    apply_grid(c, P, in, P.y);
+    apply_grid(c, P, digits ? nullptr : in, P.y);
     RowGap A{c.l2, c.l2, c.g};
     A.plain.patch = RowPatch{};
     k_sep_gap<<<blocks_for(P.patched), kBlock, 0, c.stream>>>(A, P.patched, P.prow, P.y, P.gap);
@@ -1558,6 +1865,11 @@ void setup_separable(Context &c, LinearSystem &S)
         }
     }
     P->grids = (int)grids.size();
+    // the row kernels: contiguous rows of at most 1024 places, of an operator whose rows stay
+    P->rows = alongx && nm <= 1024 && !(S.which == 2 && c.P.solverType == ST_OSC);
+    P->sums_cap = std::max(kRowBlocks, nr * P->grids);
+    CUIBM_TRY(cudaMalloc(&P->sums, 6 * (size_t)P->sums_cap * sizeof(double)));
+    CUIBM_TRY(cudaMemsetAsync(P->sums, 0, 6 * (size_t)P->sums_cap * sizeof(double), c.stream));
     if (S.which != 2 || !c.l2.patch.pid) return;
     if (c.P.solverType == ST_OSC) {
         SepDev &d = P->a.f[0];
@@ -1581,6 +1893,7 @@ void free_separable(LinearSystem &S)
     SepPlan *P = static_cast<SepPlan *>(S.sep);
     if (!P) return;
     if (P->pblock) cudaFree(P->pblock);
+    if (P->sums) cudaFree(P->sums);
     for (char *b : P->block)
         if (b) cudaFree(b);
     delete P;
@@ -1603,9 +1916,91 @@ struct SepSolve {
         else f(StoredOp2{c.l2, S.diag, S.w, c.g.nx, c.g.ny});
     }
     int nb() const { return row_blocks(S.n); }
+    const SepPlan &plan() const { return *static_cast<const SepPlan *>(S.sep); }
+    RowSums sums() const
+    {
+        const SepPlan &P = plan();
+        return RowSums{P.sums, P.sums_cap, P.max_nr() * P.grids, nb()};
+    }
+    // f(digits, pairs a thread) as compile-time constants, for the row kernels
+    template <class F>
+    void with_rows(const F &f) const
+    {
+        const SepPlan &P = plan();
+        const int np = ((P.max_nm() + kKC - 1) / kKC * kKC + 255) / 256;
+        auto pairs = [&](auto l) {
+            if (np <= 1) f(l, std::integral_constant<int, 1>{});
+            else if (np <= 2) f(l, std::integral_constant<int, 2>{});
+            else f(l, std::integral_constant<int, 4>{});
+        };
+        if (P.digits == kDigits) pairs(std::integral_constant<int, kDigits>{});
+        else pairs(std::integral_constant<int, kDigitsMixed>{});
+    }
+    dim3 row_grid() const { return dim3(plan().max_nr(), plan().grids); }
+
+    // the first iteration by rows (k_row_*)
+    template <bool CG>
+    void row_start() const
+    {
+        with_op([&](auto A) {
+            with_rows([&](auto l, auto np) {
+                k_row_start<decltype(A), l(), np(), CG>
+                    <<<row_grid(), 128, 0, c.stream>>>(plan().a, A, b, x, S.r, sums());
+            });
+        });
+        CUIBM_TRY(cudaGetLastError());
+    }
+    void row_half(cudaGraphConditionalHandle h, int use) const
+    {
+        launch_separable_apply(c, S, S.r, S.Mp, true);
+        with_op([&](auto A) {
+            k_row_apply<decltype(A), 0>
+                <<<nb(), kBlock, 0, c.stream>>>(A, S.n, S.Mp, S.AMp, S.r, nullptr, sums(), 2);
+        });
+        with_rows([&](auto l, auto np) {
+            k_row_half<l(), np()><<<row_grid(), 128, 0, c.stream>>>(plan().a, S.r, S.AMp, S.Mp, S.s, x, sums(), S.ks,
+                                                                     c.err_word, S.which, h, use);
+        });
+        CUIBM_TRY(cudaGetLastError());
+    }
+    void row_rest(cudaGraphConditionalHandle h, int use) const
+    {
+        launch_separable_apply(c, S, S.s, S.Ms, true);
+        with_op([&](auto A) {
+            k_row_apply<decltype(A), 1>
+                <<<nb(), kBlock, 0, c.stream>>>(A, S.n, S.Ms, S.AMs, S.s, nullptr, sums(), 2);
+        });
+        k_row_end<<<nb(), kBlock, 0, c.stream>>>(S.n, x, S.r, S.rs, S.p, S.s, S.Ms, S.AMs, sums(), S.ks, c.err_word,
+                                                 S.which, h, use);
+        k_bicg_5<<<blocks_for(S.n), kBlock, 0, c.stream>>>(S.n, S.p, S.r, S.AMp, S.ks);
+        CUIBM_TRY(cudaGetLastError());
+    }
+    void row_cg(bool first, cudaGraphConditionalHandle h, int use) const
+    {
+        launch_separable_apply(c, S, S.r, S.z, true);
+        with_op([&](auto A) {
+            if (first) {
+                k_row_apply<decltype(A), 2><<<nb(), kBlock, 0, c.stream>>>(A, S.n, S.z, S.q, S.r, S.p, sums(), 2);
+            } else {
+                k_cg_rz<<<blocks_for(S.n), kBlock, 0, c.stream>>>(S.n, S.r, S.z, S.partials, S.ks);
+                k_cg_3<<<blocks_for(S.n), kBlock, 0, c.stream>>>(S.n, S.p, S.z, S.ks);
+                k_cg_1<<<blocks_for(S.n), kBlock, 0, c.stream>>>(A, S.n, S.p, S.q, S.partials, S.ks);
+            }
+        });
+        with_rows([&](auto l, auto np) {
+            k_row_cg<l(), np()><<<row_grid(), 128, 0, c.stream>>>(plan().a, S.w, S.p, S.q, S.r, x, sums(), S.ks,
+                                                                   c.err_word, S.which, first, h, use);
+        });
+        CUIBM_TRY(cudaGetLastError());
+    }
 
     void init() const
     {
+        if (plan().rows) {
+            if (S.krylov == KRYLOV_CG) row_start<true>();
+            else row_start<false>();
+            return;
+        }
         with_op([&](auto A) {
             if (S.krylov == KRYLOV_CG)
                 k_cg_init<decltype(A), 2><<<blocks_for(S.n), kBlock, 0, c.stream>>>(A, S.n, b, S.w, x, S.r, S.z, S.p, S.dinv,
@@ -1618,6 +2013,10 @@ struct SepSolve {
     // BiCGSTAB to the half step
     void half(bool first, cudaGraphConditionalHandle h, int use) const
     {
+        if (first && plan().rows) {
+            row_half(h, use);
+            return;
+        }
         launch_separable_apply(c, S, first ? S.r : S.p, S.Mp);
         with_op([&](auto A) {
             k_sep_1<<<nb(), kBlock, 0, c.stream>>>(A, S.n, S.Mp, S.AMp, first ? S.r : S.rs, S.partials, S.ks, first);
@@ -1628,6 +2027,10 @@ struct SepSolve {
     // and from there
     void rest(bool first, cudaGraphConditionalHandle h, int use) const
     {
+        if (first && plan().rows) {
+            row_rest(h, use);
+            return;
+        }
         launch_separable_apply(c, S, S.s, S.Ms);
         with_op([&](auto A) {
             k_sep_3<<<nb(), kBlock, 0, c.stream>>>(A, S.n, S.s, S.Ms, S.AMs, S.partials, S.ks);
@@ -1647,6 +2050,10 @@ struct SepSolve {
     }
     void cg(bool first, cudaGraphConditionalHandle h, int use) const
     {
+        if (plan().rows) {
+            row_cg(first, h, use);
+            return;
+        }
         launch_separable_apply(c, S, S.r, S.z);
         with_op([&](auto A) {
             if (first) {
