@@ -54,6 +54,7 @@ constexpr int kFlush = 4;        // chunks between flushes: 7 x 128 x 2^14 < 2^2
 // (28 n_m^2 bytes) outgrow what was measured, and the accumulators' range ends at 4096
 constexpr int kSepMax = 2048;
 constexpr int kTriThreads = 512;
+constexpr int kRowPlaces = 400;  // the row kernels' longest rows (at most 512: two pairs a thread)
 
 // Device view of one grid's plan.  The pressure system has one grid; the velocity system
 // two (u, v), which every kernel takes in one launch.
@@ -133,13 +134,18 @@ struct StoredOp2 {
         return w ? w[i] * y : y;
     }
 };
-struct StoredOp1 {  // without patched rows or row scales (the plain and external methods)
+struct StoredOp1 {  // without row scales (the methods other than the embedded one)
     Lhs1Coef c;
     const double *diag, *w;
     int nx, ny, nU;
     template <class X>
     __device__ __forceinline__ double row(int i, const X &x) const
     {
+        const int pk = c.patch.pid ? c.patch.pid[i] : -1;
+        if (pk >= 0) {
+            const double yp = patch_row(c.patch, pk, x(i), x);
+            return w ? w[i] * yp : yp;
+        }
         const bool u = i < nU;
         const int n = u ? nx - 1 : nx, m = u ? ny : ny - 1, k = u ? i : i - nU, J = k / n, I = k - J * n;
         const double *E = u ? c.uE : c.vE, *W = u ? c.uW : c.vW, *N = u ? c.uN : c.vN, *S = u ? c.uS : c.vS;
@@ -1336,14 +1342,27 @@ static void apply_grid(Context &c, const SepPlan &P, const double *in, double *o
 // A^-1 r = A0^-1 (r - E q) where (I + P A0^-1 E) q = P A0^-1 r.  The m x m capacitance matrix
 // is inverted once, at set-up, for a body whose rows stay; an application then is two of
 // A0^-1 and a dense m x m product.
-struct RowGap {  // (P y)_k at the patched cell i: its row less the row that A0 has there
+struct RowGap {  // (P y)_k at the patched row i: its row less the row that A0 has there
+    Lhs1Coef full1, plain1;
     Lhs2Coef full, plain;
     Grid g;
+    int which;
+    __device__ double at(int i, const double *__restrict__ y) const
+    {
+        if (which == 1) return lhs1_row(full1, g, i, y) - lhs1_row(plain1, g, i, y);
+        return lhs2_row(full, g, i, y) - lhs2_row(plain, g, i, y);
+    }
 };
+static RowGap row_gap(const Context &c, int which)
+{
+    RowGap A{c.l1, c.l1, c.l2, c.l2, c.g, which};
+    A.plain1.patch = A.plain.patch = RowPatch{};
+    return A;
+}
 __global__ void k_sep_gap(RowGap A, int m, const int *__restrict__ row, const double *__restrict__ y, double *gap)
 {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < m) gap[k] = lhs2_row(A.full, A.g, row[k], y) - lhs2_row(A.plain, A.g, row[k], y);
+    if (k < m) gap[k] = A.at(row[k], y);
 }
 
 // q = cap gap, a warp a row
@@ -1461,7 +1480,9 @@ __global__ void k_sep_last(const __grid_constant__ SepArgs args, int n, const do
     if (k >= 0) z[i] = y[i] + z[i] * row_ratio(d, i, k);
 }
 
-constexpr int kPatchMax = 2048;  // patched rows: the capacitance matrix is 8 m^2 bytes, its set-up m applications
+// patched rows: the capacitance matrix is 8 m^2 bytes and its set-up m applications (a velocity
+// system's twice the work of a pressure system's, against fewer iterations saved)
+static int patch_max(int which) { return which == 1 ? 1024 : 2048; }
 
 // out = M in: five kernels, or thirteen with patched rows
 void launch_separable_apply(Context &c, LinearSystem &S, const double *in, double *out, bool digits)
@@ -1480,8 +1501,7 @@ void launch_separable_apply(Context &c, LinearSystem &S, const double *in, doubl
         return;
     }
     apply_grid(c, P, digits ? nullptr : in, P.y);
-    RowGap A{c.l2, c.l2, c.g};
-    A.plain.patch = RowPatch{};
+    const RowGap A = row_gap(c, S.which);
     k_sep_gap<<<blocks_for(P.patched), kBlock, 0, c.stream>>>(A, P.patched, P.prow, P.y, P.gap);
     k_sep_cap<<<blocks_for(32L * P.patched), kBlock, 0, c.stream>>>(P.patched, P.cap, P.gap, P.q);
     k_sep_less<<<blocks_for(S.n), kBlock, 0, c.stream>>>(S.n, in, P.pidx, P.q, P.rin);
@@ -1515,7 +1535,7 @@ static bool build_patch(Context &c, LinearSystem &S, const std::vector<int> &pid
         }
     const int m = (int)rows.size();
     if (m == 0) return true;
-    if (m > kPatchMax) return false;
+    if (m > patch_max(S.which)) return false;
     const size_t n = S.n, w = (size_t)2 * m * m;
     const size_t bytes = (2 * n + (size_t)m * m + 2 * (size_t)m) * 8 + (n + (size_t)m) * 4;
     CUIBM_TRY(cudaMalloc(&P.pblock, bytes));
@@ -1538,8 +1558,7 @@ static bool build_patch(Context &c, LinearSystem &S, const std::vector<int> &pid
     int *bad = reinterpret_cast<int *>(fac + m), hbad = 0;
     CUIBM_TRY(cudaMemsetAsync(bad, 0, 4, c.stream));
     CUIBM_TRY(cudaMemsetAsync(P.rin, 0, n * 8, c.stream));
-    RowGap A{c.l2, c.l2, c.g};
-    A.plain.patch = RowPatch{};
+    const RowGap A = row_gap(c, S.which);
     for (int j = 0; j < m; ++j) {
         k_sep_unit<<<1, 1, 0, c.stream>>>(P.rin, j ? rows[j - 1] : -1, rows[j]);
         apply_grid(c, P, P.rin, P.y);
@@ -1602,7 +1621,7 @@ static bool separable_applies(const Context &c, const LinearSystem &S)
     if (S.which == 2) {
         if (S.precond != PC_SMOOTHED_AGGREGATION || c.P.saStructured != -1 || c.P.poisson.strength >= 0) return false;
     } else {
-        if (S.precond != PC_DIAGONAL || (c.P.solverType != ST_NAVIERSTOKES && c.P.solverType != ST_LUO)) return false;
+        if (S.precond != PC_DIAGONAL || c.P.solverType == ST_OSC) return false;
     }
     if (c.P.separable == 1) return true;
     const bool level = c.P.solverType == ST_NAVIERSTOKES || c.P.solverType == ST_FADLUN ||
@@ -1865,12 +1884,14 @@ void setup_separable(Context &c, LinearSystem &S)
         }
     }
     P->grids = (int)grids.size();
-    // the row kernels: contiguous rows of at most 1024 places, of an operator whose rows stay
-    P->rows = alongx && nm <= 1024 && !(S.which == 2 && c.P.solverType == ST_OSC);
+    // the row kernels: contiguous rows, of an operator whose rows stay (64 x 64 cavity step 220
+    // -> 205 us, 270 x 270 cylinder 442 -> 437, 512 x 512 mixed 753 -> 762: there the vector
+    // kernels are bound by bandwidth and the flat ones are the better)
+    P->rows = alongx && nm <= kRowPlaces && !(S.which == 2 && c.P.solverType == ST_OSC);
     P->sums_cap = std::max(kRowBlocks, nr * P->grids);
     CUIBM_TRY(cudaMalloc(&P->sums, 6 * (size_t)P->sums_cap * sizeof(double)));
     CUIBM_TRY(cudaMemsetAsync(P->sums, 0, 6 * (size_t)P->sums_cap * sizeof(double), c.stream));
-    if (S.which != 2 || !c.l2.patch.pid) return;
+    if (!(S.which == 1 ? c.l1.patch.pid : c.l2.patch.pid)) return;
     if (c.P.solverType == ST_OSC) {
         SepDev &d = P->a.f[0];
         d.patch = c.l2.patch;
@@ -1883,7 +1904,7 @@ void setup_separable(Context &c, LinearSystem &S)
         CUIBM_TRY(cudaMalloc(&P->pblock, 2 * (size_t)S.n * sizeof(double)));
         P->y = reinterpret_cast<double *>(P->pblock);
         P->rin = P->y + S.n;
-    } else if (!build_patch(c, S, c.fadlun.pid2)) {
+    } else if (!build_patch(c, S, S.which == 1 ? c.fadlun.pid1 : c.fadlun.pid2)) {
         free_separable(S);
     }
 }
@@ -1930,8 +1951,7 @@ struct SepSolve {
         const int np = ((P.max_nm() + kKC - 1) / kKC * kKC + 255) / 256;
         auto pairs = [&](auto l) {
             if (np <= 1) f(l, std::integral_constant<int, 1>{});
-            else if (np <= 2) f(l, std::integral_constant<int, 2>{});
-            else f(l, std::integral_constant<int, 4>{});
+            else f(l, std::integral_constant<int, 2>{});
         };
         if (P.digits == kDigits) pairs(std::integral_constant<int, kDigits>{});
         else pairs(std::integral_constant<int, kDigitsMixed>{});
