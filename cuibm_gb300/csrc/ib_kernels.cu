@@ -944,8 +944,8 @@ __global__ void k_plan_build(PlanGeom G, IbPlan P)
 }
 
 // ---- per-step immersed-boundary phases -------------------------------------------------
-// One block runs a sequence of the reference's IB phases on the plan's node lists
-// (a few hundred to a few thousand nodes), with __syncthreads between them.  Ghost
+// One cluster of blocks runs a sequence of the reference's IB phases on the plan's node lists
+// (a few hundred to a few thousand nodes), with a barrier between them.  Ghost
 // phases stage their new values and write them after a barrier, so every node
 // reads the field as it was before the phase (the reference's launch: all loads
 // precede all stores).  Phases run in this order, which contains each of the
@@ -975,10 +975,29 @@ struct IbStep {
 };
 
 constexpr int kIbThreads = 512;
+constexpr int kIbBlocks = 8;  // a cluster
 
-__global__ void __launch_bounds__(kIbThreads) k_ib_step(IbStep S, int phases)
+// The blocks are one cluster: an SM issues two FP64 operations a clock, so one block's
+// gathers and weights (a dozen operations a node) were bound by that, and the phases' order
+// needs no more than the cluster's barrier.
+__device__ __forceinline__ void ib_sync()
 {
-    const int t = threadIdx.x, T = blockDim.x;
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__global__ void __cluster_dims__(kIbBlocks, 1, 1) __launch_bounds__(kIbThreads) k_ib_step(IbStep S, int phases)
+{
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, T = gridDim.x * blockDim.x;
+    // quotients that every node shares, formed by one thread (an FP64 division in each of 512
+    // threads is some 4 us of the SM's FP64 issue)
+    __shared__ double shared_q[3];
+    if (threadIdx.x == 0) {
+        if (phases & PH_ROBIN) shared_q[0] = 1.0 * S.dt / S.dx[S.nx - 1];
+        if (phases & (PH_HYBRID_P | PH_GHOST_P)) {
+            shared_q[1] = (S.uB[0] - S.uBk[0]) / S.dt;
+            shared_q[2] = (S.vB[0] - S.vBk[0]) / S.dt;
+        }
+    }
+    __syncthreads();
     const int nx = S.nx, ny = S.ny, nU = (nx - 1) * ny;
     const IbPlan &P = S.P;
     double *f = S.vel;
@@ -986,11 +1005,11 @@ __global__ void __launch_bounds__(kIbThreads) k_ib_step(IbStep S, int phases)
         for (int r = t; r < 2 * ny - 1; r += T) {
             if (r < ny) {
                 const int J = r, I = nx - 1, i = J * (nx - 1) + I;
-                const double beta = 1.0 * S.dt / S.dx[I];
+                const double beta = shared_q[0];
                 S.xp[J] = S.xp[J] * (1 - beta) + beta * f[i - 1];
             } else {
                 const int J = r - ny, I = nx, i = J * nx + I;
-                const double beta = 1.0 * S.dt / S.dx[I - 1];
+                const double beta = shared_q[0];
                 S.xp[J + ny] = S.xp[J + ny] * (1 - beta) + beta * f[i + nU - 1];
             }
         }
@@ -1002,7 +1021,7 @@ __global__ void __launch_bounds__(kIbThreads) k_ib_step(IbStep S, int phases)
             const double a = P.hvAlpha[k];
             f[n] = (1 - a) * f[n] + a * S.ustar[n];
         }
-        __syncthreads();
+        ib_sync();
     }
     if (phases & PH_GHOST_U) {
         const int cnt = P.count[0];
@@ -1019,9 +1038,9 @@ __global__ void __launch_bounds__(kIbThreads) k_ib_step(IbStep S, int phases)
             S.imageValue[n] = val;
             S.stage[k] = 2 * qb - val;
         }
-        __syncthreads();
+        ib_sync();
         for (int k = t; k < cnt; k += T) f[P.gvNode[k]] = S.stage[k];
-        __syncthreads();
+        ib_sync();
     }
     if (phases & PH_INSIDE) {
         const int cnt = P.count[4];
@@ -1030,7 +1049,7 @@ __global__ void __launch_bounds__(kIbThreads) k_ib_step(IbStep S, int phases)
             const int n = P.inNode[k];
             f[n] = n >= nU ? vb : ub;
         }
-        __syncthreads();
+        ib_sync();
     }
     if (phases & PH_HYBRID_U) {
         const int cnt = P.count[1];
@@ -1048,9 +1067,9 @@ __global__ void __launch_bounds__(kIbThreads) k_ib_step(IbStep S, int phases)
             S.ustar[n] = s;
             S.imageValue[n] = si;
         }
-        __syncthreads();
+        ib_sync();
     }
-    const double dudt = (S.uB[0] - S.uBk[0]) / S.dt, dvdt = (S.vB[0] - S.vBk[0]) / S.dt;
+    const double dudt = shared_q[1], dvdt = shared_q[2];
     if (phases & PH_HYBRID_P) {
         const int cnt = P.count[3];
         for (int k = t; k < cnt; k += T) {
@@ -1064,7 +1083,7 @@ __global__ void __launch_bounds__(kIbThreads) k_ib_step(IbStep S, int phases)
             }
             S.pstar[ip] = s;
         }
-        __syncthreads();
+        ib_sync();
     }
     if (phases & PH_WEIGHT_P) {
         const int cnt = P.count[3];
@@ -1073,7 +1092,7 @@ __global__ void __launch_bounds__(kIbThreads) k_ib_step(IbStep S, int phases)
             const double a = P.hpAlpha[k];
             S.p[ip] = (1 - a) * S.p[ip] + a * S.pstar[ip];
         }
-        __syncthreads();
+        ib_sync();
     }
     if (phases & PH_GHOST_P) {
         const int cnt = P.count[2];
@@ -1093,7 +1112,7 @@ __global__ void __launch_bounds__(kIbThreads) k_ib_step(IbStep S, int phases)
             S.dpdn[ip] = d;
             S.stage[k] = v + d;
         }
-        __syncthreads();
+        ib_sync();
         for (int k = t; k < cnt; k += T) S.p[P.gpNode[k]] = S.stage[k];
     }
 }
@@ -1618,13 +1637,13 @@ void launch_tag_points(Context &c)
     launch_embedded_rows(c);
 }
 
-// one block runs the phases in k_ib_step's order on the plan of the current tags
+// one cluster runs the phases in k_ib_step's order on the plan of the current tags
 static void launch_ib(Context &c, int phases, double *vel)
 {
     IbArrays &b = c.ib;
     IbStep S{hostside(c).plan, c.g.nx, c.g.ny, vel, c.p, b.uB, b.vB, b.uBk, b.vBk, c.P.dt, b.ustar, b.pstar,
              b.imageValue, b.biP, b.dpdn, b.gnValue, c.bc[XPLUS], c.dx};
-    k_ib_step<<<1, kIbThreads, 0, c.stream>>>(S, phases);
+    k_ib_step<<<kIbBlocks, kIbThreads, 0, c.stream>>>(S, phases);
     CUIBM_TRY(cudaGetLastError());
 }
 
