@@ -1522,6 +1522,8 @@ void launch_separable_transposed(Context &c, LinearSystem &S, const TransposeLis
     CUIBM_TRY(cudaGetLastError());
 }
 
+static char *plan_malloc(size_t bytes);
+
 // The capacitance matrix of a fixed body's patched rows and its inverse.  False where it
 // cannot be inverted or the body has too many rows for it.
 static bool build_patch(Context &c, LinearSystem &S, const std::vector<int> &pid)
@@ -1538,7 +1540,7 @@ static bool build_patch(Context &c, LinearSystem &S, const std::vector<int> &pid
     if (m > patch_max(S.which)) return false;
     const size_t n = S.n, w = (size_t)2 * m * m;
     const size_t bytes = (2 * n + (size_t)m * m + 2 * (size_t)m) * 8 + (n + (size_t)m) * 4;
-    CUIBM_TRY(cudaMalloc(&P.pblock, bytes));
+    P.pblock = plan_malloc(bytes);
     P.y = reinterpret_cast<double *>(P.pblock);
     P.rin = P.y + n;
     P.cap = P.rin + n;
@@ -1548,8 +1550,7 @@ static bool build_patch(Context &c, LinearSystem &S, const std::vector<int> &pid
     P.prow = P.pidx + n;
     CUIBM_TRY(cudaMemcpyAsync(P.pidx, idx.data(), n * 4, cudaMemcpyHostToDevice, c.stream));
     CUIBM_TRY(cudaMemcpyAsync(P.prow, rows.data(), m * 4, cudaMemcpyHostToDevice, c.stream));
-    char *tmp = nullptr;
-    CUIBM_TRY(cudaMalloc(&tmp, (w + m) * 8 + 256));
+    char *tmp = plan_malloc((w + m) * 8 + 256);
     struct Freed {
         char *p;
         ~Freed() { cudaFree(p); }
@@ -1640,6 +1641,21 @@ struct SepGrid {
     std::vector<int> pin_m, pin_r;
 };
 
+// Device memory for the plan.  A context that does not get it keeps its smoothed-aggregation
+// or diagonal preconditioner (NoRoom, caught in setup_separable) instead of failing.
+struct NoRoom {};
+static char *plan_malloc(size_t bytes)
+{
+    void *p = nullptr;
+    const cudaError_t e = cudaMalloc(&p, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        throw NoRoom{};
+    }
+    CUIBM_TRY(e);
+    return static_cast<char *>(p);
+}
+
 // The tables of grid g into P.a.f[k]; false where the eigenvalues do not converge.  cb: the
 // modes a block of k_sep_tri takes (the same for all grids of a launch).
 static bool build_grid(Context &c, SepPlan &P, int g, const SepGrid &G, bool sym, int cb)
@@ -1691,7 +1707,7 @@ static bool build_grid(Context &c, SepPlan &P, int g, const SepGrid &G, bool sym
     const size_t ocmt = reserve(nm * 8), ocrt = reserve(nr * 8), osB2t = reserve(nm * 8), owr = reserve(nr * 8);
     const size_t ocm = reserve(nm * 8), ocr = reserve(nr * 8), oF0 = reserve(nm * 8), oF1 = reserve(nm * 8);
     const size_t oG0 = reserve(d.pins > 0 ? n * 8 : 8), oG1 = reserve(d.pins > 1 ? n * 8 : 8), ogm = reserve(nr * 8);
-    CUIBM_TRY(cudaMalloc(&P.block[g], need));
+    P.block[g] = plan_malloc(need);
     char *block = P.block[g];
     auto D = [&](size_t at) { return reinterpret_cast<double *>(block + at); };
     auto H = [&](size_t at) { return reinterpret_cast<__nv_bfloat16 *>(block + at); };
@@ -1699,10 +1715,9 @@ static bool build_grid(Context &c, SepPlan &P, int g, const SepGrid &G, bool sym
         CUIBM_TRY(cudaMemcpyAsync(dst, v.data(), v.size() * 8, cudaMemcpyHostToDevice, c.stream));
     };
     // set-up scratch, freed at the end
-    char *tmp = nullptr;
     const size_t bq = ((size_t)nm * nm * 8 + 255) & ~size_t(255), bs = (sweeps.size() * sizeof(Sweep) + 511) & ~size_t(255),
                  br = (rot.size() * sizeof(double2) + 511) & ~size_t(255), bv = (size_t)(4 * nm + 2 * nr) * 8;
-    CUIBM_TRY(cudaMalloc(&tmp, bq + bs + br + bv));
+    char *tmp = plan_malloc(bq + bs + br + bv);
     struct Freed {
         char *p;
         ~Freed() { cudaFree(p); }
@@ -1825,7 +1840,19 @@ static bool build_grid(Context &c, SepPlan &P, int g, const SepGrid &G, bool sym
     return true;
 }
 
+static void build_separable(Context &c, LinearSystem &S);
+
 void setup_separable(Context &c, LinearSystem &S)
+{
+    try {
+        build_separable(c, S);
+    } catch (const NoRoom &) {
+        CUIBM_TRY(cudaStreamSynchronize(c.stream));
+        free_separable(S);
+    }
+}
+
+static void build_separable(Context &c, LinearSystem &S)
 {
     S.sep = nullptr;
     if (!separable_applies(c, S) || !S.diag) return;  // (the stored diagonal comes with the persistent solver)
@@ -1889,7 +1916,7 @@ void setup_separable(Context &c, LinearSystem &S)
     // kernels are bound by bandwidth and the flat ones are the better)
     P->rows = alongx && nm <= kRowPlaces && !(S.which == 2 && c.P.solverType == ST_OSC);
     P->sums_cap = std::max(kRowBlocks, nr * P->grids);
-    CUIBM_TRY(cudaMalloc(&P->sums, 6 * (size_t)P->sums_cap * sizeof(double)));
+    P->sums = reinterpret_cast<double *>(plan_malloc(6 * (size_t)P->sums_cap * sizeof(double)));
     CUIBM_TRY(cudaMemsetAsync(P->sums, 0, 6 * (size_t)P->sums_cap * sizeof(double), c.stream));
     if (!(S.which == 1 ? c.l1.patch.pid : c.l2.patch.pid)) return;
     if (c.P.solverType == ST_OSC) {
@@ -1901,7 +1928,7 @@ void setup_separable(Context &c, LinearSystem &S)
         d.S = c.l2.S;
         d.nx = nx;
         P->moving = true;
-        CUIBM_TRY(cudaMalloc(&P->pblock, 2 * (size_t)S.n * sizeof(double)));
+        P->pblock = plan_malloc(2 * (size_t)S.n * sizeof(double));
         P->y = reinterpret_cast<double *>(P->pblock);
         P->rin = P->y + S.n;
     } else if (!build_patch(c, S, S.which == 1 ? c.fadlun.pid1 : c.fadlun.pid2)) {

@@ -121,3 +121,26 @@ def test_patched_rows_of_a_fixed_body(tmp_path, h, points, precision):
         rng = np.random.default_rng(points)
         check(s, rng.standard_normal(s.info.numP), rng.standard_normal(s.info.numP))
         assert s.iterations()[1] <= 3
+
+
+@pytest.mark.parametrize("method,precision,moving", [("LUO", None, False), ("LUO", "MIXED", False),
+                                                     ("FADLUN", None, False), ("FADLUN", "MIXED", False),
+                                                     ("OSC_CYLINDER", None, False), ("OSC_CYLINDER", None, True)])
+def test_body_methods_agree_with_smoothed_aggregation(tmp_path, method, precision, moving):
+    """Each immersed-boundary method's steps with the separable preconditioner and with smoothed
+    aggregation, both solved to 1e-12: u to 1e-9, p less its mean (one pinned corner cell fixes
+    its level) to 1e-8, the forces to 1e-9 of their size."""
+    motion = {"xCoefficient": 0.05, "uCoefficient": 0.05 * 2 * np.pi, "xfrequency": 1.0, "xPhase": 0.0,
+              "uPhase": 0.0} if moving else None
+    f = cases.cylinder(str(tmp_path / "c"), h=0.04, ratio=1.08, extent=4.0, core=0.7, points=78, nu=0.025, dt=0.01, nt=20,
+                       vel_tol=TOL, pois_tol=TOL, method=method, precision=precision, motion=motion)
+    out = []
+    for flag in ("1", "0"):
+        with solver(f, ["-separable", flag]) as s:
+            s.stepTime(15)
+            p = s.get("p")
+            out.append((s.get("u"), p - p.mean(), np.array(s.forces())))
+    (u, p, fo), (us, ps, fs) = out
+    assert np.linalg.norm(u - us) <= 1e-9 * np.linalg.norm(us)
+    assert np.linalg.norm(p - ps) <= 1e-8 * np.linalg.norm(ps)
+    assert np.max(np.abs(fo - fs)) <= 1e-9 * max(1.0, np.max(np.abs(fs)))
