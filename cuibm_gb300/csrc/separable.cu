@@ -47,7 +47,11 @@
 namespace cuibm {
 
 constexpr int kDigits = 7;       // digits of the FP64 solves: 28 products a dense product
-constexpr int kDigitsMixed = 4;  // mixed precision: 31 bits below the row's largest value, 10 products
+// Mixed precision with a Fadlun body: 31 bits below the row's largest value, 10 products, and an
+// application more.  The plain method's mixed solves take kDigits too: one application of 28
+// products is cheaper than two of 10 (velocity, 64 x 64 71 against 131 us, 270 x 270 122 against
+// 207, 512 x 512 217 against 307)
+constexpr int kDigitsMixed = 4;
 constexpr int kKC = 32;          // terms of a chunk of the dense product's sum
 constexpr int kFlush = 4;        // chunks between flushes: 7 x 128 x 2^14 < 2^24
 // Transforms up to this length; from there on the products (n_m^2 n_r) and the tables
@@ -587,9 +591,9 @@ static int tri_modes(int nm, int nr) { return nm >= 600 && nr <= kTriRows / 2 ? 
 
 // the factors of Y + lambda_k, one thread a mode, and their products over each thread's
 // rows of k_sep_tri; the constant's mode gets reg on its first diagonal
-__global__ void k_sep_factor(int nm, int nr, int nq, int m, const double *__restrict__ up, const double *__restrict__ dn,
-                             const double *__restrict__ lam, double shift, int k0, double reg, double *l, double *c, double *inv,
-                             double *Pf, double *Pb)
+__global__ void k_sep_factor(int nm, int nr, int nq, int m, const double *__restrict__ up,
+                             const double *__restrict__ dn, const double *__restrict__ lam, double shift, int k0,
+                             double reg, double *l, double *c, double *inv, double *Pf, double *Pb)
 {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= nm) return;
@@ -1316,8 +1320,17 @@ static void launch_tri(Context &c, const SepPlan &P)
     const dim3 grid((nm + cb - 1) / cb, P.grids);
     auto go = [&](auto *fn, size_t smem) { fn<<<grid, kTriThreads, smem, c.stream>>>(P.a, m); };
     const size_t rows = (size_t)m * kTriThreads * sizeof(double);
-    if (cb == 8) m <= 4 ? go(k_sep_tri<8, 4>, 0) : m <= 8 ? go(k_sep_tri<8, 8>, 0) : m <= 16 ? go(k_sep_tri<8, 16>, 0) : go(k_sep_tri<8, 0>, rows);
-    else m <= 2 ? go(k_sep_tri<4, 2>, 0) : m <= 4 ? go(k_sep_tri<4, 4>, 0) : m <= 8 ? go(k_sep_tri<4, 8>, 0) : go(k_sep_tri<4, 0>, rows);
+    if (cb == 8) {
+        if (m <= 4) go(k_sep_tri<8, 4>, 0);
+        else if (m <= 8) go(k_sep_tri<8, 8>, 0);
+        else if (m <= 16) go(k_sep_tri<8, 16>, 0);
+        else go(k_sep_tri<8, 0>, rows);
+    } else {
+        if (m <= 2) go(k_sep_tri<4, 2>, 0);
+        else if (m <= 4) go(k_sep_tri<4, 4>, 0);
+        else if (m <= 8) go(k_sep_tri<4, 8>, 0);
+        else go(k_sep_tri<4, 0>, rows);
+    }
     CUIBM_TRY(cudaGetLastError());
 }
 
@@ -1613,7 +1626,10 @@ static double predicted_velocity_steps(const Context &c, double rtol)
     const double q = (std::sqrt(1 + 2 * s) - 1) / (std::sqrt(1 + 2 * s) + 1);
     return q > 0 ? std::log(2 / rtol) / (2 * std::log(1 / q)) : 0.0;
 }
-constexpr double kVelocitySteps = 5;
+// From this predicted count on (FP64, one application against n steps of the diagonal one: 64 x
+// 64 70 us against 97 at 3.8 and 124 at 5.2, 270 x 270 122 against 115 and 146, 512 x 512 218
+// against 191 and 247; 900 x 900 745 against 662 at 5.2 and 819 at 6.6)
+static double velocity_steps(const LinearSystem &S) { return S.n > 600000 ? 6.5 : 5; }
 
 static bool separable_applies(const Context &c, const LinearSystem &S)
 {
@@ -1628,7 +1644,7 @@ static bool separable_applies(const Context &c, const LinearSystem &S)
     const bool level = c.P.solverType == ST_NAVIERSTOKES || c.P.solverType == ST_FADLUN ||
                        (c.g.nP < kLevelMax && c.P.solverPack != 2 &&
                         c.P.poisson.precision == PRECISION_FP64);
-    return level && (S.which == 2 || predicted_velocity_steps(c, S.rtol) >= kVelocitySteps);
+    return level && (S.which == 2 || predicted_velocity_steps(c, S.rtol) >= velocity_steps(S));
 }
 
 // One grid's operator: shift + X + Y with the coefficients towards the next and the
@@ -1895,7 +1911,7 @@ static void build_separable(Context &c, LinearSystem &S)
     }
     SepPlan *P = new SepPlan();
     S.sep = P;
-    P->digits = S.precision == PRECISION_MIXED ? kDigitsMixed : kDigits;
+    P->digits = S.precision == PRECISION_MIXED && c.P.solverType == ST_FADLUN ? kDigitsMixed : kDigits;
     int nm = 0, nr = 0;
     for (const SepGrid &G : grids) {
         nm = std::max(nm, (int)G.um.size());
