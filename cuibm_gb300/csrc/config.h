@@ -63,8 +63,8 @@ struct Params {
                             // (64 registers a thread), so two solves can share an SM
     int saStructured = -1;  // -saStructured 1 / 0: the Poisson system's structured smoothed
                             // aggregation wherever it applies / never (-1: from 200k unknowns)
-    int separable = -1;     // -separable 1 / 0: the pressure system's separable preconditioner wherever
-                            // it applies / never (-1: by the rule in separable.cu)
+    int separable = -1;     // -separable 1 / 0: the separable preconditioner wherever it applies / never
+                            // (-1: by the rule in separable.cu)
     // flow
     double nu = 0.01, uInitial = 1.0, vInitial = 0.0, uPerturb = 0.0, vPerturb = 0.0;
     BC bc[4][2];

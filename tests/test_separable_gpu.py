@@ -70,7 +70,7 @@ def test_solves_meet_the_residual_bound(tmp_path, nx, ny, ratio, krylov, precisi
         rng = np.random.default_rng(nx * 1000 + ny)
         for b in (rng.standard_normal(i.numP), np.repeat(rng.standard_normal(ny), nx)):
             check(s, b, rng.standard_normal(i.numP))
-            assert s.iterations()[1] <= 3  # the inverse to rounding (mixed precision: to 2^-31)
+            assert s.iterations()[1] <= 3  # the inverse to rounding
         check(s, rng.standard_normal(i.numUV), rng.standard_normal(i.numUV), system=1)
 
 
