@@ -252,22 +252,27 @@ __global__ void k_sep_split_table(const double *__restrict__ src, int n, int nch
     if (threadIdx.x == 0) scale[r] = s * pow2(-50) * (extra ? extra[r] : 1.0);
 }
 
-// both sums over the block, in every thread
-__device__ __forceinline__ void block_sums(double &a, double &b)
+// A block's sums, the one of v[k] in every lane of warp k.  An FP64 warp instruction takes its
+// quarter of an SM 64 cycles (two lanes a clock an SM; a square root 650, a division 570:
+// measured), so that five shuffled adds a value in every warp cost more than the B / 32 + 5
+// adds of one warp a value over shared memory.
+template <int NV, int B>
+__device__ __forceinline__ double block_total(const double (&v)[NV])
 {
-    __shared__ double2 sh[32];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int o = 16; o > 0; o >>= 1) {
-        a += __shfl_xor_sync(0xffffffffu, a, o);
-        b += __shfl_xor_sync(0xffffffffu, b, o);
-    }
-    if (lane == 0) sh[w] = make_double2(a, b);
+    static_assert(NV <= B / 32, "a warp a value");
+    __shared__ double sh[NV][B];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    __syncthreads();  // (sh may be in use by an earlier call)
+#pragma unroll
+    for (int k = 0; k < NV; ++k) sh[k][threadIdx.x] = v[k];
     __syncthreads();
-    a = b = 0;
-    for (int k = 0; k < nw; ++k) {
-        a += sh[k].x;
-        b += sh[k].y;
+    double a = 0;
+    if (w < NV) {
+#pragma unroll
+        for (int j = 0; j < B / 32; ++j) a += sh[w][lane + 32 * j];
+        for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
     }
+    return a;
 }
 
 // One grid row to digits, a block a row.  SPEC false: a field (times the scaling that
@@ -328,8 +333,13 @@ __global__ void __launch_bounds__(128) k_sep_split(const __grid_constant__ SepAr
             f0 += F0[k] * h0[k];
             f1 += F1[k] * h1[k];
         }
-        const double fm = d.h[d.k0] * d.mean, gm = d.gm[R];
-        block_sums(f0, f1);
+        const double fm = d.h[d.k0] * d.mean, gm = d.gm[R], part[2] = {f0, f1};
+        __shared__ double tot[2];
+        const double total = block_total<2, 128>(part);
+        if (threadIdx.x < 64 && threadIdx.x % 32 == 0) tot[threadIdx.x / 32] = total;
+        __syncthreads();
+        f0 = tot[0];
+        f1 = tot[1];
         // f = (f0, f1, fm), without f1 for one pinned cell
         const double a1 = two ? f1 : fm, a2 = two ? fm : 0.0;
         const double q0 = d.K[0] * f0 + d.K[1] * a1 + d.K[2] * a2, q1 = d.K[3] * f0 + d.K[4] * a1 + d.K[5] * a2,
@@ -675,42 +685,47 @@ __global__ void k_sep_constant(int n, int k0, const double *__restrict__ v, doub
 static int row_blocks(int n) { return std::min(kRowBlocks, blocks_for(n)); }
 #define SEP_ROWS(i, n) for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < (n); i += gridDim.x * blockDim.x)
 
-template <int NV>
-__device__ __forceinline__ bool row_sums(double (&v)[NV], double *partials, unsigned int *arrive)
+// a block's sums to its places of the partial sums
+template <int NV, int B>
+__device__ __forceinline__ void partial_store(const double (&v)[NV], double *p, int cap, int slot)
 {
-    __shared__ double sh[NV][kBlock / 32];
+    const double a = block_total<NV, B>(v);
+    const int w = threadIdx.x >> 5;
+    if (w < NV && threadIdx.x % 32 == 0) p[(size_t)w * cap + slot] = a;
+}
+// the same, and the last of the n blocks gets the totals (true in its thread 0)
+template <int NV, int B>
+__device__ __forceinline__ bool partial_last(double (&v)[NV], double *p, int cap, int slot, int n, unsigned int *arrive)
+{
     __shared__ bool last;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-    for (int k = 0; k < NV; ++k) {
-        for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
-        if (lane == 0) sh[k][w] = v[k];
+    __shared__ double tot[NV];
+    const int w = threadIdx.x >> 5;
+    partial_store<NV, B>(v, p, cap, slot);
+    if (w < NV && threadIdx.x % 32 == 0) __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        last = atomicAdd(arrive, 1u) == (unsigned)n - 1;
+        __threadfence();
     }
     __syncthreads();
-    if (w != 0) return false;
-#pragma unroll
-    for (int k = 0; k < NV; ++k) {
-        v[k] = lane < kBlock / 32 ? sh[k][lane] : 0.0;
-        for (int o = kBlock / 64; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
-        if (lane == 0) partials[k * kRowBlocks + blockIdx.x] = v[k];
-    }
-    if (lane == 0) {
-        __threadfence();
-        last = atomicAdd(arrive, 1u) == gridDim.x - 1;
-        __threadfence();
-    }
-    __syncwarp();
     if (!last) return false;
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
-        double a = 0;
-#pragma unroll 4
-        for (int b = lane; b < (int)gridDim.x; b += 32) a += __ldcg(partials + k * kRowBlocks + b);
-        for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
-        v[k] = a;
+        v[k] = 0;
+        for (int b = threadIdx.x; b < n; b += B) v[k] += __ldcg(p + (size_t)k * cap + b);
     }
-    if (lane == 0) *arrive = 0;
-    return lane == 0;
+    const double a = block_total<NV, B>(v);
+    if (w < NV && threadIdx.x % 32 == 0) tot[w] = a;
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < NV; ++k) v[k] = tot[k];
+    if (threadIdx.x == 0) *arrive = 0;
+    return threadIdx.x == 0;
+}
+template <int NV>
+__device__ __forceinline__ bool row_sums(double (&v)[NV], double *partials, unsigned int *arrive)
+{
+    return partial_last<NV, kBlock>(v, partials, kRowBlocks, blockIdx.x, gridDim.x, arrive);
 }
 
 // BiCGSTAB as in krylov.cu with two differences: the first half iteration takes r for its
@@ -850,72 +865,14 @@ struct RowSums {
     double *sums;
     int cap, ns, nr;  // partials of the starting kernel, of the operator kernels
 };
-template <int NV>
-__device__ __forceinline__ void partial_total(const double *p, int cap, int n, double (&t)[NV])
+// the sum of n partials, by one warp, in every lane
+__device__ __forceinline__ double partial_total(const double *p, int n)
 {
-    __shared__ double sh[NV][32];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-#pragma unroll
-    for (int k = 0; k < NV; ++k) {
-        t[k] = 0;
-        for (int i = threadIdx.x; i < n; i += blockDim.x) t[k] += p[k * cap + i];
-    }
-    __syncthreads();  // (sh may be in use by an earlier call)
-#pragma unroll
-    for (int k = 0; k < NV; ++k) {
-        for (int o = 16; o > 0; o >>= 1) t[k] += __shfl_xor_sync(0xffffffffu, t[k], o);
-        if (lane == 0) sh[k][w] = t[k];
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < NV; ++k) {
-        t[k] = 0;
-        for (int q = 0; q < nw; ++q) t[k] += sh[k][q];
-    }
-}
-// a block's sums in every thread's v; thread 0 stores them
-template <int NV>
-__device__ __forceinline__ void partial_store(double (&v)[NV], double *p, int cap, int slot)
-{
-    __shared__ double sh[NV][32];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-#pragma unroll
-    for (int k = 0; k < NV; ++k) {
-        for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
-        if (lane == 0) sh[k][w] = v[k];
-    }
-    __syncthreads();
-    if (threadIdx.x == 0)
-#pragma unroll
-        for (int k = 0; k < NV; ++k) {
-            double a = 0;
-            for (int q = 0; q < nw; ++q) a += sh[k][q];
-            p[k * cap + slot] = a;
-        }
-}
-// the same, and the last block of the grid gets the totals (true in its thread 0)
-template <int NV>
-__device__ __forceinline__ bool partial_last(double (&v)[NV], double *p, int cap, int slot, int n, unsigned int *arrive)
-{
-    __shared__ bool last;
-    partial_store<NV>(v, p, cap, slot);
-    if (threadIdx.x == 0) {
-        __threadfence();
-        last = atomicAdd(arrive, 1u) == (unsigned)n - 1;
-        __threadfence();
-    }
-    __syncthreads();
-    if (!last || threadIdx.x >= 32) return false;
-#pragma unroll
-    for (int k = 0; k < NV; ++k) {
-        double a = 0;
+    double a = 0;
 #pragma unroll 4
-        for (int b = threadIdx.x; b < n; b += 32) a += __ldcg(p + k * cap + b);
-        for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-        v[k] = a;
-    }
-    if (threadIdx.x == 0) *arrive = 0;
-    return threadIdx.x == 0;
+    for (int i = threadIdx.x % 32; i < n; i += 32) a += p[i];
+    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    return a;
 }
 
 #define ROW_PLACES(u, m) \
@@ -944,7 +901,7 @@ __global__ void __launch_bounds__(128) k_row_start(const __grid_constant__ SepAr
             v[u] = ri * (d.cm[m] * cr);
         }
     }
-    partial_store<2>(t, S.sums, S.cap, blockIdx.y * gridDim.x + R);
+    partial_store<2, 128>(t, S.sums, S.cap, blockIdx.y * gridDim.x + R);
     const double e = split_values<L, NP>(n, d.nch, d.A + (size_t)R * d.nch * L * kKC, v);
     if (threadIdx.x == 0) d.sA[R] = e;
 }
@@ -969,20 +926,38 @@ __global__ void __launch_bounds__(256) k_row_apply(Op A, int n, const double *__
             if (KIND == 1) v[1] += ai * ai;
         }
     }
-    partial_store<2>(v, S.sums + (size_t)at * S.cap, S.cap, blockIdx.x);
+    partial_store<2, kBlock>(v, S.sums + (size_t)at * S.cap, S.cap, blockIdx.x);
 }
 
-// what a solve starts with, from the starting kernel's sums; false: it ends there
-__device__ __forceinline__ bool row_begin(const KrylovScalars *ks, const double (&t)[2], KrylovScalars &k)
+// What a solve starts with, from the starting kernel's sums (false: it ends there), and its
+// first alpha, from the NA sums of the operator kernel.  A warp a sum, then a warp a square
+// root or division, once a block.
+template <int NA>
+__device__ __forceinline__ bool row_begin(const RowSums &S, const KrylovScalars *ks, KrylovScalars &k)
 {
+    __shared__ double tot[2 + NA], fin[3];
+    const int w = threadIdx.x >> 5;
+    const bool head = threadIdx.x % 32 == 0;
     k = *ks;
-    k.rho = t[0];
-    k.rnorm = sqrt(t[0]);
-    k.bnorm = sqrt(t[1]);
+    if (w < 2 + NA) {
+        const double a = partial_total(S.sums + (size_t)w * S.cap, w < 2 ? S.ns : S.nr);
+        if (head) tot[w] = a;
+    }
+    __syncthreads();
+    if (w == 0 && head) fin[0] = sqrt(tot[0]);
+    if (w == 1 && head) fin[1] = sqrt(tot[1]);
+    if (w == 2 && head) fin[2] = NA == 1 ? tot[0] / tot[2] : tot[2] / tot[1 + NA];
+    __syncthreads();
+    k.rho = tot[0];
+    k.rnorm = fin[0];
+    k.bnorm = fin[1];
     k.tol = k.rtol * k.bnorm;
     k.it = k.s_done = k.body_runs = 0;
     k.status = KS_RUNNING;
-    return isfinite(k.rnorm) && isfinite(k.tol) && k.rnorm > k.tol && k.maxit > 0;
+    if (!(isfinite(k.rnorm) && isfinite(k.tol) && k.rnorm > k.tol && k.maxit > 0)) return false;
+    if (NA == 2) k.rho = tot[2];
+    k.alpha = fin[2];
+    return true;
 }
 __device__ __forceinline__ void row_keep(KrylovScalars *ks, const KrylovScalars &k)
 {
@@ -1007,11 +982,20 @@ __global__ void __launch_bounds__(128) k_row_half(const __grid_constant__ SepArg
 {
     const SepDev &d = args.f[blockIdx.y];
     const int R = blockIdx.x, n = R < d.nr ? d.nm : 0;
-    double t[2], a[1];
     KrylovScalars k;
-    partial_total<2>(S.sums, S.cap, S.ns, t);
-    const bool on = row_begin(ks, t, k);
-    if (!on) {
+    // the row's loads are under way while the sums are formed
+    double ri[2 * NP], ai[2 * NP], zi[2 * NP], xi[2 * NP], ci[2 * NP];
+    ROW_PLACES(u, m)
+    {
+        const bool in = m < n;
+        const int i = d.base + R * d.sr + m;
+        ri[u] = in ? r[i] : 0.0;
+        ai[u] = in ? AMp[i] : 0.0;
+        zi[u] = in ? Mp[i] : 0.0;
+        xi[u] = in ? x[i] : 0.0;
+        ci[u] = in ? d.cm[m] : 0.0;
+    }
+    if (!row_begin<1>(S, ks, k)) {
         if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
             row_keep(ks, k);
             finish_status(ks, err, which);
@@ -1019,8 +1003,6 @@ __global__ void __launch_bounds__(128) k_row_half(const __grid_constant__ SepArg
         }
         return;
     }
-    partial_total<1>(S.sums + 2 * (size_t)S.cap, S.cap, S.nr, a);
-    k.alpha = k.rho / a[0];
     const double cr = d.cr && n ? d.cr[R] : 1.0;
     double v[2 * NP], q[1] = {0};
     ROW_PLACES(u, m)
@@ -1028,18 +1010,18 @@ __global__ void __launch_bounds__(128) k_row_half(const __grid_constant__ SepArg
         v[u] = 0;
         if (m < n) {
             const int i = d.base + R * d.sr + m;
-            const double si = r[i] - k.alpha * AMp[i];
+            const double si = ri[u] - k.alpha * ai[u];
             s[i] = si;
-            x[i] += k.alpha * Mp[i];
+            x[i] = xi[u] + k.alpha * zi[u];
             q[0] += si * si;
-            v[u] = si * (d.cm[m] * cr);
+            v[u] = si * (ci[u] * cr);
         }
     }
     if (n) {
         const double e = split_values<L, NP>(n, d.nch, d.A + (size_t)R * d.nch * L * kKC, v);
         if (threadIdx.x == 0) d.sA[R] = e;
     }
-    if (partial_last<1>(q, S.sums + 4 * (size_t)S.cap, S.cap, blockIdx.y * gridDim.x + R, gridDim.x * gridDim.y,
+    if (partial_last<1, 128>(q, S.sums + 4 * (size_t)S.cap, S.cap, blockIdx.y * gridDim.x + R, gridDim.x * gridDim.y,
                         &ks->arrive)) {
         k.snorm = sqrt(q[0]);
         if (k.snorm <= k.tol) {
@@ -1060,9 +1042,17 @@ __global__ void __launch_bounds__(256) k_row_end(int n, double *x, double *r, do
                                                  const double *__restrict__ AMs, RowSums S, KrylovScalars *ks, int *err,
                                                  int which, cudaGraphConditionalHandle h, int use_cond)
 {
-    double o[2], v[2] = {0, 0};
-    partial_total<2>(S.sums + 2 * (size_t)S.cap, S.cap, S.nr, o);
-    const double omega = o[0] / o[1];
+    __shared__ double o[2], quotient;
+    const int w = threadIdx.x >> 5;
+    if (w < 2) {
+        const double a = partial_total(S.sums + (size_t)(2 + w) * S.cap, S.nr);
+        if (threadIdx.x % 32 == 0) o[w] = a;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) quotient = o[0] / o[1];
+    __syncthreads();
+    const double omega = quotient;
+    double v[2] = {0, 0};
     SEP_ROWS(i, n)
     {
         const double r0 = r[i];
@@ -1074,7 +1064,7 @@ __global__ void __launch_bounds__(256) k_row_end(int n, double *x, double *r, do
         v[0] += r0 * ri;
         v[1] += ri * ri;
     }
-    if (partial_last<2>(v, S.sums + 4 * (size_t)S.cap, S.cap, blockIdx.x, gridDim.x, &ks->arrive)) {
+    if (partial_last<2, kBlock>(v, S.sums + 4 * (size_t)S.cap, S.cap, blockIdx.x, gridDim.x, &ks->arrive)) {
         ks->omega = omega;
         ks->beta = (v[0] / ks->rho) * (ks->alpha / omega);
         ks->rho = v[0];
@@ -1096,9 +1086,7 @@ __global__ void __launch_bounds__(128) k_row_cg(const __grid_constant__ SepArgs 
     const int R = blockIdx.x, n = R < d.nr ? d.nm : 0;
     KrylovScalars k;
     if (first) {
-        double t[2], a[2];
-        partial_total<2>(S.sums, S.cap, S.ns, t);
-        if (!row_begin(ks, t, k)) {
+        if (!row_begin<2>(S, ks, k)) {
             if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
                 row_keep(ks, k);
                 finish_status(ks, err, which);
@@ -1106,9 +1094,6 @@ __global__ void __launch_bounds__(128) k_row_cg(const __grid_constant__ SepArgs 
             }
             return;
         }
-        partial_total<2>(S.sums + 2 * (size_t)S.cap, S.cap, S.nr, a);
-        k.rho = a[0];
-        k.alpha = a[0] / a[1];
     } else {
         k = *ks;
         if (k.status != KS_RUNNING) return;
@@ -1131,7 +1116,7 @@ __global__ void __launch_bounds__(128) k_row_cg(const __grid_constant__ SepArgs 
         const double e = split_values<L, NP>(n, d.nch, d.A + (size_t)R * d.nch * L * kKC, v);
         if (threadIdx.x == 0) d.sA[R] = e;
     }
-    if (partial_last<1>(t, S.sums + 4 * (size_t)S.cap, S.cap, blockIdx.y * gridDim.x + R, gridDim.x * gridDim.y,
+    if (partial_last<1, 128>(t, S.sums + 4 * (size_t)S.cap, S.cap, blockIdx.y * gridDim.x + R, gridDim.x * gridDim.y,
                         &ks->arrive)) {
         k.it += 1;
         k.rnorm = sqrt(t[0]);
