@@ -485,19 +485,21 @@ __global__ void __launch_bounds__(32 * WM * WN, 2) k_sep_gemm(const __grid_const
 }
 
 // ---- the tridiagonal solves -----------------------------------------------------------------
-// A block solves CB modes; kTriThreads / CB threads share a mode's rows, m = ceil(nr / that)
+// A block of T threads solves CB modes; T / CB threads share a mode's rows, m = ceil(nr / that)
 // neighbouring rows each.  Forward d_J = r_J + l_J d_J-1 and backward x_J = inv_J d_J + c_J
 // x_J+1 are linear recurrences: each thread runs its rows from zero, the threads' ends are
 // joined by a scan of affine maps in shared memory (the factors' products over a thread's
 // rows are tables), and each thread runs its rows again from the true start.  922 rows in
-// sequence would be 1844 dependent FP64 operations; this way it is 4 x 15 and two scans of
-// 6 steps.
-template <int CB>
+// sequence would be 1844 dependent FP64 operations; this way it is 5 x 15 and two scans of
+// 6 steps.  The bound is FP64 issue, 64 cycles a warp instruction on a quarter of an SM, and
+// a scan's 4 instructions a step are work that the rows alone would not need: so as few
+// threads a mode as the rows a thread can hold (16) allow.
+template <int CB, int T>
 __device__ __forceinline__ double tri_scan(double end, double prod, bool up, double *se, double *sp)
 {
     // inclusive scan over q of x -> end + prod x, from q = 0 up or from the last down;
     // returns the value that enters this thread's rows
-    constexpr int NQ = kTriThreads / CB;
+    constexpr int NQ = T / CB;
     const int tid = threadIdx.x, q = up ? tid / CB : NQ - 1 - tid / CB, step = up ? CB : -CB;
     int cur = 0;
     se[tid] = end;
@@ -505,8 +507,8 @@ __device__ __forceinline__ double tri_scan(double end, double prod, bool up, dou
     __syncthreads();
 #pragma unroll
     for (int o = 1; o < NQ; o <<= 1) {
-        const double *e = se + cur * kTriThreads, *p = sp + cur * kTriThreads;
-        double *en = se + (cur ^ 1) * kTriThreads, *pn = sp + (cur ^ 1) * kTriThreads;
+        const double *e = se + cur * T, *p = sp + cur * T;
+        double *en = se + (cur ^ 1) * T, *pn = sp + (cur ^ 1) * T;
         double ee = e[tid], pp = p[tid];
         if (q >= o) {
             const int from = tid - o * step;
@@ -518,7 +520,7 @@ __device__ __forceinline__ double tri_scan(double end, double prod, bool up, dou
         cur ^= 1;
         __syncthreads();
     }
-    const double in = q > 0 ? se[cur * kTriThreads + tid - step] : 0.0;
+    const double in = q > 0 ? se[cur * T + tid - step] : 0.0;
     __syncthreads();
     return in;
 }
@@ -526,12 +528,12 @@ __device__ __forceinline__ double tri_scan(double end, double prod, bool up, dou
 // M: rows a thread holds in registers, every load of the kernel issued at its start (0: any
 // number, the rows in shared memory and the tables read as they are needed).  512 x 512: 15
 // us with the tables read in four rounds.
-template <int CB, int M>
-__global__ void __launch_bounds__(kTriThreads) k_sep_tri(const __grid_constant__ SepArgs args, int m)
+template <int CB, int M, int T>
+__global__ void __launch_bounds__(T) k_sep_tri(const __grid_constant__ SepArgs args, int m)
 {
     const SepDev &d = args.f[blockIdx.y];
     extern __shared__ double row[];  // M = 0: [m][thread]: r, then inv d
-    __shared__ double se[2 * kTriThreads], sp[2 * kTriThreads];
+    __shared__ double se[2 * T], sp[2 * T];
     const int tid = threadIdx.x, n = d.nm;
     const int k = blockIdx.x * CB + tid % CB, q = tid / CB;
     const int J0 = min(q * m, d.nr), J1 = min(J0 + m, d.nr), cnt = k < n ? J1 - J0 : 0;
@@ -552,7 +554,7 @@ __global__ void __launch_bounds__(kTriThreads) k_sep_tri(const __grid_constant__
 #pragma unroll
         for (int t = 0; t < M; ++t)
             if (t < cnt) x = r[t] + l[t] * x;
-        x = tri_scan<CB>(x, pf, true, se, sp);
+        x = tri_scan<CB, T>(x, pf, true, se, sp);
 #pragma unroll
         for (int t = 0; t < M; ++t) {
             x = r[t] + l[t] * x;
@@ -562,7 +564,7 @@ __global__ void __launch_bounds__(kTriThreads) k_sep_tri(const __grid_constant__
 #pragma unroll
         for (int t = M - 1; t >= 0; --t)
             if (t < cnt) x = r[t] + cc[t] * x;
-        x = tri_scan<CB>(x, pb, false, se, sp);
+        x = tri_scan<CB, T>(x, pb, false, se, sp);
 #pragma unroll
         for (int t = M - 1; t >= 0; --t)
             if (t < cnt) {
@@ -573,22 +575,22 @@ __global__ void __launch_bounds__(kTriThreads) k_sep_tri(const __grid_constant__
 #pragma unroll 4
         for (int t = 0; t < cnt; ++t) {
             const double r = d.h[at + (size_t)t * n];
-            row[t * kTriThreads + tid] = r;
+            row[t * T + tid] = r;
             x = r + d.l[at + (size_t)t * n] * x;
         }
-        x = tri_scan<CB>(x, pf, true, se, sp);
+        x = tri_scan<CB, T>(x, pf, true, se, sp);
 #pragma unroll 4
         for (int t = 0; t < cnt; ++t) {
-            x = row[t * kTriThreads + tid] + d.l[at + (size_t)t * n] * x;
-            row[t * kTriThreads + tid] = x * d.inv[at + (size_t)t * n];
+            x = row[t * T + tid] + d.l[at + (size_t)t * n] * x;
+            row[t * T + tid] = x * d.inv[at + (size_t)t * n];
         }
         x = 0;
 #pragma unroll 4
-        for (int t = cnt - 1; t >= 0; --t) x = row[t * kTriThreads + tid] + d.c[at + (size_t)t * n] * x;
-        x = tri_scan<CB>(x, pb, false, se, sp);
+        for (int t = cnt - 1; t >= 0; --t) x = row[t * T + tid] + d.c[at + (size_t)t * n] * x;
+        x = tri_scan<CB, T>(x, pb, false, se, sp);
 #pragma unroll 4
         for (int t = cnt - 1; t >= 0; --t) {
-            x = row[t * kTriThreads + tid] + d.c[at + (size_t)t * n] * x;
+            x = row[t * T + tid] + d.c[at + (size_t)t * n] * x;
             d.h[at + (size_t)t * n] = x;
         }
     }
@@ -598,6 +600,15 @@ __global__ void __launch_bounds__(kTriThreads) k_sep_tri(const __grid_constant__
 // rows fit shared memory; kTriRows rows are what 4 modes a block can hold
 constexpr int kTriRows = 6400;
 static int tri_modes(int nm, int nr) { return nm >= 600 && nr <= kTriRows / 2 ? 8 : 4; }
+// Threads of a block of 4 modes: the fewest whose 32 or 64 threads a mode hold its rows.  Against
+// 128 threads a mode at every size, a step of the cavity 64 x 64 196 -> 183 us, Re 40 (270 x
+// 270) 390 -> 377, Fadlun (162 x 162) 409 -> 383, mixed cavity 512 x 512 567 -> 556, Poisson
+// 662 x 326 324 -> 316; longer rows stay in shared memory
+static int tri_threads(int nm, int nr)
+{
+    if (tri_modes(nm, nr) == 8) return kTriThreads;
+    return nr <= 32 * 16 ? 128 : nr <= 64 * 16 ? 256 : kTriThreads;
+}
 
 // the factors of Y + lambda_k, one thread a mode, and their products over each thread's
 // rows of k_sep_tri; the constant's mode gets reg on its first diagonal
@@ -1301,20 +1312,27 @@ static void split_table(Context &c, const double *src, int rows, int n, int nch,
 static void launch_tri(Context &c, const SepPlan &P)
 {
     const int nm = P.max_nm(), nr = P.max_nr();
-    const int cb = tri_modes(nm, nr), m = P.tri_rows;
+    const int cb = tri_modes(nm, nr), threads = tri_threads(nm, nr), m = P.tri_rows;
     const dim3 grid((nm + cb - 1) / cb, P.grids);
-    auto go = [&](auto *fn, size_t smem) { fn<<<grid, kTriThreads, smem, c.stream>>>(P.a, m); };
+    auto go = [&](auto *fn, size_t smem) { fn<<<grid, threads, smem, c.stream>>>(P.a, m); };
     const size_t rows = (size_t)m * kTriThreads * sizeof(double);
     if (cb == 8) {
-        if (m <= 4) go(k_sep_tri<8, 4>, 0);
-        else if (m <= 8) go(k_sep_tri<8, 8>, 0);
-        else if (m <= 16) go(k_sep_tri<8, 16>, 0);
-        else go(k_sep_tri<8, 0>, rows);
+        if (m <= 4) go(k_sep_tri<8, 4, kTriThreads>, 0);
+        else if (m <= 8) go(k_sep_tri<8, 8, kTriThreads>, 0);
+        else if (m <= 16) go(k_sep_tri<8, 16, kTriThreads>, 0);
+        else go(k_sep_tri<8, 0, kTriThreads>, rows);
+    } else if (threads == 128) {
+        if (m <= 2) go(k_sep_tri<4, 2, 128>, 0);
+        else if (m <= 4) go(k_sep_tri<4, 4, 128>, 0);
+        else if (m <= 6) go(k_sep_tri<4, 6, 128>, 0);
+        else if (m <= 9) go(k_sep_tri<4, 9, 128>, 0);
+        else if (m <= 12) go(k_sep_tri<4, 12, 128>, 0);
+        else go(k_sep_tri<4, 16, 128>, 0);
+    } else if (threads == 256) {
+        if (m <= 12) go(k_sep_tri<4, 12, 256>, 0);
+        else go(k_sep_tri<4, 16, 256>, 0);
     } else {
-        if (m <= 2) go(k_sep_tri<4, 2>, 0);
-        else if (m <= 4) go(k_sep_tri<4, 4>, 0);
-        else if (m <= 8) go(k_sep_tri<4, 8>, 0);
-        else go(k_sep_tri<4, 0>, rows);
+        go(k_sep_tri<4, 0, kTriThreads>, rows);
     }
     CUIBM_TRY(cudaGetLastError());
 }
@@ -1657,9 +1675,9 @@ static char *plan_malloc(size_t bytes)
     return static_cast<char *>(p);
 }
 
-// The tables of grid g into P.a.f[k]; false where the eigenvalues do not converge.  cb: the
-// modes a block of k_sep_tri takes (the same for all grids of a launch).
-static bool build_grid(Context &c, SepPlan &P, int g, const SepGrid &G, bool sym, int cb)
+// The tables of grid g into P.a.f[k]; false where the eigenvalues do not converge.  nq: the
+// threads a mode of k_sep_tri (the same for all grids of a launch).
+static bool build_grid(Context &c, SepPlan &P, int g, const SepGrid &G, bool sym, int nq)
 {
     SepDev &d = P.a.f[g];
     const int L = P.digits, nm = (int)G.um.size(), nr = (int)G.ur.size();
@@ -1693,7 +1711,6 @@ static bool build_grid(Context &c, SepPlan &P, int g, const SepGrid &G, bool sym
     for (int J = 0; J < nr; ++J) cr[J] = sym ? 1 / G.wr[J] : 1.0;
 
     // one allocation for all tables and work arrays
-    const int nq = kTriThreads / cb;
     const size_t n = (size_t)nm * nr, dig = (size_t)d.nch * L * kKC;
     size_t need = 0;
     auto reserve = [&](size_t bytes) {
@@ -1759,8 +1776,8 @@ static bool build_grid(Context &c, SepPlan &P, int g, const SepGrid &G, bool sym
         split_table<kDigitsMixed>(c, Q, nm, nm, d.nch, nm, 1, vet, H(oB2), D(osB2t));
         split_table<kDigitsMixed>(c, Q, nm, nm, d.nch, nm, 1, vem, H(oB2), D(osB2));
     }
-    allow_smem(k_sep_tri<8, 0>, 200 * 1024);
-    allow_smem(k_sep_tri<4, 0>, 200 * 1024);
+    allow_smem(k_sep_tri<8, 0, kTriThreads>, 200 * 1024);
+    allow_smem(k_sep_tri<4, 0, kTriThreads>, 200 * 1024);
     const double reg = d.pins ? G.ur[0] : 0.0;
     k_sep_factor<<<(nm + 31) / 32, 32, 0, c.stream>>>(nm, nr, nq, P.tri_rows, vur, vdr, vl, G.shift, k0, reg, D(ol), D(oc),
                                                       D(oi), D(oPf), D(oPb));
@@ -1902,11 +1919,11 @@ static void build_separable(Context &c, LinearSystem &S)
         nm = std::max(nm, (int)G.um.size());
         nr = std::max(nr, (int)G.ur.size());
     }
-    const int cb = tri_modes(nm, nr), nq = kTriThreads / cb;
+    const int nq = tri_threads(nm, nr) / tri_modes(nm, nr);
     P->tri_rows = (nr + nq - 1) / nq;
     for (size_t g = 0; g < grids.size(); ++g) {
         P->grids = 1;
-        if (!build_grid(c, *P, (int)g, grids[g], S.w != nullptr, cb)) {
+        if (!build_grid(c, *P, (int)g, grids[g], S.w != nullptr, nq)) {
             free_separable(S);
             return;
         }

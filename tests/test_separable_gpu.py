@@ -58,7 +58,7 @@ def check(s, b, p0, system=2):
 
 SIZES = [(3, 3, 1.0), (5, 4, 1.3), (31, 40, 1.05), (32, 33, 1.0), (33, 32, 1.0), (64, 65, 1.02), (129, 63, 1.0),
          (257, 90, 1.01), (700, 24, 1.0), (24, 700, 1.0), (290, 1100, 1.0), (521, 530, 1.004), (610, 601, 1.0),
-         (1033, 1040, 1.0)]
+         (1033, 1040, 1.0), (40, 512, 1.0), (40, 513, 1.0), (40, 1024, 1.0), (40, 1025, 1.0)]
 
 
 @pytest.mark.parametrize("nx,ny,ratio", SIZES)
@@ -74,7 +74,8 @@ def test_solves_meet_the_residual_bound(tmp_path, nx, ny, ratio, krylov, precisi
         check(s, rng.standard_normal(i.numUV), rng.standard_normal(i.numUV), system=1)
 
 
-@pytest.mark.parametrize("nx,ny,ratio", [(3, 3, 1.0), (33, 32, 1.0), (65, 31, 1.03), (120, 257, 1.0), (514, 130, 1.0)])
+@pytest.mark.parametrize("nx,ny,ratio", [(3, 3, 1.0), (33, 32, 1.0), (65, 31, 1.03), (120, 257, 1.0), (514, 130, 1.0),
+                                         (40, 512, 1.0), (40, 513, 1.0), (1024, 40, 1.0), (40, 1025, 1.0)])
 @pytest.mark.parametrize("krylov,precision", [("BICGSTAB", None), ("CG", None), ("BICGSTAB", "MIXED")])
 def test_velocity_solves_meet_the_residual_bound(tmp_path, nx, ny, ratio, krylov, precision):
     """nu large enough that the diagonal preconditioner would take tens of iterations."""
