@@ -379,7 +379,10 @@ __device__ __forceinline__ void cp16(unsigned dst, const void *src)
 // shared memory is one chunk of the tile's rows of both factors, kKC terms of every digit;
 // a row is 64 L + 16 bytes there, an odd number of 16-byte units, so ldmatrix meets no
 // bank conflict.  A warp holds its L digit fragments of A and walks the digits of B: 2 L
-// ldmatrix for L (L + 1) mma.
+// ldmatrix for L (L + 1) mma.  The bound is the latency between dependent instructions of few
+// warps: with the next fragments and the copies to a later stage issued among the mma (and the
+// copies' addresses formed once), a step of the mixed cavity 512 x 512 went from 556 to 517 us,
+// Re 40 (270 x 270) from 377 to 364, a Poisson solve at 662 x 326 from 316 to 298.
 template <int L, int WM, int WN, int ST>
 __global__ void __launch_bounds__(32 * WM * WN, 2) k_sep_gemm(const __grid_constant__ SepArgs args,
                                                              double *__restrict__ field, int back)
@@ -401,16 +404,21 @@ __global__ void __launch_bounds__(32 * WM * WN, 2) k_sep_gemm(const __grid_const
     const int wm = warp / WN, wn = warp % WN;
     const size_t rowBytes = (size_t)nch * L * kKC * 2;
 
-    auto load = [&](int ch) {
-        const unsigned s = sbase + (ch % ST) * STAGE;
-        constexpr int U = 4 * L;  // 16-byte units of a row and chunk
-        for (int u = threadIdx.x; u < (TM + TN) * U; u += T) {
-            const int row = u / U, k = u - row * U;
-            const char *g = row < TM
-                                ? reinterpret_cast<const char *>(A) + (size_t)min(m0 + row, M - 1) * rowBytes
-                                : reinterpret_cast<const char *>(B) + (size_t)min(n0 + row - TM, N - 1) * rowBytes;
-            cp16(s + row * RB + k * 16, g + (size_t)ch * U * 16 + k * 16);
-        }
+    // a thread's 16-byte units of a chunk: the same places in every stage
+    constexpr int U = 4 * L, UNITS = (TM + TN) * U, CNT = (UNITS + T - 1) / T;
+    const char *src[CNT];
+    unsigned dst[CNT];
+#pragma unroll
+    for (int i = 0; i < CNT; ++i) {
+        const int u = min((int)threadIdx.x + i * T, UNITS - 1), row = u / U, k = u - row * U;
+        src[i] = (row < TM ? reinterpret_cast<const char *>(A) + (size_t)min(m0 + row, M - 1) * rowBytes
+                           : reinterpret_cast<const char *>(B) + (size_t)min(n0 + row - TM, N - 1) * rowBytes) +
+                 k * 16;
+        dst[i] = sbase + row * RB + k * 16;
+    }
+    auto load = [&](int ch, int i) {
+        if (UNITS % T == 0 || (int)threadIdx.x + i * T < UNITS)
+            cp16(dst[i] + (ch % ST) * STAGE, src[i] + (size_t)ch * (U * 16));
     };
 
     float acc[L][2][4];
@@ -427,7 +435,9 @@ __global__ void __launch_bounds__(32 * WM * WN, 2) k_sep_gemm(const __grid_const
             for (int q = 0; q < 4; ++q) acc[d][t][q] = 0.f;
 
     for (int s = 0; s < ST - 1; ++s) {
-        if (s < nch) load(s);
+        if (s < nch)
+#pragma unroll
+            for (int i = 0; i < CNT; ++i) load(s, i);
         asm volatile("cp.async.commit_group;");
     }
     const unsigned offA = (wm * 16 + (lane & 15)) * RB + (lane >> 4) * 16;
@@ -435,25 +445,29 @@ __global__ void __launch_bounds__(32 * WM * WN, 2) k_sep_gemm(const __grid_const
     for (int ch = 0; ch < nch; ++ch) {
         asm volatile("cp.async.wait_group %0;" ::"n"(ST - 2));
         __syncthreads();
-        if (ch + ST - 1 < nch) load(ch + ST - 1);
-        asm volatile("cp.async.commit_group;");
         const unsigned s = sbase + (ch % ST) * STAGE;
+        unsigned a[L][4], b[2][4];
 #pragma unroll
-        for (int ks = 0; ks < 2; ++ks) {
-            unsigned a[L][4];
+        for (int i = 0; i < L; ++i) ldsm4(a[i], s + offA + i * 64);
+        ldsm4(b[0], s + offB);
+        // 2 L steps: the mma of one digit of B, 16 terms.  The next step's fragment of B, the
+        // next 16 terms' fragment of A that this step was the last to need, and the step's share
+        // of the copies to a later stage are issued among them.
 #pragma unroll
-            for (int i = 0; i < L; ++i) ldsm4(a[i], s + offA + i * 64 + ks * 32);
+        for (int st = 0; st < 2 * L; ++st) {
+            const int ks = st / L, j = st % L;
+            if (st + 1 < 2 * L) ldsm4(b[(st + 1) & 1], s + offB + (st + 1) % L * 64 + (st + 1) / L * 32);
 #pragma unroll
-            for (int j = 0; j < L; ++j) {
-                unsigned b[4];
-                ldsm4(b, s + offB + j * 64 + ks * 32);
-#pragma unroll
-                for (int i = 0; i < L - j; ++i) {
-                    mma_bf16(acc[i + j][0], a[i], b[0], b[1]);
-                    mma_bf16(acc[i + j][1], a[i], b[2], b[3]);
-                }
+            for (int i = L - j - 1; i >= 0; --i) {
+                mma_bf16(acc[i + j][0], a[i], b[st & 1][0], b[st & 1][1]);
+                mma_bf16(acc[i + j][1], a[i], b[st & 1][2], b[st & 1][3]);
+                if (ks == 0 && i == L - j - 1) ldsm4(a[i], s + offA + i * 64 + 32);
             }
+            if (ch + ST - 1 < nch)
+#pragma unroll
+                for (int i = st * CNT / (2 * L); i < (st + 1) * CNT / (2 * L); ++i) load(ch + ST - 1, i);
         }
+        asm volatile("cp.async.commit_group;");
         if ((ch % kFlush) == kFlush - 1 || ch == nch - 1) {
             // whole numbers below 2^24: into units of 2^-36 of the leading digits' product
 #pragma unroll
