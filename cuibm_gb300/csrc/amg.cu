@@ -26,7 +26,6 @@
 
 namespace cuibm {
 
-constexpr int kCoarse = 1500;  // dense solve below this size (about 2M FMAs per cycle)
 
 struct HostCsr {
     int n = 0, m = 0;  // rows, cols

@@ -1661,7 +1661,10 @@ static bool separable_applies(const Context &c, const LinearSystem &S)
     const bool level = c.P.solverType == ST_NAVIERSTOKES || c.P.solverType == ST_FADLUN ||
                        (c.g.nP < kLevelMax && c.P.solverPack != 2 &&
                         c.P.poisson.precision == PRECISION_FP64);
-    return level && (S.which == 2 || predicted_velocity_steps(c, S.rtol) >= velocity_steps(S));
+    // a pressure system of one level is solved by its dense inverse in one launch: 10 to 20 us less
+    // than this chain up to 1444 unknowns, bodies 10 to 490 us (a moving one's rows are exact there);
+    // at 1600, with two levels, the step takes 103 us here against 133 (1e-5) to 537 (1e-12)
+    return level && (S.which == 2 ? c.g.nP > kCoarse : predicted_velocity_steps(c, S.rtol) >= velocity_steps(S));
 }
 
 // One grid's operator: shift + X + Y with the coefficients towards the next and the

@@ -28,6 +28,7 @@ struct InputError {
 };
 
 constexpr int kBlock = 256;
+constexpr int kCoarse = 1500;  // dense solve below this size (about 2M FMAs per cycle)
 constexpr int kTraceLen = 4096;  // timestamps kept per persistent solve (diagnostic trace)
 inline int blocks_for(long n, int bs = kBlock) { return (int)((n + bs - 1) / bs); }
 

@@ -34,7 +34,7 @@ def box(folder, nx, ny, ratio, krylov, precision, tol=TOL, nu=0.01):
     return cases.write_case(folder, [sim], flow, [axis("x", nx), axis("y", ny)], [])
 
 
-def solver(folder, args=()):
+def solver(folder, args=("-separable", "1")):
     s = cb.NavierStokesSolver(folder, args)
     s.set_option("write_output", 0)
     s.initialise()
@@ -145,3 +145,15 @@ def test_body_methods_agree_with_smoothed_aggregation(tmp_path, method, precisio
     assert np.linalg.norm(u - us) <= 1e-9 * np.linalg.norm(us)
     assert np.linalg.norm(p - ps) <= 1e-8 * np.linalg.norm(ps)
     assert np.max(np.abs(fo - fs)) <= 1e-9 * max(1.0, np.max(np.abs(fs)))
+
+
+@pytest.mark.parametrize("nx,ny,separable", [(30, 50, False), (38, 39, False), (19, 79, True), (39, 39, True)])
+def test_one_level_systems_keep_their_dense_inverse(tmp_path, nx, ny, separable):
+    """Up to 1500 pressure unknowns the default is the one-level hierarchy: the bits of -separable 0."""
+    out = []
+    for args in ((), ("-separable", "0")):
+        with solver(box(str(tmp_path / ("c%d" % len(out))), nx, ny, 1.0, "BICGSTAB", None), args) as s:
+            s.set("rhs2", np.random.default_rng(5).standard_normal(s.info.numP))
+            s.run("solve_poisson")
+            out.append(s.get("p"))
+    assert np.array_equal(*out) == (not separable)
