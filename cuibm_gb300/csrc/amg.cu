@@ -273,6 +273,7 @@ static T *sa_alloc(Context &c, LinearSystem &S, size_t n)
 // goes with the context)
 void free_sa_hierarchy(LinearSystem &S)
 {
+    ++S.tables;
     for (SaLevel *L : S.amg) delete L;
     S.amg.clear();
     for (void *p : S.sa_blocks) cudaFree(p);
@@ -300,6 +301,7 @@ static void build_structured_hierarchy(Context &c, LinearSystem &S);
 
 void build_sa_hierarchy(Context &c, LinearSystem &S)
 {
+    ++S.tables;
     S.sa_structured = structured_applies(c, S);
     if (S.sa_structured) {
         build_structured_hierarchy(c, S);

@@ -584,12 +584,14 @@ void free_transposed_graph(LinearSystem &S)
 // The whole solve as one graph - the residual and a WHILE node of iterations - so that a
 // solve is one launch and one wait.  With a launch per kernel and a look at the status every
 // four iterations, the reduced adjoint (59 x 59) spent more than half its time on the host.
+// The nodes hold the preconditioner's device pointers, so the graph goes with the forward
+// system's tables (their count; a rebuilt hierarchy's objects may have the freed ones' addresses).
 template <class Op>
 static void transposed_solve(Context &c, LinearSystem &S, Op A, const TransposeList &T, const double *b, double *x)
 {
     const int n = S.n, nb = blocks_for(n);
-    const void *key[6] = {b, x, T.cnt, T.ent, S.sep, S.amg.empty() ? nullptr : S.amg[0]};
-    if (!S.t_exec || !std::equal(key, key + 6, S.t_key)) {
+    const void *key[4] = {b, x, T.cnt, T.ent};
+    if (!S.t_exec || S.t_tables != S.tables || !std::equal(key, key + 4, S.t_key)) {
         free_transposed_graph(S);
         CUIBM_TRY(cudaStreamBeginCapture(c.stream, cudaStreamCaptureModeRelaxed));
         try {
@@ -606,7 +608,8 @@ static void transposed_solve(Context &c, LinearSystem &S, Op A, const TransposeL
         }
         CUIBM_TRY(cudaStreamEndCapture(c.stream, &S.t_graph));
         CUIBM_TRY(cudaGraphInstantiate(&S.t_exec, S.t_graph, 0));
-        std::copy(key, key + 6, S.t_key);
+        std::copy(key, key + 4, S.t_key);
+        S.t_tables = S.tables;
     }
     CUIBM_TRY(cudaGraphLaunch(S.t_exec, c.stream));
 }
@@ -620,6 +623,7 @@ int launch_solve_transposed(Context &c, LinearSystem &S, LinearSystem &F, const 
 {
     S.amg = F.amg;  // the forward hierarchy (rebuilt for a moving body between steps)
     S.sep = F.sep;  // so its preconditioner
+    S.tables = F.tables;
     if (S.precond == PC_SMOOTHED_AGGREGATION && !S.sep) ensure_transposed_levels(c, F);
     // (both values are read before the calls return)
     CUIBM_TRY(cudaMemcpyAsync(&S.ks->rtol, &S.rtol, sizeof(double), cudaMemcpyHostToDevice, c.stream));

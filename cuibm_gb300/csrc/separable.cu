@@ -1889,6 +1889,7 @@ void setup_separable(Context &c, LinearSystem &S)
 
 static void build_separable(Context &c, LinearSystem &S)
 {
+    ++S.tables;
     S.sep = nullptr;
     if (!separable_applies(c, S) || !S.diag) return;  // (the stored diagonal comes with the persistent solver)
     const int nx = c.g.nx, ny = c.g.ny;
@@ -1981,6 +1982,7 @@ void free_separable(LinearSystem &S)
         if (b) cudaFree(b);
     delete P;
     S.sep = nullptr;
+    ++S.tables;
 }
 
 // ---- host side: solves --------------------------------------------------------------------

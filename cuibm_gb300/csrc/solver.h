@@ -164,11 +164,16 @@ struct LinearSystem {
     double *aedef = nullptr;                // A e (the operator's row sums), with wdef
     double *ym = nullptr, *wdef = nullptr;  // constant-mode correction of the SA cycle (Poisson):
     double Edef = 0;                        // cycle output, A^T e, e^T A e
+    // counts what builds and frees the preconditioner's device tables (the hierarchy, the
+    // separable plan): a captured solve that holds their pointers is good for one value of it
+    unsigned long long tables = 0;
     // a transposed system's whole solve as a graph (its right-hand side, solution and lists
-    // are the adjoint's own arrays): launched per solve, rebuilt when one of them changes
+    // are the adjoint's own arrays): launched per solve, rebuilt when one of them or the
+    // forward system's tables change
     cudaGraphExec_t t_exec = nullptr;
     cudaGraph_t t_graph = nullptr;
-    const void *t_key[6] = {};
+    const void *t_key[4] = {};
+    unsigned long long t_tables = 0;
     FusedSyncState *fsync = nullptr;
     void *fargs = nullptr;  // device copy of the solver arguments
 };
