@@ -1153,17 +1153,45 @@ __global__ void __launch_bounds__(128) k_row_cg(const __grid_constant__ SepArgs 
 
 // A last correction x += M r for the residual that the solve ends with (a moving body's
 // solves): where the iteration stops, the level of the pressure - fixed by one pinned cell -
-// carries up to 2e-9 of it at a relative residual of 1e-12; M resolves it exactly
+// carries up to 2e-9 of it at a relative residual of 1e-12; M resolves it exactly.  With the
+// body's rows M is no more than near the inverse, and r - A M r can be the larger residual:
+// the whole update is taken where that meets the solve's tolerance, else the length of it that
+// leaves the least residual, which is never above the one that the solve ended with.
 __global__ void k_sep_pick(int n, const double *__restrict__ r, const double *__restrict__ s, double *out,
                            const KrylovScalars *ks)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) out[i] = ks->s_done ? s[i] : r[i];
 }
+template <class Op>
+__global__ void __launch_bounds__(256) k_sep_accept(Op A, int n, const double *__restrict__ r,
+                                                    const double *__restrict__ z, double *partials, KrylovScalars *ks)
+{
+    if (ks->status != KS_CONVERGED) return;
+    double v[3] = {0, 0, 0};
+    SEP_ROWS(i, n)
+    {
+        const double ri = r[i], ai = A.row(i, PtrAccess{z}), left = ri - ai;
+        v[0] += left * left;
+        v[1] += ri * ai;
+        v[2] += ai * ai;
+    }
+    if (row_sums<3>(v, partials, &ks->arrive)) {
+        const double left = sqrt(v[0]);
+        if (left <= ks->tol) {
+            ks->alpha = 1;
+            ks->rnorm = left;
+        } else {
+            const double a = v[1] / v[2], rr = ks->rnorm * ks->rnorm;
+            ks->alpha = isfinite(a) ? a : 0.0;
+            ks->rnorm = sqrt(fmax(0.0, rr - ks->alpha * v[1]));
+        }
+    }
+}
 __global__ void k_sep_correct(int n, const double *__restrict__ z, double *x, const KrylovScalars *ks)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n && ks->status == KS_CONVERGED) x[i] += z[i];
+    if (i < n && ks->status == KS_CONVERGED) x[i] += ks->alpha * z[i];
 }
 
 // CG's first iteration: p = z, q = A z, rho = r . z, alpha = rho / (z . q)
@@ -2129,6 +2157,7 @@ struct SepSolve {
         const int nb = blocks_for(S.n);
         k_sep_pick<<<nb, kBlock, 0, c.stream>>>(S.n, S.r, S.s, S.p, S.ks);
         launch_separable_apply(c, S, S.p, S.Mp);
+        with_op([&](auto A) { k_sep_accept<<<this->nb(), kBlock, 0, c.stream>>>(A, S.n, S.p, S.Mp, S.partials, S.ks); });
         k_sep_correct<<<nb, kBlock, 0, c.stream>>>(S.n, S.Mp, x, S.ks);
         CUIBM_TRY(cudaGetLastError());
     }
