@@ -46,9 +46,10 @@ struct TagRecords {
     double *distA, *distB;
     int nrec;
     // the body segments that cross each row and each column of the box, in order
-    int *cross_count, *cross;  // [line], [line][total]: rows first, then columns
-    double *cross_at, *cross_uv;  // where each crosses, and the body velocity there
-    int lines;
+    int *cross_count, *cross_first, *cross;  // [line] (rows, then columns), [line]: its first in cross
+    double *cross_at, *cross_uv;             // where each crosses, and the body velocity there
+    unsigned long long *cross_used;          // places of cross taken, one count a list
+    int lines, cross_cap;
 };
 
 struct TagGeom {
@@ -66,72 +67,114 @@ struct TagGeom {
 // are those of the reference's node loops, as are the point where a segment crosses and the body
 // velocity there (FP64 divisions: about a microsecond of dependent instructions each); every
 // node of a line shares them, so a node visits the few segments of its row and column
-// instead of all of them.
-__global__ void k_tag_lines(TagGeom G, TagRecords R, int rows)
+// instead of all of them.  The lines' lists share one array, each a range of it as long as its
+// crossings (counted first); a list that finds no room there (the array holds what the body's
+// shape at set-up can cross, cross_capacity, and its points may be written anew) gets the
+// count -1, and its nodes look through all segments.
+__device__ __forceinline__ int segment_start(const TagGeom &G, int l) { return l > 0 ? l - 1 : G.total - 1; }
+__device__ __forceinline__ bool segment_crosses(const double *b, int k, int l, double c)
+{
+    const double lo = b[k] > b[l] ? b[l] : b[k], hi = b[k] > b[l] ? b[k] : b[l];
+    return lo - IB_EPS < c && hi - IB_EPS > c;
+}
+// where segment k, l crosses b = c, and the body velocity there (b: the coordinate across the
+// line, o: along it); nothing for a segment along the line
+__device__ __forceinline__ void segment_values(const double *b, const double *o, const double *vel, int k, int l,
+                                               double c, double &at, double &uv)
+{
+    if (fabs(b[l] - b[k]) > IB_EPS) {
+        at = o[k] + (o[l] - o[k]) * (c - b[k]) / (b[l] - b[k]);
+        uv = vel[k] + (vel[l] - vel[k]) * (c - b[k]) / (b[l] - b[k]);
+    }
+}
+
+__global__ void k_tag_lines(TagGeom G, TagRecords R, int rows, int list)
 {
     const int line = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (line >= rows + G.width) return;
     const bool row = line < rows;
     const int at = row ? G.j0 + line : G.i0 + line - rows;
+    const double *b = row ? G.by : G.bx, *o = row ? G.bx : G.by;
+    const bool inside = at < (row ? G.nyc : G.nxc);
+    const double c = inside ? (row ? G.yc[at] : G.xc[at]) : 0.0;
+    auto hits = [&](int l0) {
+        const int l = l0 + lane;
+        return __ballot_sync(0xffffffffu, l < G.total && segment_crosses(b, segment_start(G, l), l, c));
+    };
     int n = 0;
-    if (at < (row ? G.nyc : G.nxc)) {
-        const double c = row ? G.yc[at] : G.xc[at], *b = row ? G.by : G.bx, *o = row ? G.bx : G.by, *vel = G.vel;
-        const size_t first = (size_t)line * G.total;
-        for (int l0 = 0; l0 < G.total; l0 += 32) {
-            const int l = l0 + lane, k = l > 0 ? l - 1 : G.total - 1;
-            bool hit = false;
-            if (l < G.total) {
-                const double lo = b[k] > b[l] ? b[l] : b[k], hi = b[k] > b[l] ? b[k] : b[l];
-                hit = lo - IB_EPS < c && hi - IB_EPS > c;
-            }
-            const unsigned m = __ballot_sync(0xffffffffu, hit);
-            if (hit) {
-                const size_t e = first + n + __popc(m & ((1u << lane) - 1));
-                R.cross[e] = l;
-                if (fabs(b[l] - b[k]) > IB_EPS) {
-                    R.cross_at[e] = o[k] + (o[l] - o[k]) * (c - b[k]) / (b[l] - b[k]);
-                    R.cross_uv[e] = vel[k] + (vel[l] - vel[k]) * (c - b[k]) / (b[l] - b[k]);
-                }
-            }
-            n += __popc(m);
-        }
+    if (inside)
+        for (int l0 = 0; l0 < G.total; l0 += 32) n += __popc(hits(l0));
+    unsigned long long first = 0;
+    if (lane == 0 && n > 0) first = atomicAdd(R.cross_used + list, (unsigned long long)n);
+    first = __shfl_sync(0xffffffffu, first, 0);
+    if (first + n > (unsigned long long)R.cross_cap) n = -1;
+    if (lane == 0) {
+        R.cross_count[line] = n;
+        R.cross_first[line] = (int)first;
     }
-    if (lane == 0) R.cross_count[line] = n;
+    for (int l0 = 0, done = 0; done < n; l0 += 32) {
+        const unsigned m = hits(l0);
+        if (m >> lane & 1) {
+            const int e = (int)first + done + __popc(m & ((1u << lane) - 1)), l = l0 + lane;
+            R.cross[e] = l;
+            segment_values(b, o, G.vel, segment_start(G, l), l, c, R.cross_at[e], R.cross_uv[e]);
+        }
+        done += __popc(m);
+    }
 }
 
 // the crossings of a node's row and column, merged in increasing l
 struct Crossings {
+    const TagGeom &G;
     const TagRecords &R;
-    size_t row, col;
-    int nr, nc, l, k;
-    bool x, y;  // l crosses the row; the column
+    int row, col;           // the next places in the two lists
+    int nr, nc;             // crossings left there; -1: no list
+    int lr, lc;             // the next segment that crosses the row; the column
+    double cy, cx;          // the row's ordinate, the column's abscissa (without a list)
+    int l, k;
+    bool x, y;              // l crosses the row; the column
     double ax, ay, ux, uy;  // where, and the body velocity there
-    __device__ Crossings(const TagGeom &G, const TagRecords &R_, int idx) : R(R_)
+    __device__ Crossings(const TagGeom &G_, const TagRecords &R_, int idx) : G(G_), R(R_)
     {
         const int rows = (G.nthreads + G.width - 1) / G.width, j = idx / G.width, i = rows + idx % G.width;
-        row = (size_t)j * G.total;
-        col = (size_t)i * G.total;
         nr = R.cross_count[j];
         nc = R.cross_count[i];
+        row = R.cross_first[j];
+        col = R.cross_first[i];
+        cy = nr < 0 ? G.yc[G.j0 + j] : 0.0;
+        cx = nc < 0 ? G.xc[G.i0 + i - rows] : 0.0;
+        lr = segment(row, nr, 0, G.by, cy);
+        lc = segment(col, nc, 0, G.bx, cx);
     }
-    __device__ bool next(int total)
+    // the first segment from l0 on that crosses a line
+    __device__ int segment(int at, int left, int l0, const double *b, double c) const
     {
-        const int lr = nr > 0 ? R.cross[row] : total, lc = nc > 0 ? R.cross[col] : total;
+        if (left >= 0) return left > 0 ? R.cross[at] : G.total;
+        while (l0 < G.total && !segment_crosses(b, segment_start(G, l0), l0, c)) ++l0;
+        return l0;
+    }
+    // segment l's values on a line, and the line's next segment
+    __device__ void take(int &at, int &left, int &lnext, const double *b, const double *o, double c, double &a,
+                         double &u) const
+    {
+        if (left > 0) {
+            a = R.cross_at[at];
+            u = R.cross_uv[at];
+            ++at, --left;
+        } else {
+            segment_values(b, o, G.vel, k, l, c, a, u);
+        }
+        lnext = segment(at, left, l + 1, b, c);
+    }
+    __device__ bool next()
+    {
         l = min(lr, lc);
-        if (l == total) return false;
-        k = l > 0 ? l - 1 : total - 1;
+        if (l == G.total) return false;
+        k = segment_start(G, l);
         x = lr == l;
         y = lc == l;
-        if (x) {
-            ax = R.cross_at[row];
-            ux = R.cross_uv[row];
-            ++row, --nr;
-        }
-        if (y) {
-            ay = R.cross_at[col];
-            uy = R.cross_uv[col];
-            ++col, --nc;
-        }
+        if (x) take(row, nr, lr, G.by, G.bx, cy, ax, ux);
+        if (y) take(col, nc, lc, G.bx, G.by, cx, ay, uy);
         return true;
     }
 };
@@ -197,7 +240,7 @@ __global__ void k_tag_velocity_records(TagGeom G, TagRecords R)
     if (KIND == 0) flags_extra |= 1 << 17;  // dist_u_body[ip] = 0 at thread start
     double ix, iy;
     // (once flag is set the reference's remaining segments do nothing)
-    for (Crossings cr(G, R, idx); !flag && cr.next(G.total);) {
+    for (Crossings cr(G, R, idx); !flag && cr.next();) {
         const int k = cr.k, l = cr.l;
         if (cr.x) {
             if (fabs(by[l] - by[k]) > IB_EPS) {
@@ -367,7 +410,7 @@ __global__ void k_tag_pressure_records(TagGeom G, TagRecords R)
     const double midX = G.motion ? G.motion[0] : G.midX, midY = G.motion ? G.motion[1] : G.midY;
     bool flag = false;
     double x, y, ix, iy;
-    for (Crossings cr(G, R, idx); !flag && cr.next(G.total);) {
+    for (Crossings cr(G, R, idx); !flag && cr.next();) {
         const int k = cr.k, l = cr.l;
         if (cr.x) {
             if (fabs(by[l] - by[k]) > IB_EPS) {
@@ -1406,6 +1449,24 @@ static IbHost &hostside(Context &c) { return g_ib_host[c.ib_slot]; }
 
 IbPlan &ib_plan(Context &c) { return hostside(c).plan; }
 
+// The most crossings of grid lines and body segments while the body keeps its shape: an open
+// interval of length d holds at most d / h + 1 lines of spacing h and more.  About the
+// perimeter over the finest spacing and twice the points (a place for every line and segment
+// would be 500 MB at 5000 points in a box of 2500 x 2500), and never more than that product.
+static int cross_capacity(const Context &c, int lines)
+{
+    const BodyState &B = c.body;
+    const double hx = *std::min_element(c.gx.width.begin(), c.gx.width.end()),
+                 hy = *std::min_element(c.gy.width.begin(), c.gy.width.end());
+    double n = 0;
+    for (int l = 0; l < B.total; ++l) {
+        const int k = l > 0 ? l - 1 : B.total - 1;
+        n += std::floor(std::fabs(B.x[l] - B.x[k]) / hx * (1 + 1e-6)) + 1;
+        n += std::floor(std::fabs(B.y[l] - B.y[k]) / hy * (1 + 1e-6)) + 1;
+    }
+    return (int)std::min({n, (double)lines * B.total, 1e9}) + 1;
+}
+
 void setup_ib(Context &c)
 {
     IbArrays &b = c.ib;
@@ -1475,9 +1536,12 @@ void setup_ib(Context &c)
     H.rec.flags = c.carve<int>(nr);
     H.rec.lines = (int)((nr + w - 1) / w) + w;
     H.rec.cross_count = c.carve<int>(H.rec.lines);
-    H.rec.cross = c.carve<int>((size_t)H.rec.lines * c.body.total);
-    H.rec.cross_at = c.carve<double>((size_t)H.rec.lines * c.body.total);
-    H.rec.cross_uv = c.carve<double>((size_t)H.rec.lines * c.body.total);
+    H.rec.cross_first = c.carve<int>(H.rec.lines);
+    H.rec.cross_used = c.carve<unsigned long long>(3);
+    H.rec.cross_cap = cross_capacity(c, H.rec.lines);
+    H.rec.cross = c.carve<int>(H.rec.cross_cap);
+    H.rec.cross_at = c.carve<double>(H.rec.cross_cap);
+    H.rec.cross_uv = c.carve<double>(H.rec.cross_cap);
     H.rec.hyb = c.carve<int>(nr);
     H.rec.hyb2 = c.carve<int>(nr);
     H.rec.dnode = c.carve<double>(nr);
@@ -1592,12 +1656,13 @@ void launch_tag_points(Context &c)
     const int rows = (nthreads + w - 1) / w;
     const int nres = (w + 2) * (rows + 2);
     if (rows + w > H.rec.lines) throw InputError("the body's box outgrew the tagging records");
-    auto lines = [&] {
-        k_tag_lines<<<blocks_for(32L * (rows + w)), kBlock, 0, c.stream>>>(G, H.rec, rows);
+    CUIBM_TRY(cudaMemsetAsync(H.rec.cross_used, 0, 3 * sizeof(unsigned long long), c.stream));
+    auto lines = [&](int list) {
+        k_tag_lines<<<blocks_for(32L * (rows + w)), kBlock, 0, c.stream>>>(G, H.rec, rows, list);
     };
     G.nxc = nx - 1;
     G.nyc = ny;
-    lines();
+    lines(0);
     k_tag_velocity_records<0><<<blocks_for(nthreads), kBlock, 0, c.stream>>>(G, H.rec);
     k_tag_resolve<0><<<blocks_for(nres), kBlock, 0, c.stream>>>(G, H.rec, O);
     G.vel = b.vB;
@@ -1605,14 +1670,14 @@ void launch_tag_points(Context &c)
     G.yc = c.yv;
     G.nxc = nx;
     G.nyc = ny - 1;
-    lines();
+    lines(1);
     O.dist = b.distV;
     k_tag_velocity_records<1><<<blocks_for(nthreads), kBlock, 0, c.stream>>>(G, H.rec);
     k_tag_resolve<1><<<blocks_for(nres), kBlock, 0, c.stream>>>(G, H.rec, O);
     G.xc = c.xv;
     G.yc = c.yu;
     G.nyc = ny;
-    lines();
+    lines(2);
     TagOut OP{b.ghostP, b.hybridP, nullptr, nullptr, nullptr, nullptr, b.bipX, b.bipY, b.ippX, b.ippY, nullptr};
     k_tag_pressure_records<<<blocks_for(nthreads), kBlock, 0, c.stream>>>(G, H.rec);
     k_tag_resolve<2><<<blocks_for(nres), kBlock, 0, c.stream>>>(G, H.rec, OP);
