@@ -569,8 +569,10 @@ __global__ void k_tag_resolve(TagGeom G, TagRecords R, TagOut O)
 // zero_pressure_luo / zero_x_luo / zero_y_luo: a row left to right, a warp a row (blockIdx.y:
 // which of the three arrays).  The warp loads the row and finds the last tagged node up to
 // scan_end (the place the reference's inner loop looks for: nodes right of i still hold their
-// tags when the walk is at i); one lane walks the row in shared memory.  A thread a row with
-// the tags in memory took 410 us an array on the 500-node rows of the KC 10 box.
+// tags when the walk is at i); one lane walks the row in shared memory, or in memory where the
+// box is wider than kZeroPlaces.  A thread a row with the tags in memory took 410 us an array
+// on the 500-node rows of the KC 10 box.
+constexpr int kZeroPlaces = 48 * 1024 / sizeof(int);  // a launch's dynamic shared memory without asking for more
 struct ZeroRows {
     int *tags[3];
     int stride[3], scan_end[3];
@@ -578,15 +580,17 @@ struct ZeroRows {
 };
 __global__ void __launch_bounds__(32) k_zero_rows(ZeroRows Z)
 {
-    extern __shared__ int t[];  // the row from i0 - 1 to i1 - 1
+    extern __shared__ int places[];
     const int a = blockIdx.y, j = blockIdx.x, lane = threadIdx.x, J = Z.j0 + j;
     if (j >= Z.rows || J > Z.j1) return;
     int *row = Z.tags[a] + (size_t)J * Z.stride[a];
     const int end = Z.scan_end[a], n = Z.i1 - Z.i0;
+    const bool wide = n + 1 > kZeroPlaces;
+    int *t = wide ? row + Z.i0 - 1 : places;  // the row from i0 - 1 to i1 - 1
     int last = -1;
     for (int i = Z.i0 - 1 + lane; i <= max(end, Z.i1 - 1); i += 32) {
         const int v = row[i];
-        if (i < Z.i1) t[i - Z.i0 + 1] = v;
+        if (!wide && i < Z.i1) t[i - Z.i0 + 1] = v;
         if (i <= end && v != -1) last = i;
     }
     for (int o = 16; o > 0; o >>= 1) last = max(last, __shfl_xor_sync(0xffffffffu, last, o));
@@ -613,6 +617,7 @@ __global__ void __launch_bounds__(32) k_zero_rows(ZeroRows Z)
         }
     }
     __syncwarp();
+    if (wide) return;
     for (int q = 1 + lane; q <= n; q += 32) row[Z.i0 + q - 1] = t[q];
 }
 
@@ -1685,7 +1690,9 @@ void launch_tag_points(Context &c)
     const int zrows = ref_threads(i1 - i0, 1);
     const ZeroRows Z{{b.ghostP, b.ghostUV, b.ghostUV + c.g.nU}, {nx, nx - 1, nx}, {nx, nx - 1, nx - 1},
                      i0, i1, j0, j1, zrows};
-    k_zero_rows<<<dim3(std::min(zrows, j1 - j0 + 1), 3), 32, (size_t)(w + 1) * sizeof(int), c.stream>>>(Z);
+    const size_t zplaces = w + 1 <= kZeroPlaces ? (w + 1) * sizeof(int) : 0;
+    k_zero_rows<<<dim3(std::min(zrows, j1 - j0 + 1), 3), 32, zplaces, c.stream>>>(Z);
+    CUIBM_TRY(cudaGetLastError());
     // the interpolation plan of these tags
     IbPlan &P = H.plan;
     BoxLaunch B = box(c);

@@ -60,3 +60,31 @@ def test_points_written_anew(tmp_path, points, reach):
         s.set("body_y", y)
         s.run("tag_points")
         check(s, mid)
+
+
+@pytest.mark.parametrize("columns,wide", [(12000, False), (12600, True)])
+def test_boxes_wider_than_shared_memory_holds(tmp_path, columns, wide):
+    """A thin body across a box of about `columns` columns (rows of up to 12287 nodes are walked in
+    shared memory, longer ones in place)."""
+    h = 1.0 / 64
+    a = columns * h / 4  # the box is twice the body
+    t = np.arange(256) * 2 * np.pi / 256
+    dirs = tmp_path / "c" / "bodyFiles"
+    dirs.mkdir(parents=True)
+    (dirs / "thin").write_text("256\n" + "\n".join("%r %r" % (float(a * np.cos(v)), float(0.1 * np.sin(v)))
+                                                  for v in t) + "\n")
+    sim = {"type": "simulation", "dt": 0.001, "nt": 5, "nsave": 5, "SolverType": "LUO",
+           "linearSolvers": cases.solvers("DIAGONAL", 1e-5, "DIAGONAL", 1e-5, vel_krylov="BICGSTAB",
+                                          pois_krylov="BICGSTAB")}
+    flow = [{"type": "flow", "nu": 0.01, "initialVelocity": [1.0, 0.0],
+             "boundaryConditions": cases.bcs((1, 0), (1, 0), (1, 0), (1, 0), xp_type="CONVECTIVE")}]
+    half = 2 * a + 20 * h
+    f = cases.write_case(str(tmp_path / "c"), [sim], flow,
+                         [cases.axis("x", -half, h, [(half, 1.0)]), cases.axis("y", -0.5, h, [(0.5, 1.0)])],
+                         [{"type": "points", "pointsFile": "thin"}])
+    with cb.NavierStokesSolver(f) as s:
+        s.set_option("write_output", 0)
+        s.initialise()
+        assert (s.info.bb_ncx + 1 > 12288) == wide
+        T = check(s, sum(float(v) for v in s.get("body_y")) / 256)
+        assert (T.ghostTagsP > 0).sum() > 1000 and (T.ghostTagsP == 0).sum() > 1000
