@@ -934,9 +934,11 @@ int cuibm_set_option(cuibm_ctx *h, const char *key, double value)
         const int nb = (int)value;
         if (nb != value || nb < 0) return fail(h, CUIBM_ERR_BAD_INPUT, "solver_blocks must be a count >= 0");
         c.P.solverBlocks = nb;
-        set_fused_grid(c.sys1, nb);
-        set_fused_grid(c.sys2, nb);
-        if (c.initialised && c.use_graph) CUIBM_GUARD(h, { build_step_graph(c); });
+        CUIBM_GUARD(h, {
+            set_fused_grid(c.sys1, nb);
+            set_fused_grid(c.sys2, nb);
+            if (c.initialised && c.use_graph) build_step_graph(c);
+        });
     } else if (k == "force_method") {
         const int m = (int)value;
         if (m < 0 || m > 2 || m != value) return fail(h, CUIBM_ERR_BAD_INPUT, "force_method must be 0, 1 or 2");

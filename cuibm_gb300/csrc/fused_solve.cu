@@ -451,11 +451,16 @@ void set_fused_grid(LinearSystem &S, int blocks)
     if (!S.fused_fn) return;
     S.fused_grid = blocks > 0 ? std::min(S.fused_grid_max, blocks) : S.fused_grid_default;
     // the coarsest inverse's rows in shared memory (dense_solve) where a block's share fits
-    // beside the static arrays; batched solves share their SMs and keep none
+    // beside the static arrays, and all of the grid's blocks with it on the SMs at once (a grid
+    // of more blocks than SMs has several to an SM); batched solves share their SMs and keep none
     S.fused_smem = 0;
     if (S.precond == PC_SMOOTHED_AGGREGATION && S.fused_smem_max > 0) {
         const size_t n = sa_coarsest_size(S), rows = (n + S.fused_grid - 1) / S.fused_grid;
-        if (rows * n * sizeof(double) <= S.fused_smem_max) S.fused_smem = (int)(rows * n * sizeof(double));
+        const size_t bytes = rows * n * sizeof(double);
+        int per_sm = 0;
+        if (bytes <= (size_t)S.fused_smem_max)
+            CUIBM_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, S.fused_fn, S.fused_threads, bytes));
+        if (S.fused_grid <= per_sm * S.fused_sms) S.fused_smem = (int)bytes;
     }
 }
 
@@ -483,6 +488,7 @@ void setup_fused(Context &c, LinearSystem &S)
     if (const char *e = getenv("CUIBM_FUSED_BLOCKS_PER_SM")) want = std::max(1, atoi(e));
     S.fused_grid_default = sms * std::min(per_sm, want);
     S.fused_grid_max = sms * per_sm;
+    S.fused_sms = sms;
     S.fused_fn = fn;
     S.fused_smem_max = 0;
     if (S.precond == PC_SMOOTHED_AGGREGATION && c.P.solverPack != 2 && want == 1) {

@@ -141,7 +141,7 @@ struct LinearSystem {
     int body_kernels = 0;  // kernel nodes in one captured iteration body
     // persistent solver (fused_solve.cu); fused_fn is null where it does not apply
     void *fused_fn = nullptr;
-    int fused_grid = 0, fused_threads = 512;
+    int fused_grid = 0, fused_threads = 512, fused_sms = 0;
     int fused_smem = 0, fused_smem_max = 0;  // dynamic shared memory of the solve (the coarsest inverse)
     int fused_grid_default = 0, fused_grid_max = 0;  // one block per SM; every block the SMs hold
     double *p2 = nullptr, *AMp2 = nullptr, *fpartials = nullptr;
