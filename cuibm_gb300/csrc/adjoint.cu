@@ -724,7 +724,7 @@ void ensure_state(Context &c, int nsteps, int snapshots)
         A.tent2 = static_cast<int *>(dalloc(A, P * kTransposeMax * sizeof(int)));
         A.prow2 = static_cast<int *>(dalloc(A, 2 * (size_t)c.emb.cap2 * sizeof(int) + 4));
         A.overflow = static_cast<int *>(dalloc(A, sizeof(int)));
-        CUIBM_TRY(cudaMemset(A.overflow, 0, sizeof(int)));
+        CUIBM_TRY(cudaMemsetAsync(A.overflow, 0, sizeof(int), c.stream));
         for (double *&st : A.stash) st = static_cast<double *>(dalloc(A, (UV + P) * sizeof(double)));
         A.S1T.rtol = A.S2T.rtol = 1e-10;
         A.S1T.maxit = c.sys1.maxit;

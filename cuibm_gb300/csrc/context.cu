@@ -33,8 +33,9 @@ static void alloc_fields(Context &c)
     if (c.has_body) est += (nUV + nP) * 400;
     CUIBM_TRY(cudaMalloc(&c.arena, est));
     c.arena_bytes = est;
-    // device arrays start at zero, as the reference's value-initialised cusp arrays do
-    CUIBM_TRY(cudaMemset(c.arena, 0, est));
+    // device arrays start at zero, as the reference's value-initialised cusp arrays do.  On the
+    // context's stream, as every copy of the set-up: nothing orders the default stream before
+    // it, and with other contexts' work there a clear could come after the uploads below.
     c.arena_used = 0;
     CUIBM_TRY(cudaMemsetAsync(c.arena, 0, est, c.stream));
     c.u = c.carve<double>(nUV);
@@ -52,7 +53,6 @@ static void alloc_fields(Context &c)
     c.work_x = c.carve<double>(nUV > nP ? nUV : nP);
     c.work_y = c.carve<double>(nUV > nP ? nUV : nP);
     c.solve_trace = c.carve<unsigned long long>(2 * kTraceLen);
-    CUIBM_TRY(cudaMemset(c.solve_trace, 0, 2 * kTraceLen * sizeof(unsigned long long)));
     c.bc[XMINUS] = c.carve<double>(2 * ny - 1);
     c.bc[XPLUS] = c.carve<double>(2 * ny - 1);
     c.bc[YMINUS] = c.carve<double>(2 * nx - 1);

@@ -171,11 +171,14 @@ void setup_fadlun(Context &c)
         int *pcol = c.carve<int>(5 * np);
         double *pval = c.carve<double>(5 * np);
         double *pdiag = c.carve<double>(np);
-        CUIBM_TRY(cudaMemcpy(pid, B.pid.data(), n * sizeof(int), cudaMemcpyHostToDevice));
+        auto up = [&](void *dst, const auto &h) {
+            CUIBM_TRY(cudaMemcpyAsync(dst, h.data(), h.size() * sizeof(h[0]), cudaMemcpyHostToDevice, c.stream));
+        };
+        up(pid, B.pid);
         if (!B.pdiag.empty()) {
-            CUIBM_TRY(cudaMemcpy(pcol, B.pcol.data(), B.pcol.size() * sizeof(int), cudaMemcpyHostToDevice));
-            CUIBM_TRY(cudaMemcpy(pval, B.pval.data(), B.pval.size() * sizeof(double), cudaMemcpyHostToDevice));
-            CUIBM_TRY(cudaMemcpy(pdiag, B.pdiag.data(), B.pdiag.size() * sizeof(double), cudaMemcpyHostToDevice));
+            up(pcol, B.pcol);
+            up(pval, B.pval);
+            up(pdiag, B.pdiag);
         }
         R = RowPatch{pid, pcol, pval, pdiag};
         hid = B.pid;

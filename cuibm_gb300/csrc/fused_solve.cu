@@ -209,13 +209,15 @@ static void upload_fargs(Context &c, LinearSystem &S)
     if (m) {
         // the float solver shares the reduction buffers, the barrier and the trace
         FArgs<float> fa = {};
-        CUIBM_TRY(cudaMemcpy(&fa, m->dev, sizeof(fa), cudaMemcpyDeviceToHost));
+        CUIBM_TRY(cudaMemcpyAsync(&fa, m->dev, sizeof(fa), cudaMemcpyDeviceToHost, c.stream));
+        CUIBM_TRY(cudaStreamSynchronize(c.stream));
         fa.partials = S.fpartials;
         fa.sync = S.fsync;
         fa.trace = a.trace;
         fa.ks = S.ks;
         fa.err = c.err_word;
-        CUIBM_TRY(cudaMemcpy(m->dev, &fa, sizeof(fa), cudaMemcpyHostToDevice));
+        CUIBM_TRY(cudaMemcpyAsync(m->dev, &fa, sizeof(fa), cudaMemcpyHostToDevice, c.stream));
+        CUIBM_TRY(cudaStreamSynchronize(c.stream));
     }
 }
 

@@ -1600,7 +1600,9 @@ void setup_ib(Context &c)
         tab[2 * s + 1] = B.uCoeff * std::cos(2 * M_PI * B.freq * t + B.uPhase);
     }
     H.motion_table = c.carve<double>(tab.size());
-    CUIBM_TRY(cudaMemcpy(H.motion_table, tab.data(), tab.size() * sizeof(double), cudaMemcpyHostToDevice));
+    CUIBM_TRY(cudaMemcpyAsync(H.motion_table, tab.data(), tab.size() * sizeof(double), cudaMemcpyHostToDevice,
+                              c.stream));
+    CUIBM_TRY(cudaStreamSynchronize(c.stream));
 }
 
 static BoxLaunch box(Context &c)

@@ -252,7 +252,8 @@ void setup_system(Context &c, LinearSystem &S)
         hk.inner_rtol = 1e-3;
         hk.inner_maxit = 100;
         hk.status = KS_CONVERGED;
-        CUIBM_TRY(cudaMemcpy(S.ks, &hk, sizeof(hk), cudaMemcpyHostToDevice));
+        CUIBM_TRY(cudaMemcpyAsync(S.ks, &hk, sizeof(hk), cudaMemcpyHostToDevice, c.stream));
+        CUIBM_TRY(cudaStreamSynchronize(c.stream));
     }
     S.w = nullptr;
     if (S.krylov == KRYLOV_CG) {
@@ -538,7 +539,8 @@ void setup_transposed_system(Context &c, const LinearSystem &F, LinearSystem &S,
     hk.rtol = S.rtol;
     hk.maxit = S.maxit;
     hk.status = KS_CONVERGED;
-    CUIBM_TRY(cudaMemcpy(S.ks, &hk, sizeof(hk), cudaMemcpyHostToDevice));
+    CUIBM_TRY(cudaMemcpyAsync(S.ks, &hk, sizeof(hk), cudaMemcpyHostToDevice, c.stream));
+    CUIBM_TRY(cudaStreamSynchronize(c.stream));
     S.amg = F.amg;
 }
 
