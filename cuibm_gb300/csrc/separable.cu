@@ -1309,7 +1309,9 @@ static void allow_smem(K *fn, size_t bytes)
                                    (int)bytes));
 }
 
-// once per context (set-up): dynamic shared memory above 48 KB
+// once per context (set-up): dynamic shared memory above 48 KB.  The attribute is the process's,
+// so every context sets the same value, the most that any case asks for: another thread's
+// context, of another size, may set it between this one's call and launch.
 template <int L>
 static void allow_gemm()
 {
@@ -1806,7 +1808,7 @@ static bool build_grid(Context &c, SepPlan &P, int g, const SepGrid &G, bool sym
     put(D(ocrt), crt);
     put(D(owr), G.wr);
     const size_t smem = (size_t)nm * kRotWarps * 8;
-    allow_smem(k_sep_rotate, smem);
+    allow_smem(k_sep_rotate, (size_t)kSepMax * kRotWarps * 8);
     k_sep_rotate<<<(nm + kRotWarps - 1) / kRotWarps, 32 * kRotWarps, smem, c.stream>>>(nm, sw, (int)sweeps.size(), rt, Q);
     if (d.pins) k_sep_constant<<<blocks_for(nm), kBlock, 0, c.stream>>>(nm, k0, vcon, Q);
     CUIBM_TRY(cudaGetLastError());
