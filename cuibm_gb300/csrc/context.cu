@@ -1211,6 +1211,7 @@ void cuibm_destroy(cuibm_ctx *h)
     free_separable(c.sys1);
     free_separable(c.sys2);
     free_adjoint(c);
+    free_ib(c);
     if (c.arena) cudaFree(c.arena);
     if (c.h_scalars) cudaFreeHost(c.h_scalars);
     if (c.ev0) cudaEventDestroy(c.ev0);

@@ -1448,9 +1448,12 @@ struct IbHost {
     bool moving = false;
     IbPlan plan{};
 };
-static std::vector<IbHost> g_ib_host;  // one per context (indexed by Context::ib_slot)
-
-static IbHost &hostside(Context &c) { return g_ib_host[c.ib_slot]; }
+static IbHost &hostside(Context &c) { return *static_cast<IbHost *>(c.ib_host); }
+void free_ib(Context &c)
+{
+    delete static_cast<IbHost *>(c.ib_host);
+    c.ib_host = nullptr;
+}
 
 IbPlan &ib_plan(Context &c) { return hostside(c).plan; }
 
@@ -1525,12 +1528,9 @@ void setup_ib(Context &c)
     const int fblocks = 64;
     b.forcePart = c.carve<double>(6 * fblocks);
 
-    if ((int)g_ib_host.size() <= c.ib_slot || c.ib_slot < 0) {
-        c.ib_slot = (int)g_ib_host.size();
-        g_ib_host.emplace_back();
-    }
+    free_ib(c);
+    c.ib_host = new IbHost();
     IbHost &H = hostside(c);
-    H = IbHost();
     H.bb = c.carve<int>(4);
     H.force_arrive = c.carve<unsigned int>(4);
     CUIBM_TRY(cudaMemsetAsync(H.force_arrive, 0, 4 * sizeof(unsigned int), c.stream));

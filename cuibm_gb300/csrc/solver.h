@@ -240,7 +240,7 @@ struct Context {
     IbArrays ib{};
     bool has_body = false;
     bool ib_dirty = false;
-    int ib_slot = -1;                   // host-side IB bookkeeping of this context
+    void *ib_host = nullptr;            // host-side bookkeeping of the body (ib_kernels.cu)
     double ib_midX = 0, ib_midY = 0;    // body centre used by the tagging
     int force_method = 0;  // the step's force: 0 control volume, 1/2 surface integral (mode)
     // moving body with the embedded method and an SA preconditioner: the hierarchy is
@@ -383,6 +383,7 @@ int sa_coarsest_size(const LinearSystem &S);
 
 // ib_kernels.cu
 void setup_ib(Context &c);
+void free_ib(Context &c);
 void launch_tag_points(Context &c);
 void launch_ghost_velocity(Context &c, double *field, bool set);
 void launch_hybrid_velocity(Context &c, const double *field);

@@ -48,3 +48,35 @@ def test_set_ups_side_by_side(tmp_path):
     for t in threads:
         t.join()
     assert not failures, failures
+
+
+def test_bodies_side_by_side(tmp_path):
+    """Contexts with bodies come and go in several threads; each keeps its own body's lists."""
+    def cylinder(k):
+        return cases.cylinder(str(tmp_path / ("b%d" % k)), h=0.05, ratio=1.1, extent=3.0, core=0.6, points=40 + 9 * k,
+                              nu=0.025, dt=0.01, nt=10, vel_tol=1e-10, pois_tol=1e-10,
+                              method=("LUO", "FADLUN", "OSC_CYLINDER", "LUO")[k])
+
+    def run(folder):
+        with cb.NavierStokesSolver(folder) as s:
+            s.set_option("write_output", 0)
+            s.initialise()
+            s.stepTime(2)
+            return s.get("u"), s.get("ghost_tags_uv"), np.array(s.forces())
+
+    folders = [cylinder(k) for k in range(4)]
+    alone, failures = [run(f) for f in folders], []
+
+    def work(k):
+        try:
+            for _ in range(6):
+                assert all(np.array_equal(a, b) for a, b in zip(run(folders[k]), alone[k]))
+        except Exception as e:  # noqa: BLE001  (reported by the test's thread)
+            failures.append((k, repr(e)))
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failures, failures
