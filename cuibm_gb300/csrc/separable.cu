@@ -1264,7 +1264,8 @@ bool tridiagonal_qr(std::vector<double> &d, std::vector<double> e, std::vector<S
     return true;
 }
 
-// the inverse of the leading n x n block (n <= 3) of K, rows of 3, by elimination with pivoting
+// the inverse of the leading n x n block (n <= 3) of K, rows of 3, by elimination with pivoting;
+// false: singular or not finite
 bool invert3(double *K, int n)
 {
     double a[3][6] = {};
@@ -1287,7 +1288,10 @@ bool invert3(double *K, int n)
             }
     }
     for (int i = 0; i < n; ++i)
-        for (int j = 0; j < n; ++j) K[3 * i + j] = a[i][n + j];
+        for (int j = 0; j < n; ++j) {
+            K[3 * i + j] = a[i][n + j];
+            if (!std::isfinite(K[3 * i + j])) return false;
+        }
     return true;
 }
 
@@ -1722,8 +1726,9 @@ static char *plan_malloc(size_t bytes)
     return static_cast<char *>(p);
 }
 
-// The tables of grid g into P.a.f[k]; false where the eigenvalues do not converge.  nq: the
-// threads a mode of k_sep_tri (the same for all grids of a launch).
+// The tables of grid g into P.a.f[g]; false where the eigenvalues do not converge or the pinned
+// cells' correction is singular: the system then keeps its other preconditioner.  nq: the threads
+// a mode of k_sep_tri (the same for all grids of a launch).
 static bool build_grid(Context &c, SepPlan &P, int g, const SepGrid &G, bool sym, int nq)
 {
     SepDev &d = P.a.f[g];
@@ -1901,8 +1906,7 @@ static bool build_grid(Context &c, SepPlan &P, int g, const SepGrid &G, bool sym
         for (int b = 0; b <= np; ++b) d.K[3 * a + b] = b == np ? -at_pin[a][b] : at_pin[a][b];
     for (int p = 0; p < np; ++p) d.K[3 * p + p] += 1 / delta[p];
     d.K[3 * np + np] += 1 / reg;
-    if (!invert3(d.K, np + 1)) throw CudaError("the separable preconditioner's pinned-cell correction is singular");
-    return true;
+    return invert3(d.K, np + 1);
 }
 
 static void build_separable(Context &c, LinearSystem &S);
