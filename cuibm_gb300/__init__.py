@@ -126,6 +126,8 @@ def library():
         L.cuibm_batch_initialise.argtypes = [vp]
         L.cuibm_batch_step.argtypes = [vp, ip]
         L.cuibm_batch_autotune.argtypes = [vp, ip, ctypes.POINTER(ip)]
+        L.cuibm_batch_graph_steps.argtypes = [vp]
+        L.cuibm_batch_graph_steps.restype = ctypes.c_longlong
         L.cuibm_batch_size.argtypes = [vp]
         L.cuibm_batch_instance.argtypes = [vp, ip]
         L.cuibm_batch_instance.restype = vp
@@ -403,6 +405,10 @@ class Batch:
         nb = ctypes.c_int()
         self._check(self._L.cuibm_batch_autotune(self._h, int(steps), ctypes.byref(nb)))
         return nb.value
+
+    def graph_steps(self):
+        """How many of the batch's steps were one graph launch (CUIBM_BATCH_GRAPH=1)."""
+        return self._L.cuibm_batch_graph_steps(self._h)
 
     def close(self):
         if getattr(self, "_h", None):

@@ -22,8 +22,9 @@
 #include "../../include/cuibm.h"
 #include "batch_member.h"
 
-// With CUIBM_BATCH_GRAPH=1 the batch step is one CUDA graph: every instance's step graph
-// is a child of it, with no edges between them (the instances are independent),
+// With CUIBM_BATCH_GRAPH=1 the batch step is one CUDA graph: every instance's step is
+// recorded into it as a branch of its own, with no edges between them (the instances are
+// independent; a branch, not a child graph, since those take no conditional nodes),
 // launched once per batch step on the batch's own stream, and rebuilt when an
 // instance's step graph changes (a new solver grid from the autotuner, an option).  It
 // is off by default: on the 64-instance benchmark it ran at 208 Mcell-steps/s against
@@ -36,7 +37,8 @@ struct cuibm_batch {
     cudaStream_t stream = nullptr;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
-    std::vector<cudaGraph_t> members;  // the instance graphs the batch graph was built from
+    std::vector<unsigned long long> members;  // the instance graphs' numbers when it was built
+    long long graph_steps = 0;                // batch steps that were one graph launch
 };
 
 static void drop_graph(cuibm_batch *b)
@@ -52,7 +54,7 @@ static void drop_graph(cuibm_batch *b)
 // has none (the batch then steps the instances one by one)
 static bool batch_graph(cuibm_batch *b)
 {
-    std::vector<cudaGraph_t> cur(b->ctx.size());
+    std::vector<unsigned long long> cur(b->ctx.size());
     for (size_t k = 0; k < b->ctx.size(); ++k) {
         cur[k] = cuibm_batch_member_graph(b->ctx[k]);
         if (!cur[k]) {
@@ -63,13 +65,23 @@ static bool batch_graph(cuibm_batch *b)
     if (b->exec && cur == b->members) return true;
     drop_graph(b);
     if (!b->stream && cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess) return false;
-    if (cudaGraphCreate(&b->graph, 0) != cudaSuccess) return false;
-    for (cudaGraph_t g : cur) {
-        cudaGraphNode_t node;
-        if (cudaGraphAddChildGraphNode(&node, b->graph, nullptr, 0, g) != cudaSuccess) {
-            drop_graph(b);
-            return false;
+    cudaEvent_t fork;
+    if (cudaEventCreateWithFlags(&fork, cudaEventDisableTiming) != cudaSuccess) return false;
+    bool ok = cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeRelaxed) == cudaSuccess;
+    if (ok) {
+        ok = cudaEventRecord(fork, b->stream) == cudaSuccess;
+        for (size_t k = 0; k < cur.size() && ok; ++k)
+            ok = cuibm_batch_member_record(b->ctx[k], b->stream, fork) == CUIBM_OK;
+        if (cudaStreamEndCapture(b->stream, &b->graph) != cudaSuccess) {
+            b->graph = nullptr;
+            ok = false;
         }
+    }
+    cudaEventDestroy(fork);
+    if (!ok) {
+        cudaGetLastError();
+        drop_graph(b);
+        return false;
     }
     if (cudaGraphInstantiate(&b->exec, b->graph, 0) != cudaSuccess) {
         drop_graph(b);
@@ -158,6 +170,7 @@ int cuibm_batch_step(cuibm_batch *b, int nsteps)
         if (cudaStreamSynchronize(b->stream) != cudaSuccess)
             return batch_fail(b, CUIBM_ERR_CUDA, "batch: the batch step graph failed");
         for (cuibm_ctx *c : b->ctx) cuibm_batch_member_advance(c, nsteps);
+        b->graph_steps += nsteps;
     } else {
         for (int s = 0; s < nsteps; ++s)
             for (size_t k = 0; k < b->ctx.size(); ++k) {
@@ -238,6 +251,8 @@ int cuibm_batch_autotune(cuibm_batch *b, int steps, int *blocks_out)
     if (blocks_out) *blocks_out = cand[best];
     return CUIBM_OK;
 }
+
+long long cuibm_batch_graph_steps(const cuibm_batch *b) { return b ? b->graph_steps : 0; }
 
 int cuibm_batch_size(const cuibm_batch *b) { return b ? (int)b->ctx.size() : 0; }
 

@@ -314,6 +314,7 @@ static void build_step_graph(Context &c)
     CUIBM_TRY(cudaStreamEndCapture(c.stream, &c.step_graph));
     CUIBM_TRY(cudaGraphInstantiate(&c.step_exec, c.step_graph, 0));
     c.static_kernels = count_kernel_nodes(c.step_graph);
+    ++c.step_graph_number;
 }
 
 }  // namespace cuibm
@@ -646,13 +647,30 @@ int cuibm_step(cuibm_ctx *h, int nsteps)
 }
 
 // the batch's view of an instance (batch_member.h)
-cudaGraph_t cuibm_batch_member_graph(cuibm_ctx *h)
+unsigned long long cuibm_batch_member_graph(cuibm_ctx *h)
 {
-    if (!h) return nullptr;
+    if (!h) return 0;
     const Context &c = h->c;
-    if (!c.initialised || !c.use_graph || c.profile_phases || c.sa_rebuild || !c.step_exec) return nullptr;
-    if (c.sys1.sep || c.sys2.sep) return nullptr;  // conditional nodes are not taken in a child graph
-    return c.step_graph;
+    if (!c.initialised || !c.use_graph || c.profile_phases || c.sa_rebuild || !c.step_exec) return 0;
+    return c.step_graph_number;
+}
+
+int cuibm_batch_member_record(cuibm_ctx *h, cudaStream_t on, cudaEvent_t fork)
+{
+    Context &c = h->c;
+    cudaEvent_t join = nullptr;
+    CUIBM_GUARD(h, {
+        CUIBM_TRY(cudaEventCreateWithFlags(&join, cudaEventDisableTiming));
+        struct Destroyed {
+            cudaEvent_t e;
+            ~Destroyed() { cudaEventDestroy(e); }
+        } destroyed{join};
+        CUIBM_TRY(cudaStreamWaitEvent(c.stream, fork, 0));  // the stream joins the capture
+        record_step(c, true);
+        CUIBM_TRY(cudaEventRecord(join, c.stream));
+        CUIBM_TRY(cudaStreamWaitEvent(on, join, 0));
+    });
+    return CUIBM_OK;
 }
 
 cudaStream_t cuibm_batch_member_stream(cuibm_ctx *h) { return h ? h->c.stream : nullptr; }

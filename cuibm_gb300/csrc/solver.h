@@ -268,6 +268,7 @@ struct Context {
     unsigned long long *solve_trace = nullptr;  // device, 2 x kTraceLen
     cudaGraphExec_t step_exec = nullptr;
     cudaGraph_t step_graph = nullptr;
+    unsigned long long step_graph_number = 0;  // how many were built
     int static_kernels = 0;  // kernel nodes of the step graph outside the solver loops
 
     // modified Fadlun: host copies of the patched rows (for the host matrices)

@@ -319,6 +319,8 @@ int cuibm_batch_step(cuibm_batch *b, int nsteps);
  * *blocks_out (may be null) gets the choice: the block count, or minus the rows a
  * thread of a per-instance choice. */
 int cuibm_batch_autotune(cuibm_batch *b, int steps, int *blocks_out);
+/* how many of the batch's steps were one graph launch (CUIBM_BATCH_GRAPH=1 in the environment) */
+long long cuibm_batch_graph_steps(const cuibm_batch *b);
 int cuibm_batch_size(const cuibm_batch *b);
 cuibm_ctx *cuibm_batch_instance(cuibm_batch *b, int k);
 const char *cuibm_batch_error(const cuibm_batch *b);
