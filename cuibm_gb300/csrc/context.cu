@@ -941,6 +941,10 @@ int cuibm_set_option(cuibm_ctx *h, const char *key, double value)
         CUIBM_GUARD(h, {
             set_fused_trace(c, c.sys1, c.trace_solve);
             set_fused_trace(c, c.sys2, c.trace_solve);
+            // (a solve that stamps nothing leaves a count of 0, not an earlier solve's stamps)
+            if (c.trace_solve)
+                CUIBM_TRY(cudaMemsetAsync(c.solve_trace, 0, 2 * kTraceLen * sizeof(unsigned long long), c.stream));
+            if (c.initialised && c.use_graph && (c.sys1.sep || c.sys2.sep)) build_step_graph(c);
         });
     } else if (k == "step_sync") {
         c.step_sync = value != 0;

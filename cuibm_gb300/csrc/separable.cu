@@ -1297,6 +1297,39 @@ bool invert3(double *K, int n)
 
 }  // namespace
 
+// ---- the diagnostic trace -----------------------------------------------------------------
+// With the option trace_solve a solve's launches are stamped as the persistent solves' barriers
+// are: after each of them one thread writes the global timer and the line of the stamp in this
+// file (top bit of the site set, to tell it from a line of fused_kernels.cuh).  A phase is then
+// its kernels, the gaps between them and the stamp's own launch.
+__global__ void k_sep_stamp(unsigned long long *trace, int site)
+{
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    t &= 0xffffffffffffull;
+    const unsigned long long k = site ? trace[0] + 1 : 1;  // (site 0: the solve's start)
+    if (k >= (unsigned long long)kTraceLen) return;
+    trace[k] = (unsigned long long)(site & 0xffff) << 48 | t;
+    trace[0] = k;
+}
+static void stamp_site(Context &c, int site)
+{
+    if (!c.trace_which) return;
+    k_sep_stamp<<<1, 1, 0, c.stream>>>(c.solve_trace + (c.trace_which - 1) * kTraceLen, site);
+    CUIBM_TRY(cudaGetLastError());
+}
+static void stamp(Context &c, int line = __builtin_LINE()) { stamp_site(c, 0x8000 | line); }
+// stamps for the solve launched while it lives
+struct Traced {
+    Context &c;
+    Traced(Context &c_, int which) : c(c_)
+    {
+        c.trace_which = c.trace_solve ? which : 0;
+        stamp_site(c, 0);
+    }
+    ~Traced() { c.trace_which = 0; }
+};
+
 template <int L, int WM, int WN, int ST>
 static void launch_gemm_t(Context &c, const SepPlan &P, double *field, int back)
 {
@@ -1389,10 +1422,15 @@ template <int L>
 static void apply_t(Context &c, const SepPlan &P, const double *in, double *out, int tr)
 {
     if (in) launch_split<L, false>(c, P, in, tr);  // (null: the digits are there already)
+    if (in) stamp(c);  // digits of the field
     launch_gemm<L>(c, P, nullptr, 0);
+    stamp(c);  // product with Q
     launch_tri(c, P);
+    stamp(c);  // tridiagonal solves
     launch_split<L, true>(c, P, nullptr);
+    stamp(c);  // digits of z^, pinned cells
     launch_gemm<L>(c, P, out, 1 + tr);
+    stamp(c);  // product with Q^T
 }
 
 static void apply_grid(Context &c, const SepPlan &P, const double *in, double *out, int transposed = 0)
@@ -1558,6 +1596,7 @@ void launch_separable_apply(Context &c, LinearSystem &S, const double *in, doubl
         k_sep_sweep<<<blocks_for(S.n), kBlock, 0, c.stream>>>(A, S.n, in, out, P.y);
         k_sep_add<<<blocks_for(S.n), kBlock, 0, c.stream>>>(S.n, c.l2.patch.pid, P.y, out);
         CUIBM_TRY(cudaGetLastError());
+        stamp(c);  // sweep on the body's rows
         return;
     }
     if (!P.patched) {
@@ -1570,6 +1609,7 @@ void launch_separable_apply(Context &c, LinearSystem &S, const double *in, doubl
     k_sep_cap<<<blocks_for(32L * P.patched), kBlock, 0, c.stream>>>(P.patched, P.cap, P.gap, P.q);
     k_sep_less<<<blocks_for(S.n), kBlock, 0, c.stream>>>(S.n, in, P.pidx, P.q, P.rin);
     CUIBM_TRY(cudaGetLastError());
+    stamp(c);  // capacitance of the body's rows
     apply_grid(c, P, P.rin, out);
 }
 
@@ -2067,6 +2107,7 @@ struct SepSolve {
             });
         });
         CUIBM_TRY(cudaGetLastError());
+        stamp(c);  // residual and its digits
     }
     void row_half(cudaGraphConditionalHandle h, int use) const
     {
@@ -2075,11 +2116,13 @@ struct SepSolve {
             k_row_apply<decltype(A), 0>
                 <<<nb(), kBlock, 0, c.stream>>>(A, S.n, S.Mp, S.AMp, S.r, nullptr, sums(), 2);
         });
+        stamp(c);  // A M r
         with_rows([&](auto l, auto np) {
             k_row_half<l(), np()><<<row_grid(), 128, 0, c.stream>>>(plan().a, S.r, S.AMp, S.Mp, S.s, x, sums(), S.ks,
                                                                      c.err_word, S.which, h, use);
         });
         CUIBM_TRY(cudaGetLastError());
+        stamp(c);  // half step and its digits
     }
     void row_rest(cudaGraphConditionalHandle h, int use) const
     {
@@ -2088,10 +2131,12 @@ struct SepSolve {
             k_row_apply<decltype(A), 1>
                 <<<nb(), kBlock, 0, c.stream>>>(A, S.n, S.Ms, S.AMs, S.s, nullptr, sums(), 2);
         });
+        stamp(c);  // A M s
         k_row_end<<<nb(), kBlock, 0, c.stream>>>(S.n, x, S.r, S.rs, S.p, S.s, S.Ms, S.AMs, sums(), S.ks, c.err_word,
                                                  S.which, h, use);
         k_bicg_5<<<blocks_for(S.n), kBlock, 0, c.stream>>>(S.n, S.p, S.r, S.AMp, S.ks);
         CUIBM_TRY(cudaGetLastError());
+        stamp(c);  // end of the iteration, next direction
     }
     void row_cg(bool first, cudaGraphConditionalHandle h, int use) const
     {
@@ -2105,11 +2150,13 @@ struct SepSolve {
                 k_cg_1<<<blocks_for(S.n), kBlock, 0, c.stream>>>(A, S.n, S.p, S.q, S.partials, S.ks);
             }
         });
+        stamp(c);  // direction and A p
         with_rows([&](auto l, auto np) {
             k_row_cg<l(), np()><<<row_grid(), 128, 0, c.stream>>>(plan().a, S.w, S.p, S.q, S.r, x, sums(), S.ks,
                                                                    c.err_word, S.which, first, h, use);
         });
         CUIBM_TRY(cudaGetLastError());
+        stamp(c);  // CG step and the digits of r
     }
 
     void init() const
@@ -2127,6 +2174,7 @@ struct SepSolve {
                 k_sep_init<<<nb(), kBlock, 0, c.stream>>>(A, S.n, b, x, S.r, S.partials, S.ks, c.err_word, S.which);
         });
         CUIBM_TRY(cudaGetLastError());
+        stamp(c);  // residual
     }
     // BiCGSTAB to the half step
     void half(bool first, cudaGraphConditionalHandle h, int use) const
@@ -2139,8 +2187,10 @@ struct SepSolve {
         with_op([&](auto A) {
             k_sep_1<<<nb(), kBlock, 0, c.stream>>>(A, S.n, S.Mp, S.AMp, first ? S.r : S.rs, S.partials, S.ks, first);
         });
+        stamp(c);  // A M p
         k_sep_2<<<nb(), kBlock, 0, c.stream>>>(S.n, S.r, S.AMp, S.Mp, S.s, x, S.partials, S.ks, first, h, use);
         CUIBM_TRY(cudaGetLastError());
+        stamp(c);  // half step
     }
     // and from there
     void rest(bool first, cudaGraphConditionalHandle h, int use) const
@@ -2153,10 +2203,12 @@ struct SepSolve {
         with_op([&](auto A) {
             k_sep_3<<<nb(), kBlock, 0, c.stream>>>(A, S.n, S.s, S.Ms, S.AMs, S.partials, S.ks);
         });
+        stamp(c);  // A M s, omega
         k_sep_4<<<nb(), kBlock, 0, c.stream>>>(S.n, x, S.r, S.rs, S.p, S.s, S.Ms, S.AMs, S.partials, S.ks, c.err_word,
                                                S.which, first, h, use);
         k_bicg_5<<<blocks_for(S.n), kBlock, 0, c.stream>>>(S.n, S.p, S.r, S.AMp, S.ks);
         CUIBM_TRY(cudaGetLastError());
+        stamp(c);  // end of the iteration and next direction
     }
     void correct() const
     {
@@ -2166,6 +2218,7 @@ struct SepSolve {
         with_op([&](auto A) { k_sep_accept<<<this->nb(), kBlock, 0, c.stream>>>(A, S.n, S.p, S.Mp, S.partials, S.ks); });
         k_sep_correct<<<nb, kBlock, 0, c.stream>>>(S.n, S.Mp, x, S.ks);
         CUIBM_TRY(cudaGetLastError());
+        stamp(c);  // last correction
     }
     void cg(bool first, cudaGraphConditionalHandle h, int use) const
     {
@@ -2183,9 +2236,11 @@ struct SepSolve {
                 k_cg_1<<<blocks_for(S.n), kBlock, 0, c.stream>>>(A, S.n, S.p, S.q, S.partials, S.ks);
             }
         });
+        stamp(c);  // CG direction and A p
         k_cg_2<2><<<blocks_for(S.n), kBlock, 0, c.stream>>>(S.n, x, S.r, S.z, S.p, S.q, S.w, S.dinv, S.partials, S.ks, c.err_word,
                                                  S.which, h, use);
         CUIBM_TRY(cudaGetLastError());
+        stamp(c);  // CG step
     }
 };
 
@@ -2200,6 +2255,7 @@ void launch_separable_solve(Context &c, LinearSystem &S, const double *b, double
     const SepSolve L{c, S, b, x};
     SepPlan &P = *static_cast<SepPlan *>(S.sep);
     const bool cg = S.krylov == KRYLOV_CG;
+    const Traced traced(c, S.which);
     if (in_graph) {
         L.init();
         CondNode more(c);

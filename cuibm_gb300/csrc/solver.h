@@ -29,7 +29,7 @@ struct InputError {
 
 constexpr int kBlock = 256;
 constexpr int kCoarse = 1500;  // dense solve below this size (about 2M FMAs per cycle)
-constexpr int kTraceLen = 4096;  // timestamps kept per persistent solve (diagnostic trace)
+constexpr int kTraceLen = 4096;  // timestamps kept per solve (diagnostic trace)
 inline int blocks_for(long n, int bs = kBlock) { return (int)((n + bs - 1) / bs); }
 
 // ---- structured operators --------------------------------------------------
@@ -264,8 +264,9 @@ struct Context {
     bool step_sync = true;    // cuibm_step waits for the steps and checks the solves' status;
                               // when false it only enqueues them (cuibm_step(ctx, 0) then checks)
     bool fused_solve = true;  // persistent one-launch solves where available
-    bool trace_solve = false; // persistent solves record per-barrier timestamps
+    bool trace_solve = false; // persistent and separable solves record timestamps
     unsigned long long *solve_trace = nullptr;  // device, 2 x kTraceLen
+    int trace_which = 0;  // the system whose separable solve is being launched with stamps (0: none)
     cudaGraphExec_t step_exec = nullptr;
     cudaGraph_t step_graph = nullptr;
     unsigned long long step_graph_number = 0;  // how many were built

@@ -1,16 +1,19 @@
-"""Per-phase times of the persistent solves, from their in-kernel barrier stamps.
+"""Per-phase times of the linear solves, from the timer stamps they write.
 
 With the option "trace_solve" on, block 0 of a persistent solve stamps the global
 timer at every grid barrier together with the source line of the barrier's call
 site (include/cuibm.h, CUIBM_F_SOLVE_TRACE).  The time between two stamps is the
 phase that ended at the second barrier (its work, its wait for the slowest block
 and the barrier itself), so summing by call site shows where a solve spends its
-time without a profiler.
+time without a profiler.  A separable solve stamps after each of its kernels instead,
+with a line of csrc/separable.cu whose comment names the phase; its phases hold the
+stamp's own launch too.  Solves launched phase by phase (fused_solve 0, a hierarchy
+without the body's rows) write no stamps.
 
     python -m cuibm_gb300.trace CASE_FOLDER [--warm 20] [--system poisson] [--flags "-saStructured 0"]
 
-runs the case for --warm steps, traces the next step and prints, per barrier site
-of csrc/fused_kernels.cuh, the count, total and mean phase time.
+runs the case for --warm steps, traces the next step and prints, per site, the count,
+total and mean phase time.
 """
 import argparse
 import collections
@@ -18,7 +21,17 @@ import os
 
 import numpy as np
 
-SRC = os.path.join(os.path.dirname(os.path.abspath(__file__)), "csrc", "fused_kernels.cuh")
+CSRC = os.path.join(os.path.dirname(os.path.abspath(__file__)), "csrc")
+SEPARABLE = 0x8000  # this bit of a site: a line of separable.cu
+
+
+def site_text(site):
+    """(file:line, the line's text) of a stamp's site."""
+    name, line = ("separable.cu", site - SEPARABLE) if site & SEPARABLE else ("fused_kernels.cuh", site)
+    path = os.path.join(CSRC, name)
+    src = open(path).read().split("\n") if os.path.exists(path) else []
+    text = src[line - 1].strip() if 0 < line <= len(src) else ""
+    return "%s:%d" % (name, line), text[:60]
 
 
 def phases(trace):
@@ -51,7 +64,6 @@ def main(argv=None):
     ap.add_argument("--sequence", type=int, default=0, metavar="N",
                     help="also list the solve's phases N to 2N in order (one iteration's worth)")
     a = ap.parse_args(argv)
-    src = open(SRC).read().split("\n") if os.path.exists(SRC) else []
     with cb.NavierStokesSolver(a.case, a.flags.split()) as s:
         s.set_option("write_output", 0)
         s.initialise()
@@ -69,16 +81,19 @@ def main(argv=None):
             if a.system not in (name, "both"):
                 continue
             ph = phases(t)
+            if not ph:
+                print("%s solve: no stamps (it is launched phase by phase)" % name)
+                continue
             total = sum(us for _, us in ph)
             print("%s solve: %d phases, %.1f us" % (name, len(ph), total))
             for line, (n, us) in table(t):
-                text = src[line - 1].strip()[:60] if 0 < line <= len(src) else ""
-                print("  line %5d  n %4d  total %9.1f us  mean %7.2f us  %5.1f %%  %s" % (
-                    line, n, us, us / n, 100 * us / max(total, 1e-9), text))
+                at, text = site_text(line)
+                print("  %-22s  n %4d  total %9.1f us  mean %7.2f us  %5.1f %%  %s" % (
+                    at, n, us, us / n, 100 * us / max(total, 1e-9), text))
             if a.sequence:
                 print("  phases %d-%d in order:" % (a.sequence, 2 * a.sequence - 1))
                 for k, (line, us) in enumerate(ph[a.sequence:2 * a.sequence]):
-                    print("    %4d  line %5d  %7.2f us" % (a.sequence + k, line, us))
+                    print("    %4d  %-22s  %7.2f us" % (a.sequence + k, site_text(line)[0], us))
 
 
 if __name__ == "__main__":

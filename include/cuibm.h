@@ -112,11 +112,13 @@ enum {
     CUIBM_F_CFL,             /* D P  */
     CUIBM_F_WORK_X,          /* D max(UV,P) operator test input  */
     CUIBM_F_WORK_Y,          /* D max(UV,P) operator test output */
-    CUIBM_F_SOLVE_TRACE,     /* uint64 2*4096: per-barrier timestamps (ns) of the last persistent
-                                velocity (first 4096) and Poisson solve: [count, start, ...], each
-                                entry the timer's low 48 bits with the barrier's source line of
-                                fused_kernels.cuh in the top 16; written only while the option
-                                "trace_solve" is 1 */
+    CUIBM_F_SOLVE_TRACE,     /* uint64 2*4096: timestamps (ns) of the last velocity (first 4096) and
+                                Poisson solve: [count, start, ...], each entry the timer's low 48
+                                bits with a source line in the top 16: of a persistent solve's
+                                barrier in fused_kernels.cuh, or (top bit set) of a separable
+                                solve's stamp in separable.cu; written only while the option
+                                "trace_solve" is 1, cleared when that is set (a count of 0: a
+                                solve launched phase by phase stamps nothing) */
     CUIBM_F_BODY_MOTION,     /* D 12: body centre x, y and centre velocity u, v; the same at the
                                 start of the step; the coupling tolerance and the sub-iterations
                                 of the last strongly coupled step (VIV: 2); 4 spare */
@@ -205,7 +207,7 @@ int cuibm_get_timer(cuibm_ctx *ctx, const char *name, double *ms, int *count);
  * (1: time each phase with events, steps run without the graph), "step_sync"
  * (1: cuibm_step waits and checks the solves' status; 0: it only enqueues the
  * steps on the context's stream and a later cuibm_step(ctx, 0) checks),
- * "trace_solve" (1: record per-barrier timestamps in CUIBM_F_SOLVE_TRACE),
+ * "trace_solve" (1: record the solves' timestamps in CUIBM_F_SOLVE_TRACE),
  * "write_output" (0: no files), "sa_rebuild_interval" (a moving body with the
  * embedded method: the SA hierarchy is rebuilt from the current rows when the set of
  * patched rows changed and at least this many steps passed since the last rebuild;
