@@ -111,7 +111,7 @@ struct KrylovScalars {
     int body_runs, inner_maxit;  // executions of the iteration body in the last solve; mixed
                                  // precision: iterations of one FP32 solve at most
     unsigned int arrive;  // last-block-done counter of the fused reductions
-    int pad;
+    int skip;             // the separable solve's last correction is left out
 };
 
 // grid-barrier state of the persistent solver (fused_solve.cu), zeroed before each launch
