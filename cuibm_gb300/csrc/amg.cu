@@ -26,7 +26,6 @@
 
 namespace cuibm {
 
-
 struct HostCsr {
     int n = 0, m = 0;  // rows, cols
     std::vector<int> ptr, col;

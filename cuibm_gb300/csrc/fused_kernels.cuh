@@ -523,7 +523,7 @@ __device__ __forceinline__ void vcycle_residual0_row(const Op &A, const FLevel<T
 // loads in flight (they do not depend on one another).  The product runs in FP64
 // for the FP32 cycle too: the coarse pressure operator is nearly singular, its
 // inverse has entries of order 1/lambda_min, and an FP32 product of it is noise.
-constexpr int kDenseMax = 1536;  // the coarsest level's size limit (kCoarse in amg.cu is below it)
+constexpr int kDenseMax = 1536;  // the coarsest level's size limit (kCoarse in solver.h is below it)
 
 // The inverse is the same in every cycle: where a block's rows of it fit the launch's
 // dynamic shared memory (S.fused_smem in fused_solve.cu), the kernel loads them once at its

@@ -31,9 +31,10 @@
 // value, and the products of digit i of one factor with digit j of the other, i + j <
 // kDigits, are accumulated as whole numbers below 2^24, which FP32 accumulators hold
 // exactly; every 128 terms the sums of equal i + j go into one 64-bit integer.  What is
-// dropped (i + j >= 7) is 2^-51 of the factors' row maxima, below the rounding of an FP64
-// sum of the same terms (the splitting of Ozaki, Ogita, Oishi and Rump, Numer. Algorithms
-// 59, 2012).
+// dropped (i + j >= 7) is 2^-51 of the factors' row maxima: as little as the rounding of an FP64
+// sum of terms of that size, but more than it where a row's terms are far below its maximum;
+// the iteration on the FP64 residual takes out either (the splitting of Ozaki, Ogita, Oishi and
+// Rump, Numer. Algorithms 59, 2012).
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -319,9 +320,6 @@ __device__ __forceinline__ double block_total(const double (&v)[NV])
     return a;
 }
 
-// One grid row to digits, a block a row.  SPEC false: a field (times the scaling that
-// makes the transform orthonormal); true: z^, with the pinned cells' correction.  A row of
-// 922 is 7 values a thread: bound by one round of loads, the conversion and the stores.
 // the ratio of A0's diagonal to a patched row's own (1 for a row without one)
 __device__ __forceinline__ double row_ratio(const SepDev &d, int i, int k)
 {
@@ -331,6 +329,9 @@ __device__ __forceinline__ double row_ratio(const SepDev &d, int i, int k)
     return ((d.E[I] + d.W[I]) + (d.N[J] + d.S[J])) / own;
 }
 
+// One grid row to digits, a block a row.  SPEC false: a field (times the scaling that
+// makes the transform orthonormal); true: z^, with the pinned cells' correction.  A row of
+// 922 is 7 values a thread: bound by one round of loads, the conversion and the stores.
 template <int L, int NP, bool SPEC>
 __global__ void __launch_bounds__(128) k_sep_split(const __grid_constant__ SepArgs args, const double *__restrict__ in,
                                                    int transposed)
@@ -1461,10 +1462,8 @@ static void launch_tri(Context &c, const SepPlan &P)
     const dim3 grid((nm + cb - 1) / cb, P.grids);
     auto go = [&](auto *fn, size_t smem) { fn<<<grid, threads, smem, c.stream>>>(P.a, m); };
     const size_t rows = (size_t)m * kTriThreads * sizeof(double);
-    if (cb == 8) {
-        if (m <= 4) go(k_sep_tri<8, 4, kTriThreads>, 0);
-        else if (m <= 8) go(k_sep_tri<8, 8, kTriThreads>, 0);
-        else if (m <= 16) go(k_sep_tri<8, 16, kTriThreads>, 0);
+    if (cb == 8) {  // (600 modes and as many rows at least: ten rows a thread and more)
+        if (m <= 16) go(k_sep_tri<8, 16, kTriThreads>, 0);
         else go(k_sep_tri<8, 0, kTriThreads>, rows);
     } else if (threads == 128) {
         if (m <= 2) go(k_sep_tri<4, 2, 128>, 0);
