@@ -24,10 +24,10 @@ FP64 BiCGSTAB, FP32 inner solves under FP64 refinement), with both runs' C_D
 and cylinders run one after another and as one batch (cuibm_batch_*), aggregate
 Mcell-steps/s of both (--no-batch skips it).
 
---impl reference times the reference's algorithm on the host CPU cores: the
-oracle port (oracle/, a C restatement of the reference's kernels and of its
-BiCGSTAB / smoothed-aggregation solvers - the reference itself needs CUSP,
-which is not available, and a GPU build of it cannot be made here).
+"cpu_baseline" is the reference's algorithm on the host CPU cores as this repository
+restates it (oracle/, kind "port"), not the reference.  --impl reference has nothing to
+run and says so: the reference is a CUDA program on CUSP, which is not available, with no
+Python package and no host build of its own.
 """
 import argparse
 import json
@@ -42,6 +42,8 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 METRIC = "Mcell-steps/s"
+REFERENCE_UNAVAILABLE = ("cuIBM is a CUDA/CUSP program without a Python package: pip has nothing to install, and "
+                         "CUSP, which it is built on, is not available here")
 
 
 # Krylov method of both solves in the cylinder workload: BICGSTAB, the
@@ -88,6 +90,13 @@ def workload_config(workload):
     return {"workload": "impulsively started cylinder Re 40, external (Luo) ghost-node method, plain FP64",
             "nx": 270, "ny": 270, "body_points": 157, "dt": 0.01,
             "velocity": KRYLOV + " + diagonal, rtol 1e-5", "poisson": KRYLOV + " + smoothed aggregation, rtol 1e-5"}
+
+
+def separable_label(solve):
+    """A workload's solve ("BICGSTAB + smoothed aggregation, rtol 1e-5") where the library takes the
+    separable preconditioner for the one that the case names."""
+    krylov, rest = solve.split(" + ")
+    return "%s + separable direct inverse (in place of %s), %s" % ((krylov,) + tuple(rest.split(", ")))
 
 
 class ClockSampler:
@@ -249,9 +258,10 @@ def run_ours(a, rank, world, local, pg):
             "iterations_per_launch": its,
             "other_kernels": {k: {"ms": round(v[0], 5), "GB/s": round(v[1] / (v[0] * 1e-3) / 1e9, 1)}
                               for k, v in prof.items()}}
-    # the committed DRAM counts tell the separable solve (one or two iterations) from the
-    # persistent smoothed-aggregation one (four and more on these workloads)
-    label = dom + "_separable" if dom == "poisson_solve" and its is not None and its <= 2 else dom
+    # the committed DRAM counts tell the separable solve from the persistent
+    # smoothed-aggregation one
+    separable = [s.separable(1), s.separable(2)]
+    label = dom + "_separable" if dom == "poisson_solve" and separable[1] else dom
     roof["traffic"], roof["traffic_source"] = profiled_traffic(label, a.workload)
     roof["fp64_issue"] = fp64_issue_roofline(s, prof, a.workload)
     s.close()
@@ -291,6 +301,7 @@ def run_ours(a, rank, world, local, pg):
     e2e = {"value": round(world * cells * a.steps / e2e_s / 1e6, 3), "unit": METRIC,
            "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h}
     return {"value": value, "ms_per_step": ms_per_step, "wall_s": wall, "roofline": roof, "e2e": e2e,
+            "separable": separable,
             "clocks": clk.summary(), "iterations_last_step": [it1, it2], "drag_lift_last_step": [2 * fx, 2 * fy],
             "gpu_launches": launches * a.steps if launches is not None else None}
 
@@ -666,17 +677,14 @@ def main():
     if a.impl == "reference":
         if rank != 0:
             return
-        # the same steps as the GPU arm times (warm-up, then K), on all host cores
-        cb = cpu_baseline(a.workload, budget_s=240.0, warmup=a.warmup, max_steps=a.steps)
-        line = {"impl": "reference", "metric": METRIC, "value": cb["value"], "unit": METRIC, "n_gpus": a.gpus,
-                "steps": a.steps, "warmup": a.warmup, "higher_is_better": True, "dtype": "f64",
-                "data": "synthetic", "config": cfg, "cpu_baseline": cb,
-                "e2e": {"value": cb["value"], "unit": METRIC, "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0}}
-        print(json.dumps(line))
+        print(json.dumps({"impl": "reference", "unavailable": REFERENCE_UNAVAILABLE}))
         return
     r = run_ours(a, rank, world, local, pg)
     if rank != 0:
         return
+    for key, separable in (("velocity", r["separable"][0]), ("poisson", r["separable"][1])):
+        if separable:
+            cfg[key] = separable_label(cfg[key])
     line = {"metric": METRIC, "value": round(r["value"], 3), "unit": METRIC, "n_gpus": world, "steps": a.steps,
             "warmup": a.warmup, "ms_per_step": round(r["ms_per_step"], 4), "higher_is_better": True,
             "scaling": "weak", "vs_baseline": None, "dtype": "f64", "data": "synthetic", "config": cfg,

@@ -119,6 +119,7 @@ def library():
         L.cuibm_case_error.restype = cp
         L.cuibm_profile_kernel.argtypes = [vp, cp, ip, dp, dp]
         L.cuibm_launch_count.argtypes = [vp, ctypes.POINTER(ctypes.c_longlong)]
+        L.cuibm_separable.argtypes = [vp, ip]
         L.cuibm_cv_force_noalloc.argtypes = [vp, vp, vp, vp, vp, vp, ip, ip, ip, ip, ip, ip, ctypes.c_double,
                                              ctypes.c_double, vp, vp]
         L.cuibm_adjoint.argtypes = [vp, ip, ip, dp, dp, dp, dp, ctypes.c_size_t, ctypes.POINTER(AdjointStats)]
@@ -323,6 +324,10 @@ class NavierStokesSolver:
         self._check(self._L.cuibm_profile_kernel(self._h, name.encode(), int(reps), ctypes.byref(ms),
                                                  ctypes.byref(b)))
         return ms.value, b.value
+
+    def separable(self, system):
+        """Whether the solves of system 1 (velocity) or 2 (Poisson) take the separable preconditioner."""
+        return bool(self._L.cuibm_separable(self._h, int(system)))
 
     def launch_count(self):
         """Kernels of this library launched by the last step (graph nodes x loop trips)."""

@@ -1073,6 +1073,12 @@ int cuibm_profile_kernel(cuibm_ctx *h, const char *kernel, int reps, double *avg
     return CUIBM_OK;
 }
 
+int cuibm_separable(const cuibm_ctx *h, int system)
+{
+    if (!h || !h->c.created) return 0;
+    return (system == 1 ? h->c.sys1.sep : system == 2 ? h->c.sys2.sep : nullptr) ? 1 : 0;
+}
+
 int cuibm_launch_count(cuibm_ctx *h, long long *per_step)
 {
     if (!h || !h->c.initialised || !per_step) return CUIBM_ERR_STATE;

@@ -234,6 +234,10 @@ int cuibm_profile_kernel(cuibm_ctx *ctx, const char *kernel, int reps, double *a
  * of iterations it ran. */
 int cuibm_launch_count(cuibm_ctx *ctx, long long *per_step);
 
+/* 1 where the solves of system 1 (velocity) or 2 (Poisson) take the separable preconditioner,
+ * else 0: what the rule (-separable) decided for this case. */
+int cuibm_separable(const cuibm_ctx *ctx, int system);
+
 /* Control-volume force on the body (drag, lift) from caller-owned device arrays,
  * for callers that must not allocate GPU memory: a coupling code or host
  * framework whose own pool has reserved the device memory (a cudaMalloc there

@@ -47,3 +47,10 @@ def test_batch_draws(tmp_path):
 def test_benchmark_cases(tmp_path, workload, cells):
     f, n = bench.make_case(workload, str(tmp_path / "c"))
     assert n == cells and os.path.exists(os.path.join(f, "simParams.yaml"))
+
+
+def test_separable_label():
+    cfg = bench.workload_config("cylinder_re40")
+    for key, asked in (("velocity", "diagonal"), ("poisson", "smoothed aggregation")):
+        text = bench.separable_label(cfg[key])
+        assert text.startswith("BICGSTAB + separable") and asked in text and text.endswith("rtol 1e-5")
